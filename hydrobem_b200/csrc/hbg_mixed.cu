@@ -699,7 +699,11 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             Half hs[LU_GROUPS];
             for (int i = 0, f0 = 0; i < nh; i++) {
                 const int ni = ns / nh + (i < ns % nh ? 1 : 0);
-                hs[i] = Half{side.s[i], f0, ni, std::max(n_sm - 2 * (ns - ni), 1)};  // diagonal factors: two CTAs a matrix
+                // the diagonal factors of the other groups' matrices take two CTAs each: as many SMs are left to
+                // them, but a product keeps half of the device at least (with 160 systems of order 1024 the first
+                // rule alone left it one CTA: LU 50.5 ms, with the half 4.4 ms, with all SMs 4.6; the 40 systems of
+                // order 4096: 22.6 with 88 CTAs, 23.7 with all)
+                hs[i] = Half{side.s[i], f0, ni, std::max(n_sm - 2 * (ns - ni), n_sm / 2)};
                 f0 += ni;
             }
             cudaEventRecord(side.fork, s);
