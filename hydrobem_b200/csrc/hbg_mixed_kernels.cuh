@@ -289,8 +289,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
 }
 
 // ---- the diagonal block: M11 = L11 U11 (no pivoting), then L11^-1 and U11^-1.  Two CTAs per matrix
-// (blockIdx.x = 2 f + side) factor the same block in their own shared memory; side 0 then forms L^-1
-// (and writes the factors back to W), side 1 U^-1.  Outputs: PL ([Lr | Li] rows of L^-1, the A operand
+// (blockIdx.x = 2 f + side, one cluster, so that they run at once) factor the same block in their own
+// shared memory; side 0 then forms L^-1 (and writes the factors back to W, once side 1 has read the block
+// too: a cluster barrier, arrived at after the load), side 1 U^-1.  Outputs: PL ([Lr | Li] rows of L^-1, the A operand
 // of GEMM2, [F][NBL][2 NBL]), PU (U^-1 in the block-real K-major form, the B operand of GEMM1,
 // [F][2 NBL][2 NBL]) and DINV (U^-1 on and above the diagonal, L^-1 below it, per block, for the
 // triangular solves).  A pivot of modulus below 1e-15 sets err (the mixed form then reports the
@@ -457,7 +458,7 @@ __device__ __forceinline__ void df3_product(const float2* A, int lda, const floa
     }
 }
 
-__global__ void __launch_bounds__(DF_THREADS) k_diag_factor(float* __restrict__ W, int Np, size_t bstride, int k0,
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DF_THREADS) k_diag_factor(float* __restrict__ W, int Np, size_t bstride, int k0,
                                                               float* __restrict__ PL, float* __restrict__ PU,
                                                               float2* __restrict__ DINV, int* __restrict__ err) {
     extern __shared__ float2 df_smem[];
@@ -481,6 +482,7 @@ __global__ void __launch_bounds__(DF_THREADS) k_diag_factor(float* __restrict__ 
         d[2] = make_float2(re.z, im.z);
         d[3] = make_float2(re.w, im.w);
     }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // this CTA has read the block
     __syncthreads();
 #pragma unroll 1
     for (int pb = 0; pb < NBL / DF3_P; pb++) {
@@ -533,7 +535,8 @@ __global__ void __launch_bounds__(DF_THREADS) k_diag_factor(float* __restrict__ 
         }
         __syncthreads();
     }
-    // ---- the factors back to W (side 0)
+    // ---- the factors back to W (side 0), the other CTA's reads of the block done
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (side == 0)
 #pragma unroll 8
         for (int t = threadIdx.x; t < NBL * NBL / 4; t += DF_THREADS) {
