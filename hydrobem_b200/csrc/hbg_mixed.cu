@@ -1,6 +1,6 @@
 // hbg_mixed.cu -- the mixed-precision form of the frequency solve: the pair kernels in FP64 as in
 // the FP64 form, the matrices stored as complex64 (two FP32 planes), the LU on the tensor cores
-// (tcgen05 kind::tf32, FP32 accumulation, no pivoting), the right-hand sides and the residuals
+// (tcgen05 kind::tf32 and kind::f16, FP32 accumulation, no pivoting), the right-hand sides and the residuals
 // accumulated in FP64, and iterative refinement until the correction is below 1e-12 of the solution.
 // The result is the solution of the complex64-rounded system (the reference's production path
 // stores its matrices in complex64 too, lo_frequency.rs:1-6).
@@ -62,21 +62,6 @@ static bool make_map16(CUtensorMap* m, void* base, uint64_t d0, uint64_t d1, uin
            CUDA_SUCCESS;
 }
 
-// Rows of 2 w floats viewed as [rows][2][w]: dims {w, 2, rows, d3}, box {32, 1, box_rows, 1}, the
-// 128-byte swizzle (the same shared-memory tile as make_map's).
-static bool make_map_split(CUtensorMap* m, void* base, uint64_t w, uint64_t rows, uint64_t d3, uint64_t row_stride,
-                           uint64_t s3, uint32_t box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[4] = {w, 2, rows, d3};
-    cuuint64_t strides[3] = {w * 4, row_stride, s3};
-    cuuint32_t box[4] = {32, 1, box_rows, 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
-           CUDA_SUCCESS;
-}
-
 // A 4-D tensor map with an arbitrary box, no swizzle (plain row-major tiles in shared memory).
 static bool make_map_box(CUtensorMap* m, CUtensorMapDataType dt, void* base, const uint64_t dims[4],
                          const uint64_t strides[3], const uint32_t box[4]) {
@@ -132,14 +117,21 @@ static std::atomic<int> g_lu_groups_override{0};
 void mixed_lu_groups(int groups) { g_lu_groups_override = std::max(0, std::min(groups, LU_GROUPS)); }
 // the groups of a batch of ns systems of order Np: about eight systems a group, at most LU_GROUPS (a group's
 // launches cover its systems, so a group of a few small systems leaves its products and factors too
-// short to fill the device).  Measured: the 40 systems of order 4096 of the benchmark job 67.0 / 67.5 /
-// 68.1 ms a job with 4 / 3 / 2 groups; the 64 uneven bodies (16 systems a batch, orders 896-5632, two
-// pipelines) 1.79 s with 2 groups against 1.83 / 1.85-2.08 / 1.85-1.93 s with 1 / 3 / 4.
+// short to fill the device); fewer than eight large systems in up to three groups, so that one group's chain of
+// diagonal blocks (217 us a panel) runs beside the products of the others.  LU measured, ms with 1 / 2 / 3 / 4
+// groups: 40 systems of order 4096 17.1 / 16.2 / 15.8 / 15.5; six bodies of 16 systems of orders 1792-3840 on two
+// pipelines 48.3 / 45.8 / 49.2 / 49.6; 4 of order 12288 35.9 / 34.2 / 34.2 / 33.8; 5 of order 18560 114 / 114 /
+// 109 / 110; 10 of order 512 0.47 with any.
 static int lu_groups_for(int Np, int ns) {
-    (void)Np;
     const int o = g_lu_groups_override.load();
-    return std::max(1, std::min(o > 0 ? o : std::min(LU_GROUPS, ns / 8), ns));
+    const int g = ns < 8 && Np >= 2048 ? 3 : std::min(LU_GROUPS, ns / 8);
+    return std::max(1, std::min(o > 0 ? o : g, ns));
 }
+// The panels of a super-step of the LU: its trailing matrix (8 bytes an entry, read and written by the
+// reduction) passes through DRAM once for 256 q columns.  LU measured, ms with q = 1 / 2 / 4: 40 systems of order
+// 4096 19.2 / 16.6 / 15.5, 4 of order 12288 46.0 / 37.2 / 33.8, 5 of order 18560 167 / 122 / 110, 160 of order
+// 1024 4.50 / 4.45 / 4.43 (a short matrix has no more panels; its buffers stay half as large).
+static int lu_super(int Np) { return Np >= 2048 ? LU_Q : 2; }
 struct SideStreams {
     cudaStream_t s[LU_GROUPS + 1] = {};  // the LU groups, then the right-hand sides
     cudaEvent_t fork = nullptr, join[LU_GROUPS + 1] = {};
@@ -183,12 +175,14 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     if (nrhs > 32) MIXED_FAIL(HB_ERR_UNSUPPORTED, "more than 32 right-hand sides (6 per body and one per heading)", -1);
     if (!encode_fn()) MIXED_FAIL(HB_ERR_UNSUPPORTED, "the driver offers no tensor-map encoder (TMA)", -1);
     // ---- batch size from free memory
-    // GEMM operand buffers of the block row (rows 2n <= 2 (Np - NBL), 2 NBL wide), per frequency
-    const size_t prep_rows = std::max<size_t>(2 * (size_t)(Np - NBL), GBN);
-    const size_t prep = prep_rows * 2 * NBL;
+    // the LU's operands of a system: the transposed block row (FP32), the FP16 copies of a super-step's L and U,
+    // the panel's inverses (FP32), the products between its diagonal blocks
+    const int Q = lu_super(Np), SW = Q * PW;  // panels and columns of a super-step
+    const size_t prep = 2 * (size_t)Np * PW, op16 = 2 * (size_t)Np * SW, inv = 2 * (size_t)PW * PW,
+                 midsz = 2 * (size_t)NBL * NBL;
     // per system: the matrices, the LU operands, the diagonal-block inverses, the refinement vectors
-    size_t per_sys = 3 * MB * 4 + 3 * prep * 4 + (size_t)(NBL * 2 * NBL + 4 * NBL * NBL) * 4 +
-                     4 * (size_t)nrhs * Np * 16 + 64 + (size_t)(Np / NBL) * NBL * NBL * 8;
+    size_t per_sys = 3 * MB * 4 + prep * 4 + 2 * op16 * 2 + 2 * inv * 4 + midsz * 8 + 4 * (size_t)nrhs * Np * 16 + 64 +
+                     (size_t)(Np / NBL) * NBL * NBL * 8;
     // per frequency: G systems, the boundary values and incident wave of every panel (with sectors also
     // the projected right-hand sides and the recombined potentials), the finite-depth tiles
     size_t per = G * per_sys + (size_t)(nrhs + H) * N * 16 + (G > 1 ? (size_t)2 * nrhs * N * 16 : 0) +
@@ -237,16 +231,11 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     float* A32 = (float*)get(WS_A32, MB * BS * 4);
     float* W = (float*)get(WS_W, MB * BS * 4);
     float* P2 = (float*)get(WS_P2, prep * BS * 4);
-    // a later update's B operand: rows of 4 NBL (two 128-row blocks of U) for the 256-deep trailing update
-    const size_t p3size = 2 * prep;
-    float* P3 = (float*)get(WS_P3, p3size * BS * 4);
-    // FP16 operands of the trailing update: P3's 4 NBL-wide layout, and the L rows of the outer step's
-    // two block columns beyond its panel, [rows][Lr (2 NBL) | Li (2 NBL)]
-    __half* P3h = (__half*)get(WS_P3H, p3size * BS * 2);
-    const size_t l16_rows = std::max<size_t>(Np > 2 * NBL ? Np - 2 * NBL : 0, GBM);
-    __half* L16 = (__half*)get(WS_L16, l16_rows * 4 * NBL * BS * 2);
-    float* PL = (float*)get(WS_PL, (size_t)NBL * 2 * NBL * BS * 4);
-    float* PU = (float*)get(WS_PU, (size_t)4 * NBL * NBL * BS * 4);
+    __half* L16 = (__half*)get(WS_L16, op16 * BS * 2);  // [BS][2 planes][Np rows][SW]
+    __half* U16 = (__half*)get(WS_U16, op16 * BS * 2);  // [BS][2 planes][SW rows][Np]
+    float* PX = (float*)get(WS_PX, inv * BS * 4);
+    float* PY = (float*)get(WS_PY, inv * BS * 4);
+    float2* TXY = (float2*)get(WS_TXY, midsz * BS * sizeof(float2));
     float2* DINV = (float2*)get(WS_DINV, nblk * NBL * NBL * BS * sizeof(float2));
     double2* u = (double2*)get(WS_U, (size_t)nrhs * N * B * 16);
     double2* phiI = (double2*)get(WS_PHII, (size_t)std::max(H, 1) * N * B * 16);
@@ -285,25 +274,18 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     if (!okb) MIXED_FAIL(HB_ERR_INTERNAL, "device memory allocation failed for the mixed form", -1);
     last_surrogate_pairs() = 0;
     // ---- tensor maps (whole batch; the batch index is the 4th coordinate)
-    CUtensorMap mapW, mapPL, mapPU, mapP2, mapP3, mapP3h, mapL16, mapP3w16;
+    CUtensorMap mapW, mapPX, mapPY, mapP2, mapL16, mapU16;
     const uint64_t fb = 4;  // bytes per float
     bool okm = make_map(&mapW, W, Np, Np, 2, BS, Np * fb, NP2 * fb, MB * fb, GBM) &&
-               make_map(&mapPL, PL, 2 * NBL, NBL, 1, BS, 2 * NBL * fb, (uint64_t)NBL * 2 * NBL * fb,
-                        (uint64_t)NBL * 2 * NBL * fb, GBM) &&
-               make_map(&mapPU, PU, 2 * NBL, 2 * NBL, 1, BS, 2 * NBL * fb, (uint64_t)4 * NBL * NBL * fb,
-                        (uint64_t)4 * NBL * NBL * fb, GBN) &&
-               make_map(&mapP2, P2, 2 * NBL, prep_rows, 1, BS, 2 * NBL * fb, prep * fb, prep * fb, GBN) &&
-               // P3 as rows of 2 NBL (one 128-row block of U), of 4 NBL (two blocks), and the 4 NBL rows
-               // viewed as [2][2 NBL] halves (the first block alone: x = kk % NBL, half = kk / NBL)
-               make_map(&mapP3, P3, 2 * NBL, prep_rows, 1, BS, 2 * NBL * fb, p3size * fb, p3size * fb, GBN) &&
-               make_map16(&mapP3w16, P3h, 4 * NBL, prep_rows, 1, BS, 4 * NBL * 2, p3size * 2, p3size * 2, GBN) &&
-               make_map16(&mapL16, L16, 4 * NBL, l16_rows, 1, BS, 4 * NBL * 2, l16_rows * 4 * NBL * 2,
-                          l16_rows * 4 * NBL * 2, GBM) &&
-               make_map_split(&mapP3h, P3, 2 * NBL, prep_rows, BS, 4 * NBL * fb, p3size * fb, GBN);
+               make_map(&mapPX, PX, PW, PW, 2, BS, PW * fb, (uint64_t)PW * PW * fb, inv * fb, GBM) &&
+               make_map(&mapPY, PY, PW, PW, 2, BS, PW * fb, (uint64_t)PW * PW * fb, inv * fb, GBN) &&
+               make_map(&mapP2, P2, PW, Np, 2, BS, PW * fb, (uint64_t)Np * PW * fb, prep * fb, GBN) &&
+               make_map16(&mapL16, L16, SW, Np, 2, BS, SW * 2, (uint64_t)Np * SW * 2, op16 * 2, GBM) &&
+               make_map16(&mapU16, U16, Np, SW, 2, BS, Np * 2, (uint64_t)Np * SW * 2, op16 * 2, 2 * GBK);
     if (!okm) MIXED_FAIL(HB_ERR_INTERNAL, "tensor-map encoding failed", -1);
     const int smem = (int)gemm_smem_bytes();
-    cudaFuncSetAttribute(k_gemm_tf32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_gemm_tf32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(k_cgemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(k_cgemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int dev = 0, n_sm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -495,17 +477,19 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
         P.end(KF_LU_SOLVE, 8.0 * (double)NP2 * nb, s);
     };
     // matrices f0 .. f0 + nb of the batch on stream st, at most cap persistent CTAs
-    auto gemm = [&](const CUtensorMap& mA, const CUtensorMap& mB, GemmArgs g, int f0, int nb, cudaStream_t st,
+    auto gemm = [&](const CUtensorMap& mA, const CUtensorMap& mB, CgemmArgs g, int f0, int nb, cudaStream_t st,
                     int cap, bool f16) {
         g.batch = nb;
         g.b0 = f0;
-        const int tiles = ((g.M + GBM - 1) / GBM) * ((g.Nc + GBN - 1) / GBN) * nb;
+        const int units = g.mt * (g.tri == CG_RIGHT_UPPER ? 1 : g.nt) * nb;
+        if (units <= 0) return;
         P.begin(st);
         if (f16)
-            k_gemm_tf32<true><<<std::min(tiles, cap), GEMM_THREADS, smem, st>>>(mA, mB, mapW, g);
+            k_cgemm<true><<<std::min(units, cap), GEMM_THREADS, smem, st>>>(mA, mB, mapW, g);
         else
-            k_gemm_tf32<false><<<std::min(tiles, cap), GEMM_THREADS, smem, st>>>(mA, mB, mapW, g);
-        P.end(KF_MIXED_GEMM, 2.0 * g.M * (double)g.Nc * g.Kp * nb, st);
+            k_cgemm<false><<<std::min(units, cap), GEMM_THREADS, smem, st>>>(mA, mB, mapW, g);
+        const double k_all = g.tri == CG_FULL ? (double)g.K * g.mt * g.nt : 1.5 * NBL * g.mt * g.nt;
+        P.end(KF_MIXED_GEMM, 8.0 * GBM * GBN * k_all * nb, st);
         (*launches)++;
     };
     SideStreams& side = side_streams();
@@ -567,133 +551,107 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
         // ---- LU of M = A^T without pivoting, blocked by NBL, the products on the tensor cores
         {
             EventTimer t(s, &prof[2]);
-            // Two 128-column blocks per outer step: the second block is updated by the first alone, the
-            // block row of both is solved, and the trailing matrix is updated once per 256 columns
-            // (K' = 512: half the passes over it of a 128-column step).
-            // The LU of LU_GROUPS groups of the batch on side streams: the diagonal-block factors (one
-            // CTA per matrix, barrier-bound) of one group run beside the tensor-core products of the
-            // others, whose persistent grids leave that many SMs free.
+            // The LU of LU_GROUPS groups of the batch on side streams: the chain of a panel's diagonal block of
+            // one group runs beside the tensor-core products of the others, whose persistent grids leave it SMs.
             struct Half {
                 cudaStream_t st;
                 int f0, nb, cap;
             };
-            auto diag = [&](const Half& h, int k0) {
+            auto diag = [&](const Half& h, int k0, int koff) {
                 P.begin(h.st);
-                k_diag_factor<<<2 * h.nb, DF_THREADS, dsmem, h.st>>>(W + (size_t)h.f0 * MB, Np, MB, k0,
-                                                                  PL + (size_t)h.f0 * NBL * 2 * NBL,
-                                                                  PU + (size_t)h.f0 * 4 * NBL * NBL,
-                                                                  DINV + (size_t)h.f0 * nblk * NBL * NBL, err);
+                k_diag_factor<<<2 * h.nb, DF_THREADS, dsmem, h.st>>>(
+                    W + (size_t)h.f0 * MB, Np, MB, k0, koff, PX + (size_t)h.f0 * inv, PY + (size_t)h.f0 * inv,
+                    DINV + (size_t)h.f0 * nblk * NBL * NBL, err);
                 P.end(KF_LU_PANEL, 8.0 * NBL * (double)NBL * NBL * h.nb, h.st);
                 (*launches)++;
             };
-            auto prep_row = [&](const Half& h, int k0, int c0, int ncols) {  // rows k0..k0+NBL, columns c0..c0+ncols
+            auto mid = [&](const Half& h, int k0, int stage) {
                 P.begin(h.st);
-                k_prep_block_row<<<dim3(ncols / 32, NBL / 32, h.nb), dim3(32, 8), 0, h.st>>>(
-                    W + (size_t)h.f0 * MB, Np, MB, k0, c0, ncols, P2 + (size_t)h.f0 * prep, prep);
-                P.end(KF_MIXED_CONVERT, 2.0 * NBL * (double)ncols * 4 * 3 * h.nb, h.st);
+                k_mid<<<dim3(NBL / 32, NBL / 32, stage == 1 ? h.nb : 2 * h.nb), 256, 0, h.st>>>(
+                    stage, W + (size_t)h.f0 * MB, Np, MB, k0, DINV + (size_t)h.f0 * nblk * NBL * NBL, nblk * NBL * NBL,
+                    TXY + (size_t)h.f0 * midsz, PX + (size_t)h.f0 * inv, PY + (size_t)h.f0 * inv);
+                P.end(KF_LU_PANEL, (stage == 1 ? 8.0 : 16.0) * NBL * (double)NBL * NBL * h.nb, h.st);
                 (*launches)++;
             };
-            GemmArgs g0{};
+            auto prep_row = [&](const Half& h, int k0, int c0, int ncols) {  // rows k0..k0+PW, columns c0..c0+ncols
+                P.begin(h.st);
+                k_prep_block_row<<<dim3(ncols / 32, PW / 32, 2 * h.nb), dim3(32, 8), 0, h.st>>>(
+                    W + (size_t)h.f0 * MB, Np, MB, k0, c0, P2 + (size_t)h.f0 * prep);
+                P.end(KF_MIXED_CONVERT, 2.0 * PW * (double)ncols * 8 * h.nb, h.st);
+                (*launches)++;
+            };
+            CgemmArgs g0{};
             g0.err = err;
-            // L(rows below the block) = M(., block k0) U_kk^-1; the rows from h16_row0 on also into L16 at
-            // column offset h16_koff (0: the outer step's first block, NBL: its second)
-            auto gemm_l = [&](const Half& h, int k0, int rows, int h16_row0, int h16_koff) {
-                GemmArgs g = g0;
-                g.h16 = L16;
-                g.h16_bstride = l16_rows * 4 * NBL;
-                g.h16_ld = 4 * NBL;
-                g.h16_row0 = h16_row0;
-                g.h16_koff = h16_koff;
-                g.M = rows;
-                g.Nc = 2 * NBL;
-                g.Kp = 2 * NBL;
-                g.a_planar = 1;
-                g.a_x0 = k0;
-                g.a_kc = NBL;
-                g.a_row0 = k0 + NBL;
-                g.mode = 0;
-                g.o_row0 = k0 + NBL;
+            // W(rows r0 .. , mt tiles; columns c0 .. , nt tiles) -= [L of the super-step's first k columns] [U of its
+            // first k rows], S0 its first column, FP16 operands, FP32 accumulation and reduction into W
+            auto update = [&](const Half& h, int r0, int mt, int c0, int nt, int k) {
+                CgemmArgs g = g0;
+                g.mt = mt;
+                g.nt = nt;
+                g.K = k;
+                g.a_row0 = r0;
+                g.b_n0 = c0;
+                g.subtract = 1;
+                g.o_row0 = r0;
+                g.o_col0 = c0;
+                gemm(mapL16, mapU16, g, h.f0, h.nb, h.st, h.cap, true);
+            };
+            // L(rows k0 + PW ..) = M(., columns k0 .. k0 + PW) Y in place, and into L16 at column koff
+            auto gemm_l = [&](const Half& h, int k0, int koff) {
+                CgemmArgs g = g0;
+                g.mt = (Np - k0 - PW) / GBM;
+                g.nt = 2;
+                g.K = PW;
+                g.tri = CG_RIGHT_UPPER;
+                g.a_k0 = k0;
+                g.a_row0 = k0 + PW;
+                g.o_row0 = k0 + PW;
                 g.o_col0 = k0;
-                g.o_nc = NBL;
-                gemm(mapW, mapPU, g, h.f0, h.nb, h.st, h.cap, false);
+                g.h16 = L16;
+                g.h_bstride = op16;
+                g.h_plane = (size_t)Np * SW;
+                g.h_ld = SW;
+                g.h_row0 = k0 + PW;
+                g.h_col0 = koff;
+                gemm(mapW, mapPY, g, h.f0, h.nb, h.st, h.cap, false);
             };
-            // U(rows k0..k0+NBL, columns c0..c0+ncols) = L_kk^-1 B (prepared in P2), and its block-real
-            // copy into P3 (rows of ld floats, this block's rows from koff, second half at kh)
-            auto gemm_u = [&](const Half& h, int k0, int c0, int ncols, int ld, int kh, int koff) {
-                GemmArgs g = g0;
-                g.M = NBL;
-                g.Nc = 2 * ncols;
-                g.Kp = 2 * NBL;
-                g.a_planar = 0;
-                g.mode = 1;
+            // U(rows k0 .. k0 + PW, columns k0 + PW ..) = X M (transposed in P2), and into U16 at row koff
+            auto gemm_u = [&](const Half& h, int k0, int koff) {
+                CgemmArgs g = g0;
+                g.mt = 2;
+                g.nt = (Np - k0 - PW) / GBN;
+                g.K = PW;
+                g.tri = CG_LEFT_LOWER;
                 g.o_row0 = k0;
-                g.o_col0 = c0;
-                g.o_nc = ncols;
-                g.p3 = P3;
-                g.p3_bstride = p3size;
-                g.p3_n = ncols;
-                g.p3_ld = ld;
-                g.p3_kh = kh;
-                g.p3_koff = koff;
-                g.p3h = ld == 4 * NBL ? P3h : nullptr;  // the trailing update's FP16 copy
-                gemm(mapPL, mapP2, g, h.f0, h.nb, h.st, h.cap, false);
+                g.o_col0 = k0 + PW;
+                g.h16 = U16;
+                g.h_bstride = op16;
+                g.h_plane = (size_t)Np * SW;
+                g.h_ld = Np;
+                g.h_row0 = koff;
+                g.h_col0 = k0 + PW;
+                gemm(mapPX, mapP2, g, h.f0, h.nb, h.st, h.cap, false);
             };
-            // M(rows row0.., columns c0..c0+ncols) -= L(rows, columns a_x0..a_x0+a_kc) U (B operand)
-            auto update = [&](const Half& h, int rows, int row0, int c0, int ncols, int a_x0, int a_kc,
-                              const CUtensorMap& mB, int b_split) {
-                GemmArgs g = g0;
-                g.M = rows;
-                g.Nc = 2 * ncols;
-                g.Kp = 2 * a_kc;
-                g.a_planar = 1;
-                g.a_x0 = a_x0;
-                g.a_kc = a_kc;
-                g.a_row0 = row0;
-                g.mode = 2;
-                g.o_row0 = row0;
-                g.o_col0 = c0;
-                g.o_nc = ncols;
-                g.b_split = b_split;
-                gemm(mapW, mB, g, h.f0, h.nb, h.st, h.cap, false);
-            };
-            // the trailing matrix (rows and columns c2.., n of each) -= [L of the step's two blocks] U13,
-            // K' = 512, FP16 operands (L16, P3h), FP32 accumulation and reduction into W
-            auto trailing = [&](const Half& h, int c2, int n) {
-                GemmArgs g = g0;
-                g.M = n;
-                g.Nc = 2 * n;
-                g.Kp = 4 * NBL;
-                g.a_planar = 0;
-                g.a_row0 = 0;
-                g.mode = 2;
-                g.o_row0 = c2;
-                g.o_col0 = c2;
-                g.o_nc = n;
-                gemm(mapL16, mapP3w16, g, h.f0, h.nb, h.st, h.cap, true);
-            };
-            // one outer step (columns K0 .. K0 + 2 NBL) of one half
-            auto outer_step = [&](const Half& h, int K0) {
-                const int k1 = K0 + NBL, c2 = K0 + 2 * NBL, n = Np - c2;
-                // first block: factor, L below it, U of the second block's columns, update of the second block
-                diag(h, K0);
-                prep_row(h, K0, k1, NBL);
-                gemm_l(h, K0, Np - k1, c2, 0);
-                gemm_u(h, K0, k1, NBL, 2 * NBL, NBL, 0);
-                update(h, Np - k1, k1, k1, NBL, K0, NBL, mapP3, 0);
-                // U of the first block's rows beyond the panel (while L_KK^-1 is at hand)
-                if (n > 0) {
-                    prep_row(h, K0, c2, n);
-                    gemm_u(h, K0, c2, n, 4 * NBL, 2 * NBL, 0);
+            // the panel at column k0 of the super-step that begins at S0
+            auto panel = [&](const Half& h, int S0, int k0) {
+                const int w = std::min(PW, Np - k0), c2 = k0 + w, n = Np - c2, koff = k0 - S0;
+                if (koff > 0) {
+                    update(h, k0, (Np - k0) / GBM, k0, w / GBN, koff);
+                    if (n > 0) update(h, k0, w / GBM, c2, n / GBN, koff);
                 }
-                // second block
-                diag(h, k1);
-                if (n > 0) {
-                    gemm_l(h, k1, n, c2, NBL);
-                    update(h, NBL, k1, c2, n, K0, NBL, mapP3h, NBL);  // its rows beyond the panel: -= L21 U13
-                    prep_row(h, k1, c2, n);
-                    gemm_u(h, k1, c2, n, 4 * NBL, 2 * NBL, NBL);
-                    trailing(h, c2, n);  // the trailing matrix, K' = 512
-                }
+                diag(h, k0, 0);
+                if (w < PW) return;  // an odd last block
+                mid(h, k0, 0);
+                mid(h, k0, 1);
+                diag(h, k0 + NBL, NBL);
+                if (n == 0) return;
+                mid(h, k0, 2);
+                mid(h, k0, 3);
+                prep_row(h, k0, c2, n);
+                gemm_l(h, k0, koff);
+                gemm_u(h, k0, koff);
+                if (koff + PW == SW)
+                    update(h, c2, n / GBM, c2, n / GBN, koff + PW);
             };
             const int nh = lu_groups_for(Np, ns);
             Half hs[LU_GROUPS];
@@ -718,11 +676,9 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             }
             gemv(S32, G > 1 ? up : u, Nm, nullptr, b, ns, KF_RHS, srhs);
             cudaEventRecord(side.join[LU_GROUPS], srhs);
-            int K0 = 0;
-            for (; K0 + 2 * NBL <= Np; K0 += 2 * NBL)
-                for (int i = 0; i < nh; i++) outer_step(hs[i], K0);
-            if (K0 < Np)  // an odd last block
-                for (int i = 0; i < nh; i++) diag(hs[i], K0);
+            for (int S0 = 0; S0 < Np; S0 += SW)
+                for (int k0 = S0; k0 < std::min(S0 + SW, Np); k0 += PW)
+                    for (int i = 0; i < nh; i++) panel(hs[i], S0, k0);
             for (int i = 0; i < nh; i++) {
                 cudaEventRecord(side.join[i], hs[i].st);
                 cudaStreamWaitEvent(s, side.join[i], 0);
@@ -946,10 +902,10 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
 }
 
 // Test support: C (M x N, row-major FP32) = A (M x K, row-major) B^T where B is given N x K
-// (K-major), or C -= A B^T, on the tcgen05 TF32 path of the mixed LU.  M, N, K multiples of 128,
-// 128, 32.
+// (K-major), or C -= A B^T, on the tcgen05 TF32 path of the mixed LU (its complex product, the imaginary planes
+// zero).  M, N, K multiples of 128, 128, 32.
 int debug_gemm_tf32(int M, int N, int K, const float* A, const float* B, float* C, bool subtract, const char** msg) {
-    if (M % GBM || N % 128 || K % GBK || M <= 0 || N <= 0 || K <= 0) {
+    if (M % GBM || N % GBN || K % GBK || M <= 0 || N <= 0 || K <= 0) {
         *msg = "debug GEMM shape: M % 128, N % 128, K % 32";
         return HB_ERR_VALUE;
     }
@@ -958,46 +914,47 @@ int debug_gemm_tf32(int M, int N, int K, const float* A, const float* B, float* 
         return HB_ERR_UNSUPPORTED;
     }
     MixedBuffers mb;
-    float* dA = mb.get<float>((size_t)M * K);
-    float* dB = mb.get<float>((size_t)N * K);
-    float* dC = mb.get<float>((size_t)M * N);
+    const size_t nA = (size_t)M * K, nB = (size_t)N * K, nC = (size_t)M * N;
+    float* dA = mb.get<float>(2 * nA);
+    float* dB = mb.get<float>(2 * nB);
+    float* dC = mb.get<float>(2 * nC);
     int* err = mb.get<int>(1);
     if (!dA || !dB || !dC || !err) {
         *msg = "allocation failed";
         return HB_ERR_INTERNAL;
     }
-    cudaMemcpy(dA, A, sizeof(float) * M * K, cudaMemcpyHostToDevice);
-    cudaMemcpy(dB, B, sizeof(float) * N * K, cudaMemcpyHostToDevice);
-    if (subtract) cudaMemcpy(dC, C, sizeof(float) * M * N, cudaMemcpyHostToDevice);
+    cudaMemset(dA + nA, 0, sizeof(float) * nA);
+    cudaMemset(dB + nB, 0, sizeof(float) * nB);
+    cudaMemset(dC, 0, sizeof(float) * 2 * nC);
+    cudaMemcpy(dA, A, sizeof(float) * nA, cudaMemcpyHostToDevice);
+    cudaMemcpy(dB, B, sizeof(float) * nB, cudaMemcpyHostToDevice);
+    if (subtract) cudaMemcpy(dC, C, sizeof(float) * nC, cudaMemcpyHostToDevice);
     cudaMemset(err, 0, sizeof(int));
     CUtensorMap mA, mB, mC;
-    if (!make_map(&mA, dA, K, M, 1, 1, (uint64_t)K * 4, (uint64_t)M * K * 4, (uint64_t)M * K * 4, GBM) ||
-        !make_map(&mB, dB, K, N, 1, 1, (uint64_t)K * 4, (uint64_t)N * K * 4, (uint64_t)N * K * 4, GBN) ||
-        !make_map(&mC, dC, N, M, 1, 1, (uint64_t)N * 4, (uint64_t)M * N * 4, (uint64_t)M * N * 4, GBM)) {
+    if (!make_map(&mA, dA, K, M, 2, 1, (uint64_t)K * 4, nA * 4, 2 * nA * 4, GBM) ||
+        !make_map(&mB, dB, K, N, 2, 1, (uint64_t)K * 4, nB * 4, 2 * nB * 4, GBN) ||
+        !make_map(&mC, dC, N, M, 2, 1, (uint64_t)N * 4, nC * 4, 2 * nC * 4, GBM)) {
         *msg = "tensor-map encoding failed";
         return HB_ERR_INTERNAL;
     }
-    GemmArgs g{};
-    g.M = M;
-    g.Nc = N;
-    g.Kp = K;
-    g.a_planar = 0;
-    g.mode = subtract ? 2 : 0;
-    g.o_nc = N;
+    CgemmArgs g{};
+    g.mt = M / GBM;
+    g.nt = N / GBN;
+    g.K = K;
+    g.subtract = subtract;
     g.batch = 1;
     g.err = err;
     const int smem = (int)gemm_smem_bytes();
-    cudaFuncSetAttribute(k_gemm_tf32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_gemm_tf32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(k_cgemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     int dev = 0, n_sm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     // fewer CTAs than tiles, so that the persistent loop and both accumulator buffers are exercised
-    const int tiles = (M / GBM) * ((N + GBN - 1) / GBN);
-    k_gemm_tf32<false><<<std::max(1, std::min(tiles / 3, n_sm)), GEMM_THREADS, smem>>>(mA, mB, mC, g);
+    const int tiles = g.mt * g.nt;
+    k_cgemm<false><<<std::max(1, std::min(tiles / 3, n_sm)), GEMM_THREADS, smem>>>(mA, mB, mC, g);
     int herr = 0;
     cudaMemcpy(&herr, err, sizeof(int), cudaMemcpyDeviceToHost);
-    cudaMemcpy(C, dC, sizeof(float) * M * N, cudaMemcpyDeviceToHost);
+    cudaMemcpy(C, dC, sizeof(float) * nC, cudaMemcpyDeviceToHost);
     if (cudaGetLastError() != cudaSuccess) {
         *msg = "CUDA error";
         return HB_ERR_INTERNAL;

@@ -3,16 +3,16 @@
 // Storage: every matrix of a frequency is two FP32 planes (real, imaginary), Np x Np with Np the
 // panel count rounded up to a multiple of 128, column-major as the assembly writes it: entry (k, n)
 // of A at n Np + k.  Read row-major, that buffer is M = A^T, and the LU runs on M without pivoting
-// (blocked by NBL = 128 columns): M = L U, so A = U^T L^T and A x = b is U^T y = b, L^T x = y.
-// Per block step k0 (m = n = Np - k0 - NBL):
-//   diag      M11 = L11 U11 in shared memory; L11^-1 and U11^-1 into small operand buffers
-//   prep2     the block row M12 in the block-real K-major form the GEMM's B operand takes
-//   GEMM1     L21 = M21 U11^-1                    (in place)
-//   GEMM2     U12 = L11^-1 M12                    (in place; also the B operand of GEMM3)
-//   GEMM3     M22 -= L21 U12
-// A complex product C = A B runs as one real product [Cr | Ci] = [Ar | Ai] [[Br, Bi], [-Bi, Br]]
-// on the tensor cores (kind::tf32, FP32 accumulation); the refinement in FP64 restores the
-// accuracy of the solution (iterative refinement against the stored complex64 matrix).
+// (in panels of PW = 256 columns): M = L U, so A = U^T L^T and A x = b is U^T y = b, L^T x = y.
+// Up to LU_Q panels form a super-step, after which the trailing matrix is updated once: its FP32 entries pass
+// through DRAM N / (256 q) times instead of N / 256.  Panel j of a super-step (columns k0 .. k0 + 255):
+//   update    its columns, then its rows to their right, by the super-step's panels before it (FP16 operands)
+//   diag      the 256 x 256 block: two 128 blocks factored and inverted in shared memory, the products
+//             between them in FP32 (k_mid); X = L^-1 and Y = U^-1 of the whole block
+//   L, U      L = M Y below the block (in place), U = X M to its right (from a transposed copy), TF32
+// and after the last panel the trailing matrix -= [L of the super-step] [U of the super-step] (FP16 copies
+// of L and U, FP32 accumulation); the refinement in FP64 restores the accuracy of the solution
+// (iterative refinement against the stored complex64 matrix).
 #pragma once
 #include <cuda_fp16.h>
 
@@ -20,29 +20,29 @@
 
 namespace hbg {
 
-constexpr int NBL = 128;  // LU block width (complex columns)
-constexpr int GBM = 128, GBK = 32, GSTAGES = 4, GBN = 256;
-constexpr int GNBOX = 2;  // ring of 32-column output boxes in shared memory
+constexpr int NBL = 128;    // order of the diagonal blocks
+constexpr int PW = 2 * NBL;  // columns of a panel
+constexpr int LU_Q = 4;      // panels of a super-step, at most
+constexpr int GBM = 128, GBN = 128, GBK = 32, GSTAGES = 3;  // rows, complex columns; FP32 complex entries of a chunk
+constexpr int GNBOX = 2;     // ring of 32-column output boxes in shared memory
 
-struct GemmArgs {
-    int M, Nc, Kp;         // rows, real output columns, real inner dimension
-    int a_planar;          // A from the planar matrix (x = a_x0 + kk % a_kc, plane = kk / a_kc) or a packed buffer
-    int a_x0, a_kc, a_row0;
-    int mode;              // 0 store, 1 store and scatter into the GEMM3 operand, 2 subtract
-    int o_row0, o_col0, o_nc;  // output placement in the planar matrix: column j' -> plane j' / o_nc
-    int batch;             // matrices in the launch
-    int b0;                // index of the launch's first matrix in the tensor maps
-    int b_split;           // 0: B coordinates (kk, row); > 0: B viewed as [row][2][.]: (kk % b_split, kk / b_split, row)
-    float* p3;             // a later update's B operand [F][2 p3_n][p3_ld] (mode 1)
-    size_t p3_bstride;
-    int p3_n;
-    int p3_ld, p3_kh, p3_koff;  // row length, offset of the second (imaginary-weight) half, first row of this block
-    __half* p3h;           // mode 1: an FP16 copy of the p3 scatter (same layout), or null
-    // mode 0: an FP16 copy of the output rows from h16_row0 on, [F][rows][h16_ld]: output column j' of
-    // plane p at p * (h16_ld / 2) + h16_koff + j' % o_nc, row o_row0 + i at o_row0 + i - h16_row0
+enum CgemmTri { CG_FULL, CG_RIGHT_UPPER, CG_LEFT_LOWER };
+struct CgemmArgs {
+    int mt, nt;            // row tiles and column tiles (128 complex columns) of a matrix
+    int K;                 // complex inner length
+    int tri;               // CG_RIGHT_UPPER: C = A Y with Y upper triangular, K = 256: column tile 1 first, then tile 0 with
+                           // its 128 k alone, by the same CTA (C may lie over A); CG_LEFT_LOWER: C = X B with X lower
+                           // triangular, K = 256: row tile 0 with its 128 k alone
+    int a_k0, a_row0;      // A's first k and row in its map
+    int b_k0, b_n0;        // B's first k and column (K-major: row) in its map
+    int subtract;          // C -= A B by a reduction at L2, else C = A B
+    int o_row0, o_col0;    // C's first row and column in the planar matrix
+    int batch, b0;         // matrices of the launch, the first one's index in the maps
+    // an FP16 copy of C: planes of h_plane halves, row o_row0 + i at i + h_row0 (none while negative), column o_col0 + j
+    // at j + h_col0
     __half* h16;
-    size_t h16_bstride;
-    int h16_ld, h16_row0, h16_koff;
+    size_t h_bstride, h_plane;
+    int h_ld, h_row0, h_col0;
     int* err;
 };
 
@@ -51,28 +51,33 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 }
 
 constexpr int GEMM_THREADS = 192;  // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
-constexpr size_t GEMM_STAGE_BYTES = (size_t)(GBM + GBN) * GBK * 4;
+constexpr size_t GEMM_TILE_BYTES = (size_t)GBM * GBK * 4;        // one plane of one operand's chunk
+constexpr size_t GEMM_STAGE_BYTES = 4 * GEMM_TILE_BYTES;         // Ar, Ai, Br, Bi
 constexpr size_t GEMM_BOX_BYTES = (size_t)GBM * 32 * 4;  // one 32-column box of the output tile
 constexpr size_t gemm_smem_bytes() { return 1024 + GSTAGES * GEMM_STAGE_BYTES + GNBOX * GEMM_BOX_BYTES + 256; }
 
-// Persistent, warp-specialized TF32 GEMM of the mixed LU: tiles of 128 x 256 (real columns) taken
-// round-robin over (row tile, column tile, matrix).  Warp 0 lane 0 streams the A/B k-chunks through a
-// 3-stage TMA ring; warp 1 lane 0 issues tcgen05.mma (M 128, N 256) into one of two TMEM
-// accumulators; warps 2..5 read the accumulator (tcgen05.ld) in 32-column chunks, place each chunk in
-// a ring of four shared-memory boxes (128-byte swizzle, conflict-free 16-byte accesses) and write it
-// out by TMA: a store, or for the trailing update a TMA reduction that adds -acc to C in L2 (so C
-// never passes through the SM).  The epilogue of one tile overlaps the main loop of the next.
-// F16: the same pipeline on FP16 operands (kind::f16, 64 halves per 128-byte k-chunk row, packed A only).
-template <bool F16 = false>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_constant__ CUtensorMap mapA,
-                                                               const __grid_constant__ CUtensorMap mapB,
-                                                               const __grid_constant__ CUtensorMap mapC,
-                                                               GemmArgs g) {
+// Persistent, warp-specialized complex product of the mixed LU, C = A B or C -= A B on planar operands:
+// tiles of 128 rows x 128 complex columns taken round-robin over (row tile, column tile, matrix).  A k-chunk
+// is the four planes Ar, Ai, Br, Bi (128-byte rows: 32 FP32 or 64 FP16 entries), streamed by warp 0 through a
+// three-stage TMA ring; warp 1 issues per 32 bytes of k the four M 128, N 128 products Cr += Ar Br,
+// Ci += Ar Bi, Cr += (-Ai) Bi (the descriptor's negation), Ci += Ai Br into one of two TMEM accumulators [Cr | Ci].
+// Each operand byte is loaded once for two products: 64 KB from L2 per 128 x 128 x 64 complex chunk against
+// 96 KB for the real product on the doubled operand [[Br, Bi], [-Bi, Br]], which also had to be stored.
+// F16: FP16 operands (kind::f16), B in its natural row-major form (k rows, N contiguous: MN-major); otherwise
+// FP32 read as TF32, B given transposed (K-major).  Warps 2..5 read the accumulator (tcgen05.ld) in 32-column
+// chunks, place each chunk in a ring of shared-memory boxes (128-byte swizzle, conflict-free 16-byte accesses) and
+// write it out by TMA: a store, or for an update a TMA reduction that adds -acc to C in L2 (so C never
+// passes through the SM).  The epilogue of one tile overlaps the main loop of the next.
+// Bound by the tensor pipe and, over a whole LU, the power cap: the first trailing update of five systems of
+// order 18560 (K = 1024) runs at 1231 TFLOP/s (10.2 ms) where cuBLAS bf16 reaches 1361 sustained; the doubled real
+// product at K = 256 a step ran at 530 on 88 SMs, its C passing through DRAM four times as often.
+template <bool F16>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) k_cgemm(const __grid_constant__ CUtensorMap mapA,
+                                                           const __grid_constant__ CUtensorMap mapB,
+                                                           const __grid_constant__ CUtensorMap mapC, CgemmArgs g) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = align1024(smem_raw);
-    float* sA = reinterpret_cast<float*>(base);
-    float* sB = sA + GSTAGES * GBM * GBK;
-    float* sBox = sB + GSTAGES * GBN * GBK;  // [GNBOX][128 rows][32]
+    float* sBox = reinterpret_cast<float*>(base + GSTAGES * GEMM_STAGE_BYTES);  // [GNBOX][128 rows][32]
     uint64_t* full = reinterpret_cast<uint64_t*>(sBox + GNBOX * GBM * 32);
     uint64_t* empty = full + GSTAGES;
     uint64_t* tfull = empty + GSTAGES;  // [2]
@@ -80,10 +85,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
     uint64_t* drain = tempty + 2;       // the MMA warp's last commit (every issued MMA complete)
     uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mt = (g.M + GBM - 1) / GBM, nt = (g.Nc + GBN - 1) / GBN;
-    const int ntiles = mt * nt * g.batch;
-    constexpr int KE = F16 ? 2 * GBK : GBK;  // operand elements per k-chunk (128 bytes a row either way)
-    const int nk = g.Kp / KE;
+    constexpr int KE = F16 ? 2 * GBK : GBK;  // entries per chunk row (128 bytes either way)
     if (threadIdx.x == 0) {
         for (int s = 0; s < GSTAGES; s++) {
             tc::mbar_init(&full[s], 1);
@@ -99,24 +101,31 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
         tc::prefetch_tensormap(&mapB);
         tc::prefetch_tensormap(&mapC);
     }
-    if (warp == 0) tc::tmem_alloc(tslot, 2 * GBN);
+    if (warp == 0) tc::tmem_alloc(tslot, 4 * GBN);
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *tslot;
-    auto tile_coords = [&](int t, int& m0, int& n0, int& f) {
-        f = g.b0 + t / (mt * nt);
-        int r = t % (mt * nt);
-        n0 = (r / mt) * GBN;  // row tiles fastest: consecutive CTAs share the B block
-        m0 = (r % mt) * GBM;
+    // the CTA's it-th tile: row and column tile, matrix, chunks of k; false beyond the last
+    auto tile = [&](int it, int& m, int& n, int& f, int& nk) -> bool {
+        int u = it, sub = -1;
+        if (g.tri == CG_RIGHT_UPPER) u = it >> 1, sub = 1 - (it & 1);  // units of one row tile
+        const int per = sub < 0 ? g.mt * g.nt : g.mt, t = blockIdx.x + u * gridDim.x;
+        if (t >= per * g.batch) return false;
+        f = t / per;
+        const int r = t - f * per;
+        n = sub < 0 ? r / g.mt : sub;  // row tiles fastest: consecutive CTAs share the B block
+        m = r % g.mt;
+        const bool half = (g.tri == CG_RIGHT_UPPER && n == 0) || (g.tri == CG_LEFT_LOWER && m == 0);
+        nk = (half ? NBL : g.K) / KE;
+        return true;
     };
+    int m, n, f, nk;
     if (warp == 0) {
         if (lane == 0) {
             int kc_global = 0;
             bool bad = false;
-            for (int t = blockIdx.x; t < ntiles && !bad; t += gridDim.x) {
-                int m0, n0, f;
-                tile_coords(t, m0, n0, f);
+            for (int it = 0; !bad && tile(it, m, n, f, nk); it++) {
                 for (int kc = 0; kc < nk; kc++, kc_global++) {
                     const int s = kc_global % GSTAGES;
                     if (kc_global >= GSTAGES && !tc::mbar_wait(&empty[s], ((kc_global / GSTAGES) - 1) & 1)) {
@@ -125,17 +134,24 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
                         break;
                     }
                     tc::mbar_arrive_expect_tx(&full[s], (uint32_t)GEMM_STAGE_BYTES);
+                    uint8_t* st = base + s * GEMM_STAGE_BYTES;
                     const int kk = kc * KE;
-                    int ax = kk, plane = 0;
-                    if (!F16 && g.a_planar) {
-                        ax = g.a_x0 + kk % g.a_kc;
-                        plane = kk / g.a_kc;
+#pragma unroll
+                    for (int p = 0; p < 2; p++)
+                        tc::tma_load_4d(st + p * GEMM_TILE_BYTES, &mapA, &full[s], g.a_k0 + kk, g.a_row0 + m * GBM, p,
+                                        g.b0 + f);
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        uint8_t* sb = st + (2 + p) * GEMM_TILE_BYTES;
+                        if constexpr (F16) {
+#pragma unroll
+                            for (int h = 0; h < 2; h++)  // 64 columns a box
+                                tc::tma_load_4d(sb + h * (GEMM_TILE_BYTES / 2), &mapB, &full[s], g.b_n0 + n * GBN + 64 * h,
+                                                g.b_k0 + kk, p, g.b0 + f);
+                        } else {
+                            tc::tma_load_4d(sb, &mapB, &full[s], g.b_k0 + kk, g.b_n0 + n * GBN, p, g.b0 + f);
+                        }
                     }
-                    tc::tma_load_4d(sA + s * GBM * GBK, &mapA, &full[s], ax, g.a_row0 + m0, plane, f);
-                    if (g.b_split)
-                        tc::tma_load_4d(sB + s * GBN * GBK, &mapB, &full[s], kk % g.b_split, kk / g.b_split, n0, f);
-                    else
-                        tc::tma_load_4d(sB + s * GBN * GBK, &mapB, &full[s], kk, n0, 0, f);
                 }
             }
             // every load still in flight lands before the CTA leaves (also after an error): the last
@@ -148,9 +164,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = F16 ? tc::idesc_f16(GBM, GBN) : tc::idesc_tf32(GBM, GBN);
-            int kc_global = 0, it = 0;
-            for (int t = blockIdx.x; t < ntiles; t += gridDim.x, it++) {
+            constexpr uint32_t idesc = F16 ? (tc::idesc_f16(GBM, GBN) | tc::IDESC_B_MN) : tc::idesc_tf32(GBM, GBN);
+            constexpr uint32_t TB_ = (uint32_t)GEMM_TILE_BYTES;
+            int kc_global = 0;
+            for (int it = 0; tile(it, m, n, f, nk); it++) {
                 const int b = it & 1;
                 // the accumulator buffer must have been drained by the epilogue of tile it - 2
                 if (it >= 2 && !tc::mbar_wait(&tempty[b], ((it >> 1) - 1) & 1)) {
@@ -158,7 +175,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
                     break;
                 }
                 tc::tc_fence_after();
-                const uint32_t d = tmem + b * GBN;
+                const uint32_t cr = tmem + b * 2 * GBN, ci = cr + GBN;
                 bool bad = false;
                 for (int kc = 0; kc < nk; kc++, kc_global++) {
                     const int s = kc_global % GSTAGES;
@@ -168,16 +185,31 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
                         break;
                     }
                     tc::tc_fence_after();
-                    const uint32_t a0 = tc::smem_u32(sA + s * GBM * GBK), b0 = tc::smem_u32(sB + s * GBN * GBK);
-                    // four MMAs per 128-byte row: K = 8 (tf32) or 16 (f16), 32 bytes apart
+                    const uint32_t a0 = tc::smem_u32(base + s * GEMM_STAGE_BYTES), b0 = a0 + 2 * TB_;
+                    // four k-steps per 128-byte row: K = 8 (tf32) or 16 (f16); in the MN-major B, 16 rows of 128 bytes
 #pragma unroll
-                    for (int k8 = 0; k8 < 4; k8++) {
-                        if constexpr (F16)
-                            tc::mma_f16(d, tc::desc_kmajor_sw128(a0 + 32 * k8), tc::desc_kmajor_sw128(b0 + 32 * k8),
-                                        idesc, (kc | k8) != 0);
-                        else
-                            tc::mma_tf32(d, tc::desc_kmajor_sw128(a0 + 32 * k8), tc::desc_kmajor_sw128(b0 + 32 * k8),
-                                         idesc, (kc | k8) != 0);
+                    for (int ks = 0; ks < 4; ks++) {
+                        const uint64_t ar = tc::desc_kmajor_sw128(a0 + 32 * ks), ai = tc::desc_kmajor_sw128(a0 + TB_ + 32 * ks);
+                        uint64_t br, bi;
+                        if constexpr (F16) {
+                            br = tc::desc_mnmajor_sw128(b0 + 2048 * ks, TB_ / 2);
+                            bi = tc::desc_mnmajor_sw128(b0 + TB_ + 2048 * ks, TB_ / 2);
+                        } else {
+                            br = tc::desc_kmajor_sw128(b0 + 32 * ks);
+                            bi = tc::desc_kmajor_sw128(b0 + TB_ + 32 * ks);
+                        }
+                        const uint32_t acc = (kc | ks) != 0;
+                        if constexpr (F16) {
+                            tc::mma_f16(cr, ar, br, idesc, acc);
+                            tc::mma_f16(ci, ar, bi, idesc, acc);
+                            tc::mma_f16(cr, ai, bi, idesc | tc::IDESC_NEG_A, 1);
+                            tc::mma_f16(ci, ai, br, idesc, 1);
+                        } else {
+                            tc::mma_tf32(cr, ar, br, idesc, acc);
+                            tc::mma_tf32(ci, ar, bi, idesc, acc);
+                            tc::mma_tf32(cr, ai, bi, idesc | tc::IDESC_NEG_A, 1);
+                            tc::mma_tf32(ci, ai, br, idesc, 1);
+                        }
                     }
                     tc::mma_commit(&empty[s]);
                 }
@@ -194,10 +226,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
         const int quad = warp & 3;
         const int r = quad * 32 + lane;  // row within the tile
         const bool issuer = threadIdx.x == 64;
-        int it = 0, bx = 0;
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x, it++) {
-            int m0, n0, f;
-            tile_coords(t, m0, n0, f);
+        int bx = 0;
+        for (int it = 0; tile(it, m, n, f, nk); it++) {
             const int b = it & 1;
             const bool ok = tc::mbar_wait(&tfull[b], (it >> 1) & 1);
             // one decision for the four epilogue warps, so none waits at a barrier the others left
@@ -207,52 +237,23 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
                 break;
             }
             tc::tc_fence_after();
-            for (int q = 0; q < GBN / 32; q++, bx++) {
+            const int hr = m * GBM + r + g.h_row0;  // the row of the FP16 copy
+            const float sg = g.subtract ? -1.f : 1.f;
+            for (int q = 0; q < 2 * GBN / 32; q++, bx++) {
                 float v[32];
-                tc::tmem_ld32(tmem + b * GBN + ((uint32_t)(quad * 32) << 16) + q * 32, v);
-                const int jg = n0 + 32 * q;  // real output column of the chunk
-                const bool live = jg < g.Nc;
-                const int plane = jg >= g.o_nc ? 1 : 0, col = jg - plane * g.o_nc;
+                tc::tmem_ld32(tmem + b * 2 * GBN + ((uint32_t)(quad * 32) << 16) + q * 32, v);
+                const int plane = q / (GBN / 32), col = n * GBN + 32 * (q % (GBN / 32));
                 // the box slot is free once the write issued GNBOX boxes ago has read it
                 if (issuer && bx >= GNBOX) tc::bulk_wait_read_n<GNBOX - 1>();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 float* row = sBox + (bx % GNBOX) * GBM * 32 + r * 32;  // 128 B, 16-byte chunks swizzled by r % 8
-                const float sg = g.mode == 2 ? -1.f : 1.f;  // the trailing update adds -acc to C
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     *reinterpret_cast<float4*>(row + 4 * (j ^ (r & 7))) =
                         make_float4(sg * v[4 * j], sg * v[4 * j + 1], sg * v[4 * j + 2], sg * v[4 * j + 3]);
-                if (g.mode == 1 && live && m0 + r < g.M) {
-                    // U(kk = row, j) into the block-real K-major operand of a later update (rows 2n,
-                    // p3_ld wide): row j [Ur(:, j) | -Ui(:, j)], row n + j [Ui(:, j) | Ur(:, j)]
-                    float* p3f = g.p3 + (size_t)f * g.p3_bstride;
-                    __half* p3hf = g.p3h ? g.p3h + (size_t)f * g.p3_bstride : nullptr;
-                    const int n = g.p3_n, kk = g.p3_koff + m0 + r, ld = g.p3_ld, kh = g.p3_kh;
-#pragma unroll
-                    for (int i = 0; i < 32; i++) {
-                        const int j = col + i;
-                        size_t o1, o2;
-                        float w1;
-                        if (plane == 0) {
-                            o1 = (size_t)j * ld + kk;
-                            o2 = (size_t)(n + j) * ld + kh + kk;
-                            w1 = v[i];
-                        } else {
-                            o1 = (size_t)j * ld + kh + kk;
-                            o2 = (size_t)(n + j) * ld + kk;
-                            w1 = -v[i];
-                        }
-                        p3f[o1] = w1;
-                        p3f[o2] = v[i];
-                        if (p3hf) {
-                            p3hf[o1] = __float2half_rn(w1);
-                            p3hf[o2] = __float2half_rn(v[i]);
-                        }
-                    }
-                }
-                if (g.mode == 0 && g.h16 && live && m0 + r < g.M && g.o_row0 + m0 + r >= g.h16_row0) {
-                    __half* h = g.h16 + (size_t)f * g.h16_bstride + (size_t)(g.o_row0 + m0 + r - g.h16_row0) * g.h16_ld +
-                                plane * (g.h16_ld / 2) + g.h16_koff + col;
+                if (g.h16 && hr >= 0) {
+                    __half* h = g.h16 + (size_t)(g.b0 + f) * g.h_bstride + (size_t)plane * g.h_plane +
+                                (size_t)hr * g.h_ld + g.h_col0 + col;
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         __half2 hv[4];
@@ -265,13 +266,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (issuer) {
                     const float* box = sBox + (bx % GNBOX) * GBM * 32;
-                    if (live) {
-                        if (g.mode == 2)
-                            tc::tma_reduce_add_4d(&mapC, box, g.o_col0 + col, g.o_row0 + m0, plane, f);
-                        else
-                            tc::tma_store_4d(&mapC, box, g.o_col0 + col, g.o_row0 + m0, plane, f);
-                    }
-                    tc::bulk_commit();  // one group per box (empty for a chunk beyond the output)
+                    if (g.subtract)
+                        tc::tma_reduce_add_4d(&mapC, box, g.o_col0 + col, g.o_row0 + m * GBM, plane, g.b0 + f);
+                    else
+                        tc::tma_store_4d(&mapC, box, g.o_col0 + col, g.o_row0 + m * GBM, plane, g.b0 + f);
+                    tc::bulk_commit();  // one group per box
                 }
             }
             // the accumulator buffer is free for the MMA of tile it + 2
@@ -285,7 +284,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tf32(const __grid_cons
     __syncthreads();
     // freed even when a drain wait above gave up (err set, the results discarded): a CTA that left
     // holding TMEM would stall every later allocation on its SM
-    if (warp == 0) tc::tmem_dealloc(tmem, 2 * GBN);
+    if (warp == 0) tc::tmem_dealloc(tmem, 4 * GBN);
 }
 
 // ---- the diagonal block: M11 = L11 U11 (no pivoting), then L11^-1 and U11^-1.  Two CTAs per matrix
@@ -459,7 +458,7 @@ __device__ __forceinline__ void df3_product(const float2* A, int lda, const floa
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DF_THREADS) k_diag_factor(float* __restrict__ W, int Np, size_t bstride, int k0,
-                                                              float* __restrict__ PL, float* __restrict__ PU,
+                                                              int koff, float* __restrict__ PX, float* __restrict__ PY,
                                                               float2* __restrict__ DINV, int* __restrict__ err) {
     extern __shared__ float2 df_smem[];
     float2* blk = df_smem;                   // [NBL][DF_LD]: the block, then its factors, then the inverse
@@ -637,54 +636,141 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DF_THREADS) k_diag_f
             if ((i > c) == !upper) D[t] = blk[i * DF_LD + c];
         }
     }
-    if (!upper) {
-        float* PLf = PL + (size_t)f * NBL * 2 * NBL;
-        for (int t = threadIdx.x; t < NBL * NBL; t += DF_THREADS) {  // [Lr | Li] rows of L^-1 (c fastest)
-            const int i = t / NBL, c = t % NBL;
-            const float2 l = i > c ? blk[i * DF_LD + c] : make_float2(i == c ? 1.f : 0.f, 0.f);
-            PLf[(size_t)i * 2 * NBL + c] = l.x;
-            PLf[(size_t)i * 2 * NBL + NBL + c] = l.y;
-        }
-    } else {
-        float* PUf = PU + (size_t)f * 2 * NBL * 2 * NBL;
-        for (int t = threadIdx.x; t < NBL * NBL; t += DF_THREADS) {
-            // U^-1 block-real K-major (i fastest): row c: [Ur(:, c); -Ui(:, c)], row NBL + c: [Ui(:, c); Ur(:, c)]
-            const int c = t / NBL, i = t % NBL;
-            const float2 u = i <= c ? blk[i * DF_LD + c] : make_float2(0.f, 0.f);
-            PUf[(size_t)c * 2 * NBL + i] = u.x;
-            PUf[(size_t)c * 2 * NBL + NBL + i] = -u.y;
-            PUf[(size_t)(NBL + c) * 2 * NBL + i] = u.y;
-            PUf[(size_t)(NBL + c) * 2 * NBL + NBL + i] = u.x;
-        }
+    float* Pf = (upper ? PY : PX) + (size_t)f * 2 * PW * PW + (size_t)koff * PW + koff;
+    for (int t = threadIdx.x; t < NBL * NBL; t += DF_THREADS) {
+        const int a = t / NBL, b = t % NBL, i = upper ? b : a, c = upper ? a : b;  // PX: row i, PY: row c (b fastest)
+        const float2 v = (upper ? i <= c : i > c) ? blk[i * DF_LD + c] : make_float2(!upper && i == c ? 1.f : 0.f, 0.f);
+        Pf[(size_t)a * PW + b] = v.x;
+        Pf[(size_t)PW * PW + (size_t)a * PW + b] = v.y;
     }
 }
 
-// The block row B = rows k0..k0+NBL, columns c0..c0+n in the block-real K-major form
-// [F][2n][2 NBL]: row j: [Br(:, j); -Bi(:, j)], row n + j: [Bi(:, j); Br(:, j)] (32 x 32 tiles
-// transposed through shared memory).
-__global__ void k_prep_block_row(const float* __restrict__ W, int Np, size_t bstride, int k0, int c0, int n,
-                                 float* __restrict__ P2, size_t p2_bstride) {
-    __shared__ float tr[32][33], ti[32][33];
-    const int f = blockIdx.z;
+// The products between the two 128 blocks of a panel's diagonal block, in FP32, a launch a stage (two problems
+// each, blockIdx.z = 2 f + problem, but for stage 1).  The chain of a panel waits for them, so each is spread over
+// 16 CTAs of 32 x 32 output tiles (13-14 us a launch).  X = L^-1 and Y = U^-1 of the blocks from DINV.
+//   stage 0: T0 = L21 = M21 Y11, T1 = U12 = X11 M12    stage 1: M22 -= T0 T1; T0, T1 into W
+//   stage 2: T0 = X22 L21, T1 = U12 Y22                stage 3: X21 = -T0 X11, Y12 = -Y11 T1 (into PX, PY)
+__global__ void __launch_bounds__(256) k_mid(int stage, float* __restrict__ W, int Np, size_t bstride, int k0,
+                                             const float2* __restrict__ DINV, size_t dstride, float2* __restrict__ TXY,
+                                             float* __restrict__ PX, float* __restrict__ PY) {
+    constexpr int KC = 32, LD = 33;
+    __shared__ float2 As[32 * LD], Bs[KC * LD];
+    const int prob = stage == 1 ? 0 : blockIdx.z & 1, f = stage == 1 ? blockIdx.z : blockIdx.z >> 1;
+    float* Wr = W + (size_t)f * bstride + (size_t)k0 * Np + k0;
+    float* Wi = Wr + (size_t)Np * Np;
+    const float2* D = DINV + (size_t)f * dstride + (size_t)(k0 / NBL) * NBL * NBL;  // the two blocks' inverses
+    float2* T = TXY + ((size_t)f * 2 + prob) * NBL * NBL;
+    const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, tid = threadIdx.x;
+    auto w = [&](int r, int c) { const size_t o = (size_t)r * Np + c; return make_float2(Wr[o], Wi[o]); };
+    auto xi = [&](int b, int r, int c) {  // L^-1 of block b
+        return r > c ? D[b * NBL * NBL + r * NBL + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
+    };
+    auto yi = [&](int b, int r, int c) { return r <= c ? D[b * NBL * NBL + r * NBL + c] : make_float2(0.f, 0.f); };
+    // entry (i, k) of the left and (k, j) of the right operand; the triangular operands' zero blocks are left out
+    auto left = [&](int i, int k) {
+        switch (2 * stage + prob) {
+            case 0: return w(NBL + i, k);
+            case 1: return xi(0, i, k);
+            case 2: return T[i * NBL + k];
+            case 4: return xi(1, i, k);
+            case 5: return w(i, NBL + k);
+            case 6: return T[i * NBL + k];
+            default: return yi(0, i, k);
+        }
+    };
+    auto right = [&](int k, int j) {
+        switch (2 * stage + prob) {
+            case 0: return yi(0, k, j);
+            case 1: return w(k, NBL + j);
+            case 2: return T[NBL * NBL + k * NBL + j];
+            case 4: return w(NBL + k, j);
+            case 5: return yi(1, k, j);
+            case 6: return xi(0, k, j);
+            default: return T[k * NBL + j];
+        }
+    };
+    int klo = 0, khi = NBL;
+    if ((stage == 0 && prob == 1) || (stage == 2 && prob == 0)) khi = i0 + 32;  // lower on the left
+    if ((stage == 0 && prob == 0) || (stage == 2 && prob == 1)) khi = j0 + 32;  // upper on the right
+    if (stage == 3) klo = prob == 0 ? j0 : i0;                                 // lower right, upper left
+    const int tr = tid / 16, tc_ = tid % 16;  // outputs (tr, tr + 16) x (tc, tc + 16)
+    float2 acc[2][2];
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 2; b++) acc[a][b] = make_float2(0.f, 0.f);
+    float2 la[4], lb[4];
+    auto load = [&](int kc) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int t = tid + 256 * q, r = t / 32, c = t % 32;
+            la[q] = left(i0 + r, kc + c);
+            lb[q] = right(kc + r, j0 + c);
+        }
+    };
+    load(klo);
+    for (int kc = klo; kc < khi; kc += KC) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int t = tid + 256 * q, r = t / 32, c = t % 32;
+            As[r * LD + c] = la[q];
+            Bs[r * LD + c] = lb[q];
+        }
+        __syncthreads();
+        if (kc + KC < khi) load(kc + KC);  // in flight during the products
+#pragma unroll 8
+        for (int k = 0; k < KC; k++) {
+            const float2 a0 = As[tr * LD + k], a1 = As[(tr + 16) * LD + k];
+            const float2 b0 = Bs[k * LD + tc_], b1 = Bs[k * LD + tc_ + 16];
+            cfma_add(acc[0][0], a0, b0);
+            cfma_add(acc[0][1], a0, b1);
+            cfma_add(acc[1][0], a1, b0);
+            cfma_add(acc[1][1], a1, b1);
+        }
+    }
+    float* Pf = (prob == 0 ? PX : PY) + (size_t)f * 2 * PW * PW + (size_t)NBL * PW;
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const int i = i0 + tr + 16 * a, j = j0 + tc_ + 16 * b;
+            const float2 v = acc[a][b];
+            if (stage == 1) {
+                const size_t o = (size_t)(NBL + i) * Np + NBL + j, ol = (size_t)(NBL + i) * Np + j,
+                             ou = (size_t)i * Np + NBL + j;
+                Wr[o] -= v.x;
+                Wi[o] -= v.y;
+                const float2 l = T[i * NBL + j], u = T[NBL * NBL + i * NBL + j];
+                Wr[ol] = l.x;
+                Wi[ol] = l.y;
+                Wr[ou] = u.x;
+                Wi[ou] = u.y;
+            } else if (stage == 0 || stage == 2) {
+                T[i * NBL + j] = v;
+            } else {  // PX row 128 + i, column j; PY row 128 + j (the column of Y), entry i
+                const size_t o = prob == 0 ? (size_t)i * PW + j : (size_t)j * PW + i;
+                Pf[o] = -v.x;
+                Pf[(size_t)PW * PW + o] = -v.y;
+            }
+        }
+}
+
+// The panel's rows k0 .. k0 + PW, columns c0 .. c0 + n, transposed (32 x 32 tiles through shared memory): row j
+// of P2 [F][2 planes][Np][PW] holds column c0 + j, the K-major B operand of the U product.
+__global__ void k_prep_block_row(const float* __restrict__ W, int Np, size_t bstride, int k0, int c0,
+                                 float* __restrict__ P2) {
+    __shared__ float t[32][33];
+    const int f = blockIdx.z >> 1, p = blockIdx.z & 1;
     const int j0 = blockIdx.x * 32, kk0 = blockIdx.y * 32;
-    const float* Wr = W + (size_t)f * bstride;
-    const float* Wi = Wr + (size_t)Np * Np;
+    const float* Wp = W + (size_t)f * bstride + (size_t)p * Np * Np;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    for (int r = ty; r < 32; r += blockDim.y) {
-        size_t o = (size_t)(k0 + kk0 + r) * Np + c0 + j0 + tx;
-        tr[r][tx] = Wr[o];
-        ti[r][tx] = Wi[o];
-    }
+#pragma unroll
+    for (int r = 0; r < 32; r += 8) t[ty + r][tx] = Wp[(size_t)(k0 + kk0 + ty + r) * Np + c0 + j0 + tx];
     __syncthreads();
-    float* Pf = P2 + (size_t)f * p2_bstride;
-    for (int r = ty; r < 32; r += blockDim.y) {
-        const int j = j0 + r, kk = kk0 + tx;
-        float br = tr[tx][r], bi = ti[tx][r];
-        Pf[(size_t)j * 2 * NBL + kk] = br;
-        Pf[(size_t)j * 2 * NBL + NBL + kk] = -bi;
-        Pf[(size_t)(n + j) * 2 * NBL + kk] = bi;
-        Pf[(size_t)(n + j) * 2 * NBL + NBL + kk] = br;
-    }
+    float* Pf = P2 + ((size_t)f * 2 + p) * Np * PW;
+#pragma unroll
+    for (int r = 0; r < 32; r += 8) Pf[(size_t)(j0 + ty + r) * PW + kk0 + tx] = t[tx][ty + r];
 }
 
 // Partial products of y = M x over column chunks: part[z][f][c][k] = sum_{n in chunk z} M(k, n) x[f][c][n],

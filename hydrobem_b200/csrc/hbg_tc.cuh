@@ -188,6 +188,21 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
            | (0u << 10)              // B format F16
            | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+// Instruction-descriptor bits: A negated, B given M/N-major (its N extent contiguous).
+constexpr uint32_t IDESC_NEG_A = 1u << 13, IDESC_B_MN = 1u << 16;
+
+// Shared-memory descriptor of an MN-major 16-bit tile in the 128-byte swizzle layout: groups of 64
+// elements of the contiguous extent (128 B a row, one row per k), 8 rows a 1024-byte atom: the next 8 k
+// 1024 B on (SBO), the next 64 elements `group` bytes on (LBO).
+__device__ __forceinline__ uint64_t desc_mnmajor_sw128(uint32_t saddr, uint32_t group) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t)(group >> 4) << 16;  // LBO
+    d |= (uint64_t)(1024 >> 4) << 32;   // SBO
+    d |= (uint64_t)1 << 46;             // descriptor version (Blackwell)
+    d |= (uint64_t)2 << 61;             // SWIZZLE_128B
+    return d;
+}
 
 }  // namespace tc
 }  // namespace hbg
