@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "hbg_mixed.h"
@@ -132,6 +133,21 @@ static int lu_groups_for(int Np, int ns) {
 // 4096 19.2 / 16.6 / 15.5, 4 of order 12288 46.0 / 37.2 / 33.8, 5 of order 18560 167 / 122 / 110, 160 of order
 // 1024 4.50 / 4.45 / 4.43 (a short matrix has no more panels; its buffers stay half as large).
 static int lu_super(int Np) { return Np >= 2048 ? LU_Q : 2; }
+// The column pairs of a group of the triangular sweeps, for npair pairs, nblk blocks and nb matrices: the smallest of
+// the larger of two times, the dependency chain of a system (a step: two products of one block, 0.52 us a pair each,
+// and 6 us) and the blocks' products over the SMs (their factor tiles loaded anew for every group: 1.4 us at least).
+static int tri_group_pairs(int npair, int nblk, int nb, int n_sm) {
+    int best = TRI_MAXQ;
+    double tbest = 1e300;
+    for (int q : {8, 6, 5, 4, 3, 2, 1}) {
+        const int groups = (npair + q - 1) / q;
+        const double t = std::max(1.4, 0.52 * q + 0.4), chain = nblk * (2.0 * (0.52 * q + 0.4) + 6.0);
+        const double work = nb * groups * (0.5 * nblk * (nblk - 1) * t + nblk * (t + 4.0)) / n_sm;
+        const double all = std::max(chain, work) + 0.25 * std::min(chain, work);
+        if (all < tbest) tbest = all, best = q;
+    }
+    return best;
+}
 struct SideStreams {
     cudaStream_t s[LU_GROUPS + 1] = {};  // the LU groups, then the right-hand sides
     cudaEvent_t fork = nullptr, join[LU_GROUPS + 1] = {};
@@ -236,7 +252,8 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     float* PX = (float*)get(WS_PX, inv * BS * 4);
     float* PY = (float*)get(WS_PY, inv * BS * 4);
     float2* TXY = (float2*)get(WS_TXY, midsz * BS * sizeof(float2));
-    float2* DINV = (float2*)get(WS_DINV, nblk * NBL * NBL * BS * sizeof(float2));
+    const size_t dinv = nblk * 2 * NBL * NBL;
+    float* DINV = (float*)get(WS_DINV, dinv * BS * 4);
     double2* u = (double2*)get(WS_U, (size_t)nrhs * N * B * 16);
     double2* phiI = (double2*)get(WS_PHII, (size_t)std::max(H, 1) * N * B * 16);
     // symmetry sectors: the right-hand sides projected on the sectors, the potentials of every panel
@@ -244,11 +261,12 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     double2* phi = G > 1 ? (double2*)get(WS_PHI, (size_t)nrhs * N * B * 16) : nullptr;
     double2* b = (double2*)get(WS_B, (size_t)nrhs * Np * BS * 16);
     double2* x = (double2*)get(WS_XM, (size_t)nrhs * Np * BS * 16);
-    float2* r = (float2*)get(WS_R, (size_t)nrhs * Np * BS * 8);
-    float2* rs = (float2*)get(WS_RS, (size_t)nrhs * Np * BS * 8);  // a residual kept for r - A d
+    const int npair = (nrhs + 1) / 2;  // complex64 vectors by column pairs
+    float4* r = (float4*)get(WS_R, (size_t)npair * Np * BS * 16);
+    float4* rs = (float4*)get(WS_RS, (size_t)npair * Np * BS * 16);  // a residual kept for r - A d
     double* norms = (double*)get(WS_NORMS, IR_MAX_IT * 2 * (size_t)BS * 8);  // [iteration][batch][2]
     int* err = (int*)get(WS_ERR, sizeof(int));
-    int* tctrl = (int*)get(WS_TRI_CTRL, sizeof(int) * (1 + (size_t)BS));  // the triangular sweeps' tickets
+    int* tctrl = (int*)get(WS_TRI_CTRL, sizeof(int) * (1 + (size_t)BS * ((nrhs + 1) / 2)));  // the triangular sweeps' tickets
     FreqInfo* dfi = (FreqInfo*)get(WS_FI, sizeof(FreqInfo) * B);
     FdParams* dfd = (FdParams*)get(WS_FD, sizeof(FdParams) * B);
     double* dheads = (double*)get(WS_HEADS, sizeof(double) * std::max(H, 1));
@@ -282,6 +300,14 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
                make_map(&mapP2, P2, PW, Np, 2, BS, PW * fb, (uint64_t)Np * PW * fb, prep * fb, GBN) &&
                make_map16(&mapL16, L16, SW, Np, 2, BS, SW * 2, (uint64_t)Np * SW * 2, op16 * 2, GBM) &&
                make_map16(&mapU16, U16, Np, SW, 2, BS, Np * 2, (uint64_t)Np * SW * 2, op16 * 2, 2 * GBK);
+    CUtensorMap mapF, mapD;  // the sweeps' factor and diagonal-inverse tiles
+    {
+        const uint64_t df[4] = {(uint64_t)Np, (uint64_t)Np, 2, (uint64_t)BS}, sf[3] = {Np * fb, NP2 * fb, MB * fb};
+        const uint64_t dd[4] = {TB, TB, 2, nblk * BS}, sd[3] = {TB * fb, TB * TB * fb, 2 * TB * TB * fb};
+        const uint32_t bx[4] = {TB, TRI_SK, 1, 1};
+        okm = okm && make_map_box(&mapF, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, W, df, sf, bx) &&
+              make_map_box(&mapD, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, DINV, dd, sd, bx);
+    }
     if (!okm) MIXED_FAIL(HB_ERR_INTERNAL, "tensor-map encoding failed", -1);
     const int smem = (int)gemm_smem_bytes();
     cudaFuncSetAttribute(k_cgemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -291,30 +317,6 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     const int dsmem = (int)df_smem_bytes();
     cudaFuncSetAttribute(k_diag_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, dsmem);
-    cudaFuncSetAttribute(k_tri_step<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem_bytes(8));
-    cudaFuncSetAttribute(k_tri_step<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem_bytes(10));
-    cudaFuncSetAttribute(k_tri_step<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem_bytes(12));
-    cudaFuncSetAttribute(k_tri_step<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem_bytes(16));
-    // the persistent sweeps: as many CTAs as fit at once
-    // (the sweep's products are FP32-FMA bound beyond 16 columns: no more padded columns than needed)
-    const int nr_sweep = nrhs <= 8    ? 8
-                         : nrhs <= 10 ? 10
-                         : nrhs <= 12 ? 12
-                         : nrhs <= 16 ? 16
-                         : nrhs <= 20 ? 20
-                         : nrhs <= 24 ? 24
-                                      : 32;
-    const void* sweep_fn = nr_sweep == 8    ? (const void*)k_tri_sweep<8>
-                           : nr_sweep == 10 ? (const void*)k_tri_sweep<10>
-                           : nr_sweep == 12 ? (const void*)k_tri_sweep<12>
-                           : nr_sweep == 16 ? (const void*)k_tri_sweep<16>
-                           : nr_sweep == 20 ? (const void*)k_tri_sweep<20>
-                           : nr_sweep == 24 ? (const void*)k_tri_sweep<24>
-                                            : (const void*)k_tri_sweep<32>;
-    cudaFuncSetAttribute(sweep_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_smem_bytes(nr_sweep));
-    int sweep_per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sweep_per_sm, sweep_fn, TRI_THREADS, tri_smem_bytes(nr_sweep));
-    const int sweep_ctas = n_sm * std::max(sweep_per_sm, 1);
     std::vector<double> heads(std::max(H, 1));
     for (int h = 0; h < H; h++) heads[h] = pr.headings_deg[h] * PI / 180.0;
     std::vector<FreqInfo> fi(B);
@@ -368,18 +370,18 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gv32_smem_bytes<16>());
     // r = rk - M d with the complex64 correction d (FP32 products, FP64 sums; beyond 16 columns in chunks):
     // the residual after a correction that is small against the solution
-    auto gemv32 = [&](const float* Mm, const float2* dv, const float2* rk, float2* out, int nb) {
+    auto gemv32 = [&](const float* Mm, const float4* dv, const float4* rk, float4* out, int nb) {
         CUtensorMap mM, mD;
         const uint64_t dm[4] = {(uint64_t)Np, (uint64_t)Np, 2, (uint64_t)nb};
         const uint64_t sm[3] = {(uint64_t)Np * 4, NP2 * 4, MB * 4};
         const uint32_t bm[4] = {GV_ROWS, GV_COLS, 1, 1};
-        const uint64_t dd[4] = {2 * (uint64_t)Np, (uint64_t)nrhs, (uint64_t)nb, 1};
-        const uint64_t sd[3] = {(uint64_t)Np * 8, (uint64_t)nrhs * Np * 8, (uint64_t)nb * nrhs * Np * 8};
+        const uint64_t dd[4] = {4 * (uint64_t)Np, (uint64_t)npair, (uint64_t)nb, 1};
+        const uint64_t sd[3] = {(uint64_t)Np * 16, (uint64_t)npair * Np * 16, (uint64_t)nb * npair * Np * 16};
         if (!make_map_box(&mM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (void*)Mm, dm, sm, bm)) return false;
         CUtensorMap mDc[2];  // the map of each chunk width (a full chunk, the last one)
         const int nrc[2] = {chunk_width(std::min(16, nrhs)), chunk_width(nrhs - (nrhs - 1) / 16 * 16)};
         for (int q = 0; q < 2; q++) {
-            const uint32_t bd[4] = {2 * GV_COLS, (uint32_t)nrc[q], 1, 1};
+            const uint32_t bd[4] = {4 * GV_COLS, (uint32_t)nrc[q] / 2, 1, 1};
             if (!make_map_box(&mDc[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (void*)dv, dd, sd, bd)) return false;
         }
         P.begin(s);
@@ -399,8 +401,8 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             else
                 k_cgemv32_tma<16><<<g, GV_THREADS, gv32_smem_bytes<16>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
         }
-        k_gemv_reduce<float2, float2><<<dim3((unsigned)(((size_t)nrhs * Nm + 255) / 256), nb), 256, 0, s>>>(
-            Nm, nrhs, nb, nz_tma, part, rk, Np, out, Np);
+        k_residual_reduce<true><<<dim3((unsigned)(((size_t)npair * Nm + 255) / 256), nb), 256, 0, s>>>(
+            Nm, Np, nrhs, nb, nz_tma, part, rk, out);
         P.end(KF_MIXED_RESIDUAL, 8.0 * (double)Nm * Nm * nb, s);
         *launches += 2;
         return true;
@@ -422,59 +424,40 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             k_cgemv_part<16><<<g, 128, 0, s>>>(Nm, Np, MB, nrhs, Mm, xv, ldx, part, nb);
         else
             k_cgemv_part<32><<<g, 128, 0, s>>>(Nm, Np, MB, nrhs, Mm, xv, ldx, part, nb);
-        k_gemv_reduce<<<dim3((unsigned)(((size_t)nrhs * Nm + 255) / 256), nb), 256, 0, s>>>(Nm, nrhs, nb, nzr, part,
-                                                                                           bias, Np, out, Np);
+        if constexpr (std::is_same_v<decltype(out), float4*>)  // a residual, for the sweeps
+            k_residual_reduce<false><<<dim3((unsigned)(((size_t)npair * Nm + 255) / 256), nb), 256, 0, s>>>(
+                Nm, Np, nrhs, nb, nzr, part, bias, out);
+        else
+            k_gemv_reduce<<<dim3((unsigned)(((size_t)nrhs * Nm + 255) / 256), nb), 256, 0, s>>>(Nm, nrhs, nb, nzr, part,
+                                                                                               bias, Np, out, Np);
         P.end(fam, 8.0 * (double)Nm * Nm * nb, s);
         *launches += 2;
     };
     // d = A^-1 d in place (complex64) with the FP32 factors in W: U^T y = d, then L^T d = y, the
     // diagonal blocks by the products with their inverses (stored by the LU)
-    auto trisolve = [&](float2* xv, int nb) {
-        const int nblk_i = Np / TB;
+    auto sweep = [&](auto nq, float4* xv, int nb, int groups, int up) {
+        constexpr int NQ = decltype(nq)::value;
+        cudaFuncSetAttribute(k_tri_sweep<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TriCfg<NQ>::SMEM);
+        k_tri_sweep<NQ><<<std::min((int)nblk * nb * groups, n_sm), TRI_THREADS, TriCfg<NQ>::SMEM, s>>>(
+            mapF, mapD, Np, npair, xv, nb, groups, up, tctrl, err);
+    };
+    auto trisolve = [&](float4* xv, int nb) {  // one persistent sweep per direction
         P.begin(s);
-        if (nrhs <= 32) {  // one persistent sweep per direction
-            const int grid = std::min(nblk_i * nb, sweep_ctas);
-            const size_t sm = tri_smem_bytes(nr_sweep);
-            for (int up = 1; up >= 0; up--) {
-                cudaMemsetAsync(tctrl, 0, sizeof(int) * (1 + (size_t)nb), s);
-                if (nr_sweep == 8)
-                    k_tri_sweep<8><<<grid, TRI_THREADS, sm, s>>>(Np, MB, W, DINV, nrhs, xv, nb, up, tctrl, err);
-                else if (nr_sweep == 10)
-                    k_tri_sweep<10><<<grid, TRI_THREADS, sm, s>>>(Np, MB, W, DINV, nrhs, xv, nb, up, tctrl, err);
-                else if (nr_sweep == 12)
-                    k_tri_sweep<12><<<grid, TRI_THREADS, sm, s>>>(Np, MB, W, DINV, nrhs, xv, nb, up, tctrl, err);
-                else if (nr_sweep == 16)
-                    k_tri_sweep<16><<<grid, TRI_THREADS, sm, s>>>(Np, MB, W, DINV, nrhs, xv, nb, up, tctrl, err);
-                else if (nr_sweep == 20)
-                    k_tri_sweep<20><<<grid, TRI_THREADS, sm, s>>>(Np, MB, W, DINV, nrhs, xv, nb, up, tctrl, err);
-                else if (nr_sweep == 24)
-                    k_tri_sweep<24><<<grid, TRI_THREADS, sm, s>>>(Np, MB, W, DINV, nrhs, xv, nb, up, tctrl, err);
-                else
-                    k_tri_sweep<32><<<grid, TRI_THREADS, sm, s>>>(Np, MB, W, DINV, nrhs, xv, nb, up, tctrl, err);
-                (*launches)++;
+        const int nq = tri_group_pairs(npair, (int)nblk, nb, n_sm), groups = (npair + nq - 1) / nq;
+        for (int up = 1; up >= 0; up--) {
+            cudaMemsetAsync(tctrl, 0, sizeof(int) * (1 + (size_t)nb * groups), s);
+            switch (nq) {
+                case 1: sweep(std::integral_constant<int, 1>(), xv, nb, groups, up); break;
+                case 2: sweep(std::integral_constant<int, 2>(), xv, nb, groups, up); break;
+                case 3: sweep(std::integral_constant<int, 3>(), xv, nb, groups, up); break;
+                case 4: sweep(std::integral_constant<int, 4>(), xv, nb, groups, up); break;
+                case 5: sweep(std::integral_constant<int, 5>(), xv, nb, groups, up); break;
+                case 6: sweep(std::integral_constant<int, 6>(), xv, nb, groups, up); break;
+                default: sweep(std::integral_constant<int, 8>(), xv, nb, groups, up); break;
             }
-            P.end(KF_LU_SOLVE, 8.0 * (double)NP2 * nb, s);
-            return;
+            (*launches)++;
         }
-        for (int dir = 0; dir < 2; dir++) {
-            const int up = dir == 0;
-            for (int st = -1; st < nblk_i - 1; st++) {
-                const int cnt = st < 0 ? 1 : nblk_i - 1 - st;
-                const int stepi = st < 0 ? -1 : (up ? st : nblk_i - 1 - st);
-                dim3 g(cnt, nb);
-                if (nrhs <= 8)
-                    k_tri_step<8><<<g, TRI_THREADS, tri_smem_bytes(8), s>>>(Np, MB, W, DINV, nrhs, xv, stepi, up);
-                else if (nrhs <= 10)
-                    k_tri_step<10><<<g, TRI_THREADS, tri_smem_bytes(10), s>>>(Np, MB, W, DINV, nrhs, xv, stepi, up);
-                else if (nrhs <= 12)
-                    k_tri_step<12><<<g, TRI_THREADS, tri_smem_bytes(12), s>>>(Np, MB, W, DINV, nrhs, xv, stepi, up);
-                else
-                    k_tri_step<16><<<g, TRI_THREADS, tri_smem_bytes(16), s>>>(Np, MB, W, DINV, nrhs, xv, stepi, up);
-                (*launches)++;
-            }
-        }
-        // the factors read once per direction (8 B per entry)
-        P.end(KF_LU_SOLVE, 8.0 * (double)NP2 * nb, s);
+        P.end(KF_LU_SOLVE, 8.0 * (double)NP2 * nb, s);  // the factors read once
     };
     // matrices f0 .. f0 + nb of the batch on stream st, at most cap persistent CTAs
     auto gemm = [&](const CUtensorMap& mA, const CUtensorMap& mB, CgemmArgs g, int f0, int nb, cudaStream_t st,
@@ -561,14 +544,14 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
                 P.begin(h.st);
                 k_diag_factor<<<2 * h.nb, DF_THREADS, dsmem, h.st>>>(
                     W + (size_t)h.f0 * MB, Np, MB, k0, koff, PX + (size_t)h.f0 * inv, PY + (size_t)h.f0 * inv,
-                    DINV + (size_t)h.f0 * nblk * NBL * NBL, err);
+                    DINV + (size_t)h.f0 * dinv, err);
                 P.end(KF_LU_PANEL, 8.0 * NBL * (double)NBL * NBL * h.nb, h.st);
                 (*launches)++;
             };
             auto mid = [&](const Half& h, int k0, int stage) {
                 P.begin(h.st);
                 k_mid<<<dim3(NBL / 32, NBL / 32, stage == 1 ? h.nb : 2 * h.nb), 256, 0, h.st>>>(
-                    stage, W + (size_t)h.f0 * MB, Np, MB, k0, DINV + (size_t)h.f0 * nblk * NBL * NBL, nblk * NBL * NBL,
+                    stage, W + (size_t)h.f0 * MB, Np, MB, k0, DINV + (size_t)h.f0 * dinv, dinv,
                     TXY + (size_t)h.f0 * midsz, PX + (size_t)h.f0 * inv, PY + (size_t)h.f0 * inv);
                 P.end(KF_LU_PANEL, (stage == 1 ? 8.0 : 16.0) * NBL * (double)NBL * NBL * h.nb, h.st);
                 (*launches)++;
@@ -692,7 +675,8 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
         {
             EventTimer t(s, &prof[3]);
             cudaMemsetAsync(x, 0, sizeof(double2) * nrhs * Np * ns, s);
-            k_to_c64<<<592, 256, 0, s>>>((size_t)nrhs * Np * ns, b, r);
+            k_to_pairs<<<dim3((Np + 255) / 256, npair, ns), 256, 0, s>>>(Np, nrhs, b, r);
+            cudaMemsetAsync(norms, 0, sizeof(double) * IR_MAX_IT * 2 * ns, s);
             (*launches)++;
             IrHistory& hist = last_ir_history();
             hist.n = 0;
@@ -708,7 +692,8 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             };
             auto correction = [&](int i) {  // d = A^-1 r (FP32), x += d, norms into slot i
                 trisolve(r, ns);
-                k_ir_update<<<ns, 256, 0, s>>>(Np, nrhs, x, r, norms + (size_t)i * 2 * ns);
+                k_ir_update<<<dim3((Np + 255) / 256, npair, ns), 256, 0, s>>>(
+                    Np, nrhs, x, r, reinterpret_cast<unsigned long long*>(norms) + (size_t)i * 2 * ns);
                 *launches += 1;
             };
             // the forces and the readback of outputs, norms and the error flag (one wait for all)
@@ -765,7 +750,7 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             const int guess = std::min(std::max(ir_guess(), 2), IR_MAX_IT);
             for (int i = 0; i < guess; i++) {
                 const bool more = i + 1 < guess, inc = more && i >= 1 && rs;
-                if (inc) cudaMemcpyAsync(rs, r, sizeof(float2) * nrhs * Np * ns, cudaMemcpyDeviceToDevice, s);
+                if (inc) cudaMemcpyAsync(rs, r, sizeof(float4) * npair * Np * ns, cudaMemcpyDeviceToDevice, s);
                 correction(i);
                 if (more && !(inc && gemv32(A32, r, rs, r, ns))) gemv(A32, x, Np, b, r, ns, KF_MIXED_RESIDUAL, s);
             }

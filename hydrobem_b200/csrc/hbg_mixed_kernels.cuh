@@ -290,10 +290,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_cgemm(const __grid_constant
 // ---- the diagonal block: M11 = L11 U11 (no pivoting), then L11^-1 and U11^-1.  Two CTAs per matrix
 // (blockIdx.x = 2 f + side, one cluster, so that they run at once) factor the same block in their own
 // shared memory; side 0 then forms L^-1 (and writes the factors back to W, once side 1 has read the block
-// too: a cluster barrier, arrived at after the load), side 1 U^-1.  Outputs: PL ([Lr | Li] rows of L^-1, the A operand
-// of GEMM2, [F][NBL][2 NBL]), PU (U^-1 in the block-real K-major form, the B operand of GEMM1,
-// [F][2 NBL][2 NBL]) and DINV (U^-1 on and above the diagonal, L^-1 below it, per block, for the
-// triangular solves).  A pivot of modulus below 1e-15 sets err (the mixed form then reports the
+// too: a cluster barrier, arrived at after the load), side 1 U^-1.  Outputs: PX (rows of L^-1, the A operand of
+// the U product) and PY (columns of U^-1 as rows, the B operand of the L product), the 128 blocks at
+// (koff, koff) of [F][2 planes][PW][PW], and DINV (U^-1 on and above the diagonal, L^-1 below it, two planes
+// a block, for the triangular solves).  A pivot of modulus below 1e-15 sets err (the mixed form then reports the
 // frequency; the FP64 form pivots).
 constexpr int DF_THREADS = 512, DF_LD = NBL + 1, DF_BLK = 32, DF_NB = NBL / DF_BLK, DF_SLD = DF_BLK + 1;
 
@@ -459,7 +459,7 @@ __device__ __forceinline__ void df3_product(const float2* A, int lda, const floa
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DF_THREADS) k_diag_factor(float* __restrict__ W, int Np, size_t bstride, int k0,
                                                               int koff, float* __restrict__ PX, float* __restrict__ PY,
-                                                              float2* __restrict__ DINV, int* __restrict__ err) {
+                                                              float* __restrict__ DINV, int* __restrict__ err) {
     extern __shared__ float2 df_smem[];
     float2* blk = df_smem;                   // [NBL][DF_LD]: the block, then its factors, then the inverse
     float2* T = blk + NBL * DF_LD;  // scratch: the diagonal-block inverses, then the products of the recursion
@@ -630,10 +630,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DF_THREADS) k_diag_f
     __syncthreads();
     // ---- outputs: this side's triangle of the inverse
     {
-        float2* D = DINV + ((size_t)f * (Np / NBL) + k0 / NBL) * NBL * NBL;
+        float* D = DINV + ((size_t)f * (Np / NBL) + k0 / NBL) * 2 * NBL * NBL;
         for (int t = threadIdx.x; t < NBL * NBL; t += DF_THREADS) {
             const int i = t / NBL, c = t % NBL;
-            if ((i > c) == !upper) D[t] = blk[i * DF_LD + c];
+            if ((i > c) == !upper) {
+                const float2 v = blk[i * DF_LD + c];
+                D[t] = v.x;
+                D[NBL * NBL + t] = v.y;
+            }
         }
     }
     float* Pf = (upper ? PY : PX) + (size_t)f * 2 * PW * PW + (size_t)koff * PW + koff;
@@ -651,21 +655,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DF_THREADS) k_diag_f
 //   stage 0: T0 = L21 = M21 Y11, T1 = U12 = X11 M12    stage 1: M22 -= T0 T1; T0, T1 into W
 //   stage 2: T0 = X22 L21, T1 = U12 Y22                stage 3: X21 = -T0 X11, Y12 = -Y11 T1 (into PX, PY)
 __global__ void __launch_bounds__(256) k_mid(int stage, float* __restrict__ W, int Np, size_t bstride, int k0,
-                                             const float2* __restrict__ DINV, size_t dstride, float2* __restrict__ TXY,
+                                             const float* __restrict__ DINV, size_t dstride, float2* __restrict__ TXY,
                                              float* __restrict__ PX, float* __restrict__ PY) {
     constexpr int KC = 32, LD = 33;
     __shared__ float2 As[32 * LD], Bs[KC * LD];
     const int prob = stage == 1 ? 0 : blockIdx.z & 1, f = stage == 1 ? blockIdx.z : blockIdx.z >> 1;
     float* Wr = W + (size_t)f * bstride + (size_t)k0 * Np + k0;
     float* Wi = Wr + (size_t)Np * Np;
-    const float2* D = DINV + (size_t)f * dstride + (size_t)(k0 / NBL) * NBL * NBL;  // the two blocks' inverses
+    const float* D = DINV + (size_t)f * dstride + (size_t)(k0 / NBL) * 2 * NBL * NBL;  // the two blocks' inverses
     float2* T = TXY + ((size_t)f * 2 + prob) * NBL * NBL;
     const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32, tid = threadIdx.x;
     auto w = [&](int r, int c) { const size_t o = (size_t)r * Np + c; return make_float2(Wr[o], Wi[o]); };
-    auto xi = [&](int b, int r, int c) {  // L^-1 of block b
-        return r > c ? D[b * NBL * NBL + r * NBL + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
+    auto dv = [&](int b, int r, int c) {
+        const int o = b * 2 * NBL * NBL + r * NBL + c;
+        return make_float2(D[o], D[o + NBL * NBL]);
     };
-    auto yi = [&](int b, int r, int c) { return r <= c ? D[b * NBL * NBL + r * NBL + c] : make_float2(0.f, 0.f); };
+    auto xi = [&](int b, int r, int c) { return r > c ? dv(b, r, c) : make_float2(r == c ? 1.f : 0.f, 0.f); };  // L^-1
+    auto yi = [&](int b, int r, int c) { return r <= c ? dv(b, r, c) : make_float2(0.f, 0.f); };                // U^-1
     // entry (i, k) of the left and (k, j) of the right operand; the triangular operands' zero blocks are left out
     auto left = [&](int i, int k) {
         switch (2 * stage + prob) {
@@ -849,10 +855,7 @@ __global__ void __launch_bounds__(128) k_cgemv_part(int N, int Np, size_t bstrid
 // chunk of columns n, 16 columns per stage (both FP32 planes, 32 KB, and the 16 complex entries of
 // every right-hand side), GV_STAGES stages in flight from a producer warp, so the bytes in flight do
 // not depend on registers; FP64 accumulation as above.
-// Packed FP32 pairs (fma.rn.f32x2: two FP32 FMAs per instruction).  A complex multiply-add
-// acc += m v is two packed FMAs: acc += (m.re, m.re) (v.re, v.im), then acc += (-m.im, m.im) (v.im, v.re);
-// the right-hand sides are kept in shared memory as {re, im, im, re} so one 16-byte load gives both
-// orders.
+// Packed FP32 pairs (fma.rn.f32x2: two FP32 FMAs per instruction), here over two right-hand sides.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 f2pack(float a, float b) {
     f32x2 r;
@@ -869,7 +872,6 @@ __device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-__device__ __forceinline__ float4 dup_swap(float2 v) { return make_float4(v.x, v.y, v.y, v.x); }
 
 constexpr int GV_ROWS = 256, GV_COLS = 16, GV_STAGES = 3, GV_CHUNK = 1024;
 constexpr int GV_WORKERS = GV_ROWS / 2;
@@ -974,9 +976,11 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv_tma(const __grid_constant_
 // each product and each 16-column sum in FP32, the sums added into FP64.  For a correction d that is
 // small against the solution (|d| ~ 1e-3 |x| after the first), FP32 products put errors of ~1e-10 of
 // |A x| into the residual r - M d, far below what the refinement converges to.
+// The complex64 vectors of the refinement are kept by column pairs, [F][pairs][Np] of {re, re', im, im'}, so that a
+// 16-byte load of shared memory feeds the packed FMAs of two columns as it is.
 template <int NR>
 __host__ __device__ constexpr size_t gv32_tx_bytes() {
-    return (size_t)2 * GV_COLS * GV_ROWS * 4 + (size_t)NR * GV_COLS * 8;
+    return (size_t)2 * GV_COLS * GV_ROWS * 4 + (size_t)(NR / 2) * GV_COLS * 16;
 }
 template <int NR>
 __host__ __device__ constexpr size_t gv32_stage_bytes() {
@@ -1024,7 +1028,7 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
                 tc::mbar_arrive_expect_tx(&full[s], (uint32_t)gv32_tx_bytes<NR>());
                 tc::tma_load_4d(st, &mapM, &full[s], k0, n0, 0, f);
                 tc::tma_load_4d(st + GV_COLS * GV_ROWS * 4, &mapM, &full[s], k0, n0, 1, f);
-                tc::tma_load_4d(st + 2 * GV_COLS * GV_ROWS * 4, &mapD, &full[s], 2 * n0, c0, f, 0);
+                tc::tma_load_4d(st + 2 * GV_COLS * GV_ROWS * 4, &mapD, &full[s], 4 * n0, c0 / 2, f, 0);
             }
         }
         return;
@@ -1042,33 +1046,34 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
         const uint8_t* st = base + s * gv32_stage_bytes<NR>();
         const float* sMr = reinterpret_cast<const float*>(st);
         const float* sMi = sMr + GV_COLS * GV_ROWS;
-        const float2* sd = reinterpret_cast<const float2*>(st + 2 * GV_COLS * GV_ROWS * 4);  // [NR][GV_COLS]
+        const float4* sd = reinterpret_cast<const float4*>(st + 2 * GV_COLS * GV_ROWS * 4);  // [NR / 2][GV_COLS]
         const int lim = min(GV_COLS, nend - (nbeg + si * GV_COLS));
-        f32x2 a0[NR], a1[NR];
+        f32x2 r0[NR / 2], i0[NR / 2], r1[NR / 2], i1[NR / 2];
 #pragma unroll
-        for (int c = 0; c < NR; c++) a0[c] = a1[c] = f2pack(0.f, 0.f);
+        for (int c = 0; c < NR / 2; c++) r0[c] = i0[c] = r1[c] = i1[c] = f2pack(0.f, 0.f);
 #pragma unroll 4
         for (int j = 0; j < lim; j++) {
             const float mr = sMr[j * GV_ROWS + t], mi = sMi[j * GV_ROWS + t];
             const float nr = sMr[j * GV_ROWS + t + GV_WORKERS], ni = sMi[j * GV_ROWS + t + GV_WORKERS];
-            const f32x2 m0 = f2pack(mr, mr), q0 = f2pack(-mi, mi), m1 = f2pack(nr, nr), q1 = f2pack(-ni, ni);
+            const f32x2 a0 = f2pack(mr, mr), b0 = f2pack(mi, mi), e0 = f2pack(-mi, -mi);
+            const f32x2 a1 = f2pack(nr, nr), b1 = f2pack(ni, ni), e1 = f2pack(-ni, -ni);
 #pragma unroll
-            for (int c = 0; c < NR; c++) {
-                const float2 v = sd[c * GV_COLS + j];
-                const f32x2 vv = f2pack(v.x, v.y), vs = f2pack(v.y, v.x);
-                a0[c] = ffma2(m0, vv, a0[c]);
-                a0[c] = ffma2(q0, vs, a0[c]);
-                a1[c] = ffma2(m1, vv, a1[c]);
-                a1[c] = ffma2(q1, vs, a1[c]);
+            for (int c = 0; c < NR / 2; c++) {
+                const float4 v = sd[c * GV_COLS + j];
+                const f32x2 vr = f2pack(v.x, v.y), vi = f2pack(v.z, v.w);
+                r0[c] = ffma2(e0, vi, ffma2(a0, vr, r0[c]));
+                i0[c] = ffma2(b0, vr, ffma2(a0, vi, i0[c]));
+                r1[c] = ffma2(e1, vi, ffma2(a1, vr, r1[c]));
+                i1[c] = ffma2(b1, vr, ffma2(a1, vi, i1[c]));
             }
         }
 #pragma unroll
         for (int c = 0; c < NR; c++) {
-            const float2 u0 = f2unpack(a0[c]), u1 = f2unpack(a1[c]);
-            acc[c].x += (double)u0.x;
-            acc[c].y += (double)u0.y;
-            acd[c].x += (double)u1.x;
-            acd[c].y += (double)u1.y;
+            const float2 x0 = f2unpack(r0[c / 2]), y0 = f2unpack(i0[c / 2]), x1 = f2unpack(r1[c / 2]), y1 = f2unpack(i1[c / 2]);
+            acc[c].x += (double)(c & 1 ? x0.y : x0.x);
+            acc[c].y += (double)(c & 1 ? y0.y : y0.x);
+            acd[c].x += (double)(c & 1 ? x1.y : x1.x);
+            acd[c].y += (double)(c & 1 ? y1.y : y1.x);
         }
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&empty[s]);
@@ -1082,23 +1087,9 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
         }
 }
 
-template <class T>
-__device__ __forceinline__ T make_out(double x, double y);
-template <>
-__device__ __forceinline__ double2 make_out<double2>(double x, double y) {
-    return make_double2(x, y);
-}
-template <>
-__device__ __forceinline__ float2 make_out<float2>(double x, double y) {
-    return make_float2((float)x, (float)y);
-}
-
-__device__ __forceinline__ double2 to_d2(double2 v) { return v; }
-__device__ __forceinline__ double2 to_d2(float2 v) { return make_double2((double)v.x, (double)v.y); }
-
-template <class T, class BT = double2>
+// out = bias - sum of the partial products (fixed order), FP64 [F][nrhs][ldo]
 __global__ void k_gemv_reduce(int N, int nrhs, int F, int nz, const double2* __restrict__ part,
-                              const BT* __restrict__ bias, int ldb, T* __restrict__ out, int ldo) {
+                              const double2* __restrict__ bias, int ldb, double2* __restrict__ out, int ldo) {
     const int f = blockIdx.y;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (size_t)nrhs * N) return;
@@ -1109,186 +1100,75 @@ __global__ void k_gemv_reduce(int N, int nrhs, int F, int nz, const double2* __r
         sr += v.x;
         si += v.y;
     }
-    double2 b = bias ? to_d2(bias[((size_t)f * nrhs + c) * ldb + k]) : make_double2(0.0, 0.0);
-    out[((size_t)f * nrhs + c) * ldo + k] = make_out<T>(b.x - sr, b.y - si);
+    double2 b = bias ? bias[((size_t)f * nrhs + c) * ldb + k] : make_double2(0.0, 0.0);
+    out[((size_t)f * nrhs + c) * ldo + k] = make_double2(b.x - sr, b.y - si);
+}
+
+// The residual bias - sum of the partial products as complex64 column pairs; the bias is FP64 [F][nrhs][Np]
+// (the right-hand sides) or, PAIRS, the residual before the correction in the pairs' layout.
+template <bool PAIRS>
+__global__ void k_residual_reduce(int N, int Np, int nrhs, int F, int nz, const double2* __restrict__ part,
+                                  const void* __restrict__ bias, float4* __restrict__ out) {
+    const int f = blockIdx.y, np = (nrhs + 1) / 2;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (size_t)np * N) return;
+    const int q = (int)(t / N), k = (int)(t % N);
+    const size_t o = ((size_t)f * np + q) * Np + k;
+    double2 v[2];
+    float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (PAIRS) b4 = static_cast<const float4*>(bias)[o];
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const int c = 2 * q + e;
+        v[e] = make_double2(0.0, 0.0);
+        if (c >= nrhs) continue;
+        double sr = 0.0, si = 0.0;
+        for (int z = 0; z < nz; z++) {
+            const double2 p = part[(((size_t)z * F + f) * nrhs + c) * N + k];
+            sr += p.x;
+            si += p.y;
+        }
+        const double2 b = PAIRS ? make_double2((double)(e ? b4.y : b4.x), (double)(e ? b4.w : b4.z))
+                                : static_cast<const double2*>(bias)[((size_t)f * nrhs + c) * Np + k];
+        v[e] = make_double2(b.x - sr, b.y - si);
+    }
+    out[o] = make_float4((float)v[0].x, (float)v[1].x, (float)v[0].y, (float)v[1].y);
 }
 
 // d = A^-1 r with the factors of M = A^T = L U (FP32 planar, row-major in W): U^T y = r, then
 // L^T d = y, in FP32 (the correction only needs the accuracy of the TF32 factors; the residual that
-// sets the attainable accuracy is formed in FP64), vectors [F][nrhs][Np] complex64 in place, in
-// blocks of TB = 128 rows.  One launch per block step: every CTA of the step owns 128 rows and
-// subtracts the contribution of the block solved by the previous step (row s0 + p of W read along
-// its rows: coalesced); the CTA that owns the next diagonal block then solves it by the stored
-// inverse of that block.
+// sets the attainable accuracy is formed in FP64), complex64 column pairs in place, in blocks of TB = 128 rows:
+// one persistent launch a direction.  The columns are split into groups that are solved independently, v = (matrix,
+// group) the systems; the work items are (k, v), block k in solve order of system v, handed out by a ticket counter in
+// the order k nv + v.  An item streams the block row of the factor against the blocks 0 .. k-1 as their solutions
+// are published (ctrl[1 + v] = blocks of system v done), subtracts the sum, solves its diagonal block by the
+// stored inverse and publishes it.  An item waits only on items of smaller ticket, which running CTAs
+// hold and work on in order, so the sweep cannot deadlock; every wait is bounded (error 8: from then on nothing
+// waits, the results are discarded).  ctrl = [ticket, done[nv]], zero at launch.
+//
+// One CTA an SM.  Warp 8 takes the tickets and streams the factor by TMA (32 rows of the solved block x 128 rows, both
+// planes, 32 KB a stage) without waiting for solutions, the item's diagonal inverse after its last block and then the
+// next item's blocks; warp 9 waits for the solutions and copies them (cp.async) beside them; warps 0 .. 7 multiply:
+// four rows a lane, a part of each stage's k and (KS = 4) half of the column pairs a warp, so that one 16-byte load
+// of a pair's solution feeds 16 packed FMAs and the k-parts are summed through shared memory only at an item's end.
+// A chain step is the last block's product, the diagonal's product (each 0.52 us a column pair on one SM's FP32 pipe)
+// and about 6 us of waiting, copying and summing; the whole is bound by the chain with few matrices and by the FP32 pipe with
+// many.  A sweep measured, ms before / now: 40 matrices of order 4096, 10 columns 1.31 / 0.72; 4 of order 12288, 19
+// columns 4.4 / 1.42; 5 of order 18560, 14 columns 7.2 / 3.2.  What it replaces (two rows a thread, the factor loaded into registers after the wait, one CTA doing
+// everything in turn) spent 25-45 us a chain step, its shared-memory loads twice the FMAs' time.
 constexpr int TB = 128;
-constexpr int TRI_THREADS = 256;
-
-
-// The diagonal block of U^T (upper_t) or L^T, solved by its stored inverse: y_b = D^T r_b with
-// D = U_bb^-1 (upper part of the stored block, with the diagonal) or L_bb^-1 (lower part, unit
-// diagonal).  Rows b0..b0+TB of X in place, right-hand sides in chunks of NR.  Thread t < TB owns
-// column t for the first half of the block's rows, thread t + TB the same column for the second
-// half; each loads the 16 entries of a chunk before using them (one memory latency per chunk).
-template <int NR>
-__device__ __forceinline__ void tri_diag_f32(const float2* __restrict__ D, float2* X, int Np, int nrhs, int b0,
-                                             bool upper_t, float4 (*rs)[NR], float2 (*pt)[NR]) {
-    const int i = threadIdx.x % TB, half = threadIdx.x / TB;
-    for (int c0 = 0; c0 < nrhs; c0 += NR) {
-        const int nc = min(NR, nrhs - c0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < TB * NR; t += blockDim.x) {
-            const int p = t % TB, c = t / TB;
-            rs[p][c] = dup_swap(c < nc ? X[(size_t)(c0 + c) * Np + b0 + p] : make_float2(0.f, 0.f));
-        }
-        __syncthreads();
-        f32x2 acc[NR];
-#pragma unroll
-        for (int c = 0; c < NR; c++)  // the unit diagonal of L^-1
-            acc[c] = (!upper_t && half == (i >= TB / 2 ? 1 : 0)) ? f2pack(rs[i][c].x, rs[i][c].y) : f2pack(0.f, 0.f);
-        const int pb = half * (TB / 2);
-#pragma unroll 1
-        for (int pc = 0; pc < TB / 2; pc += 16) {
-            // the chunk's rows p = pb + pc .. + 15 that this row uses (p <= i for U^-1, p > i for L^-1):
-            // none, and its loads are skipped (half of the triangle's inverse is zero)
-            const int p0 = pb + pc;
-            if (upper_t ? p0 > i : p0 + 15 <= i) continue;
-            float2 dv[16];
-#pragma unroll
-            for (int q = 0; q < 16; q++) dv[q] = D[(pb + pc + q) * TB + i];
-#pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int p = pb + pc + q;
-                if (upper_t ? p <= i : p > i) {
-                    const f32x2 m = f2pack(dv[q].x, dv[q].x), mn = f2pack(-dv[q].y, dv[q].y);
-#pragma unroll
-                    for (int c = 0; c < NR; c++) {
-                        const float4 v = rs[p][c];
-                        acc[c] = ffma2(m, f2pack(v.x, v.y), acc[c]);
-                        acc[c] = ffma2(mn, f2pack(v.z, v.w), acc[c]);
-                    }
-                }
-            }
-        }
-        if (half == 1)
-#pragma unroll
-            for (int c = 0; c < NR; c++) pt[i][c] = f2unpack(acc[c]);
-        __syncthreads();
-        if (half == 0)
-#pragma unroll
-            for (int c = 0; c < NR; c++)
-                if (c < nc) {
-                    const float2 q2 = pt[i][c], a = f2unpack(acc[c]);
-                    X[(size_t)(c0 + c) * Np + b0 + i] = make_float2(a.x + q2.x, a.y + q2.y);
-                }
-    }
-}
-
-// One block step of the forward (upper_t) or backward solve.  step = index of the block solved by
-// the previous launch (-1: none, only the first diagonal block is solved).  Thread layout: warp w
-// owns rows 32 (w % 2) + lane and 64 more, and the quarter w / 2 of the solved block's 128
-// entries, loaded 16 at a time before use; every lane of a warp reads the same solved entry (a
-// shared-memory broadcast).
-template <int NR>
-__global__ void __launch_bounds__(TRI_THREADS, 2) k_tri_step(int Np, size_t bstride, const float* __restrict__ W,
-                                                          const float2* __restrict__ DINV, int nrhs,
-                                                          float2* __restrict__ Xall, int step, int upper_t) {
-    extern __shared__ float4 tri_smem4[];  // ys [TB][NR] as {re, im, im, re}, partial sums [3][TB][NR]
-    float4(*ys)[NR] = reinterpret_cast<float4(*)[NR]>(tri_smem4);
-    float2(*pt)[NR] = reinterpret_cast<float2(*)[NR]>(tri_smem4 + TB * NR);
-    const int f = blockIdx.y;
-    const float* Mr = W + (size_t)f * bstride;
-    const float* Mi = Mr + (size_t)Np * Np;
-    float2* X = Xall + (size_t)f * nrhs * Np;
-    const int nblk = Np / TB;
-    const float2* Df = DINV + (size_t)f * nblk * TB * TB;
-    if (step < 0) {
-        const int first = upper_t ? 0 : nblk - 1;
-        tri_diag_f32<NR>(Df + (size_t)first * TB * TB, X, Np, nrhs, first * TB, upper_t, ys, pt);
-        return;
-    }
-    const int s0 = step * TB;
-    const int cb = upper_t ? step + 1 + blockIdx.x : step - 1 - blockIdx.x;
-    const int r0 = cb * TB;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int li = 32 * (warp & 1) + lane;  // local rows li and li + 64
-    const int pq = warp >> 1;               // quarter of the solved block
-    const float* pr = Mr + (size_t)(s0 + pq * 32) * Np + r0 + li;
-    const float* pi = Mi + (size_t)(s0 + pq * 32) * Np + r0 + li;
-    for (int c0 = 0; c0 < nrhs; c0 += NR) {
-        const int nc = min(NR, nrhs - c0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < TB * NR; t += blockDim.x) {
-            const int p = t % TB, c = t / TB;
-            ys[p][c] = dup_swap(c < nc ? X[(size_t)(c0 + c) * Np + s0 + p] : make_float2(0.f, 0.f));
-        }
-        __syncthreads();
-        f32x2 a0[NR], a1[NR];
-#pragma unroll
-        for (int c = 0; c < NR; c++) a0[c] = a1[c] = f2pack(0.f, 0.f);
-#pragma unroll 1
-        for (int pc = 0; pc < 32; pc += 16) {
-            float r0v[16], i0v[16], r1v[16], i1v[16];
-#pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const size_t o = (size_t)(pc + q) * Np;
-                r0v[q] = pr[o];
-                i0v[q] = pi[o];
-                r1v[q] = pr[o + 64];
-                i1v[q] = pi[o + 64];
-            }
-#pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const f32x2 m0 = f2pack(r0v[q], r0v[q]), n0 = f2pack(-i0v[q], i0v[q]);
-                const f32x2 m1 = f2pack(r1v[q], r1v[q]), n1 = f2pack(-i1v[q], i1v[q]);
-#pragma unroll
-                for (int c = 0; c < NR; c++) {
-                    const float4 v4 = ys[pq * 32 + pc + q][c];
-                    const f32x2 v = f2pack(v4.x, v4.y), vs = f2pack(v4.z, v4.w);
-                    a0[c] = ffma2(m0, v, a0[c]);
-                    a0[c] = ffma2(n0, vs, a0[c]);
-                    a1[c] = ffma2(m1, v, a1[c]);
-                    a1[c] = ffma2(n1, vs, a1[c]);
-                }
-            }
-        }
-        if (pq > 0)
-#pragma unroll
-            for (int c = 0; c < NR; c++) {
-                pt[(pq - 1) * TB + li][c] = f2unpack(a0[c]);
-                pt[(pq - 1) * TB + li + 64][c] = f2unpack(a1[c]);
-            }
-        __syncthreads();
-        if (pq == 0)
-#pragma unroll
-            for (int c = 0; c < NR; c++)
-                if (c < nc) {
-                    float2 s0v = f2unpack(a0[c]), s1v = f2unpack(a1[c]);
-#pragma unroll
-                    for (int h = 0; h < 3; h++) {
-                        const float2 q0 = pt[h * TB + li][c], q1 = pt[h * TB + li + 64][c];
-                        s0v.x += q0.x;
-                        s0v.y += q0.y;
-                        s1v.x += q1.x;
-                        s1v.y += q1.y;
-                    }
-                    float2* x0 = X + (size_t)(c0 + c) * Np + r0 + li;
-                    const float2 v0 = x0[0], v1 = x0[64];
-                    x0[0] = make_float2(v0.x - s0v.x, v0.y - s0v.y);
-                    x0[64] = make_float2(v1.x - s1v.x, v1.y - s1v.y);
-                }
-    }
-    if (blockIdx.x == 0) tri_diag_f32<NR>(Df + (size_t)cb * TB * TB, X, Np, nrhs, r0, upper_t, ys, pt);
-}
-
-constexpr size_t tri_smem_bytes(int nr) { return (size_t)TB * nr * (sizeof(float4) + 3 * sizeof(float2)); }
-
-// The same solve as one persistent launch per direction (up to NR right-hand sides): the work items
-// are (k, f), block k in solve order of matrix f, handed out by a ticket counter in the order
-// k nb + f.  An item streams the block row of the factor against the blocks 0 .. k-1 as their
-// solutions are published (ctrl[1 + f] = blocks of matrix f done), subtracts the sum, solves its
-// diagonal block by the stored inverse and publishes it.  An item waits only on items of smaller
-// ticket, which running CTAs hold, so the sweep cannot deadlock; every wait is bounded (error 8).
-// ctrl = [ticket, done[nb]], zero at launch.
+constexpr int TRI_THREADS = 320, TRI_SK = 32;  // k rows of a stage
+constexpr size_t TRI_STAGE = (size_t)2 * TRI_SK * TB * 4;
+template <int NQ>  // column pairs of a group
+struct TriCfg {
+    static constexpr int KS = NQ <= 5 ? 8 : 4, NH = KS == 8 ? NQ : NQ / 2;  // k-parts, pairs of a warp
+    static constexpr int NST = NQ <= 4 ? 4 : 3;                             // factor stages
+    static constexpr size_t VEC = (size_t)NQ * TB * 16;                     // one block's vectors
+    static constexpr size_t SMEM = 1024 + NST * TRI_STAGE + (2 + 1 + KS) * VEC + 256;
+    static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
+    static_assert(NH * 8 / KS == NQ, "the warps cover the pairs");
+};
+constexpr int TRI_MAXQ = 8;  // pairs of a group, at most
 constexpr uint32_t TRI_WAIT_LIMIT = 1u << 20;
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
@@ -1299,163 +1179,298 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
 __device__ __forceinline__ void st_release_gpu(int* p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ void cp_async_f4(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(smem)), "l"(gmem) : "memory");
+}
+// this thread's arrival on the barrier once its cp.async so far have landed
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
+}
 
-template <int NR>
-__global__ void __launch_bounds__(TRI_THREADS, NR > 16 ? 1 : 2) k_tri_sweep(int Np, size_t bstride, const float* __restrict__ W,
-                                                           const float2* __restrict__ DINV, int nrhs,
-                                                           float2* __restrict__ Xall, int nb, int upper_t,
-                                                           int* __restrict__ ctrl, int* __restrict__ err) {
-    extern __shared__ float4 tri_smem4[];  // ys [TB][NR] as {re, im, im, re}, partial sums [3][TB][NR]
-    float4(*ys)[NR] = reinterpret_cast<float4(*)[NR]>(tri_smem4);
-    float2(*pt)[NR] = reinterpret_cast<float2(*)[NR]>(tri_smem4 + TB * NR);
-    __shared__ int s_item, s_stop;
-    const int nblk = Np / TB, items = nblk * nb;
+// acc (4 rows x NH pairs, real and imaginary sums) += the warp's k-part of a stage times the vectors at v
+// ([pair][128], from the stage's first k on); MASK: the diagonal inverse, of which entry (p, row) counts where
+// p <= row (upper) or p > row
+template <int KS, int NH, bool MASK>
+__device__ __forceinline__ void tri_stage(const float* sF, const float4* v, int k0, int lane, int p0, bool upper,
+                                          f32x2 (&ar)[4][NH], f32x2 (&ai)[4][NH]) {
+#pragma unroll(NH <= 5 ? 4 : 2)
+    for (int kk = 0; kk < TRI_SK / KS; kk++) {
+        const int k = k0 + kk;
+        float4 fr = *reinterpret_cast<const float4*>(sF + k * TB + 4 * lane);
+        float4 fi = *reinterpret_cast<const float4*>(sF + (TRI_SK + k) * TB + 4 * lane);
+        if (MASK) {
+            const int p = p0 + k, r = 4 * lane;
+            if (upper != (p <= r)) fr.x = fi.x = 0.f;
+            if (upper != (p <= r + 1)) fr.y = fi.y = 0.f;
+            if (upper != (p <= r + 2)) fr.z = fi.z = 0.f;
+            if (upper != (p <= r + 3)) fr.w = fi.w = 0.f;
+        }
+        const float fre[4] = {fr.x, fr.y, fr.z, fr.w}, fim[4] = {fi.x, fi.y, fi.z, fi.w};
+#pragma unroll
+        for (int c = 0; c < NH; c++) {
+            const float4 y = v[c * TB + k];
+            const f32x2 yr = f2pack(y.x, y.y), yi = f2pack(y.z, y.w);
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const f32x2 a = f2pack(fre[r], fre[r]), b = f2pack(fim[r], fim[r]), bn = f2pack(-fim[r], -fim[r]);
+                ar[r][c] = ffma2(bn, yi, ffma2(a, yr, ar[r][c]));
+                ai[r][c] = ffma2(b, yr, ffma2(a, yi, ai[r][c]));
+            }
+        }
+    }
+}
+
+template <int NQ>
+__global__ void __launch_bounds__(TRI_THREADS, 1) k_tri_sweep(const __grid_constant__ CUtensorMap mapF,
+                                                              const __grid_constant__ CUtensorMap mapD, int Np,
+                                                              int npair, float4* __restrict__ Xall, int nb, int ngroup,
+                                                              int upper_t,
+                                                              int* __restrict__ ctrl, int* __restrict__ err) {
+    using C = TriCfg<NQ>;
+    constexpr int NH = C::NH, KS = C::KS, NYB = 2;
+    extern __shared__ uint8_t tri_raw[];
+    uint8_t* base = align1024(tri_raw);
+    float4* ys = reinterpret_cast<float4*>(base + C::NST * TRI_STAGE);  // [NYB][NQ][TB]
+    float4* rb = ys + NYB * NQ * TB;                              // [NQ][TB]: the item's right-hand side
+    float4* pt = rb + NQ * TB;                                       // [KS][NQ][TB]: partial sums
+    uint64_t* full = reinterpret_cast<uint64_t*>(pt + KS * NQ * TB);
+    uint64_t* empty = full + C::NST;
+    uint64_t* yfull = empty + C::NST;
+    uint64_t* yempty = yfull + NYB;
+    uint64_t* rfull = yempty + NYB;  // then rempty, the item ring's full[2] and empty[2]
+    uint64_t* rempty = rfull + 1;
+    uint64_t* ifull = rempty + 1;
+    uint64_t* iempty = ifull + 2;
+    int* s_item = reinterpret_cast<int*>(iempty + 2);  // [2]
+    const int nblk = Np / TB, nv = nb * ngroup, items = nblk * nv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int li = 32 * (warp & 1) + lane;  // local rows li and li + 64
-    const int pq = warp >> 1;               // quarter of each solved block
-    for (;;) {
-        __syncthreads();  // the previous item's shared data consumed
-        if (threadIdx.x == 0) s_item = atomicAdd(ctrl, 1);
-        __syncthreads();
-        const int t = s_item;
-        if (t >= items) return;
-        const int k = t / nb, f = t % nb;
-        const int r0 = (upper_t ? k : nblk - 1 - k) * TB;
-        const float* Mr = W + (size_t)f * bstride;
-        const float* Mi = Mr + (size_t)Np * Np;
-        float2* X = Xall + (size_t)f * nrhs * Np;
-        int* done = ctrl + 1 + f;
-        f32x2 a0[NR], a1[NR];
-#pragma unroll
-        for (int c = 0; c < NR; c++) a0[c] = a1[c] = f2pack(0.f, 0.f);
-#pragma unroll 1
-        for (int kk = 0; kk < k; kk++) {
-            const int s0 = (upper_t ? kk : nblk - 1 - kk) * TB;
-            if (threadIdx.x == 0) {
-                int stop = 0;
-                uint32_t n = 0;
-                while (ld_acquire_gpu(done) <= kk) {
-                    if (*(volatile int*)err != 0) {
-                        stop = 1;
-                        break;
-                    }
-                    if (++n > TRI_WAIT_LIMIT) {
-                        atomicExch(err, 8);
-                        stop = 1;
-                        break;
-                    }
-                    __nanosleep(64);
-                }
-                s_stop = stop;
-            }
-            __syncthreads();
-            if (s_stop) return;
-            // the solved block (written by another CTA: read through L2)
-            for (int tt = threadIdx.x; tt < TB * NR; tt += blockDim.x) {
-                const int p = tt % TB, c = tt / TB;
-                ys[p][c] = dup_swap(c < nrhs ? __ldcg(X + (size_t)c * Np + s0 + p) : make_float2(0.f, 0.f));
-            }
-            __syncthreads();
-            const float* pr = Mr + (size_t)(s0 + pq * 32) * Np + r0 + li;
-            const float* pi = Mi + (size_t)(s0 + pq * 32) * Np + r0 + li;
-#pragma unroll 1
-            for (int pc = 0; pc < 32; pc += 16) {
-                float r0v[16], i0v[16], r1v[16], i1v[16];
-#pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const size_t o = (size_t)(pc + q) * Np;
-                    r0v[q] = __ldg(pr + o);
-                    i0v[q] = __ldg(pi + o);
-                    r1v[q] = __ldg(pr + o + 64);
-                    i1v[q] = __ldg(pi + o + 64);
-                }
-#pragma unroll
-                for (int q = 0; q < 16; q++) {
-                    const f32x2 m0 = f2pack(r0v[q], r0v[q]), n0 = f2pack(-i0v[q], i0v[q]);
-                    const f32x2 m1 = f2pack(r1v[q], r1v[q]), n1 = f2pack(-i1v[q], i1v[q]);
-#pragma unroll
-                    for (int c = 0; c < NR; c++) {
-                        const float4 v4 = ys[pq * 32 + pc + q][c];
-                        const f32x2 v = f2pack(v4.x, v4.y), vs = f2pack(v4.z, v4.w);
-                        a0[c] = ffma2(m0, v, a0[c]);
-                        a0[c] = ffma2(n0, vs, a0[c]);
-                        a1[c] = ffma2(m1, v, a1[c]);
-                        a1[c] = ffma2(n1, vs, a1[c]);
-                    }
-                }
-            }
-            __syncthreads();  // ys read by every warp before the next block overwrites it
-        }
-        if (k > 0) {
-            if (pq > 0)
-#pragma unroll
-                for (int c = 0; c < NR; c++) {
-                    pt[(pq - 1) * TB + li][c] = f2unpack(a0[c]);
-                    pt[(pq - 1) * TB + li + 64][c] = f2unpack(a1[c]);
-                }
-            __syncthreads();
-            if (pq == 0)
-#pragma unroll
-                for (int c = 0; c < NR; c++)
-                    if (c < nrhs) {
-                        float2 s0v = f2unpack(a0[c]), s1v = f2unpack(a1[c]);
-#pragma unroll
-                        for (int h = 0; h < 3; h++) {
-                            const float2 q0 = pt[h * TB + li][c], q1 = pt[h * TB + li + 64][c];
-                            s0v.x += q0.x;
-                            s0v.y += q0.y;
-                            s1v.x += q1.x;
-                            s1v.y += q1.y;
-                        }
-                        float2* x0 = X + (size_t)c * Np + r0 + li;
-                        const float2 v0 = x0[0], v1 = x0[64];
-                        x0[0] = make_float2(v0.x - s0v.x, v0.y - s0v.y);
-                        x0[64] = make_float2(v1.x - s1v.x, v1.y - s1v.y);
-                    }
-        }
-        tri_diag_f32<NR>(DINV + ((size_t)f * nblk + r0 / TB) * TB * TB, X, Np, nrhs, r0, upper_t, ys, pt);
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) st_release_gpu(done, k + 1);
-    }
-}
-
-// FP64 vectors to complex64 (the right-hand sides entering the first correction).
-__global__ void k_to_c64(size_t n, const double2* __restrict__ a, float2* __restrict__ b) {
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-        b[t] = make_float2((float)a[t].x, (float)a[t].y);
-}
-
-// x += d; per matrix the largest |d| and |x| (for the refinement's stopping test), [F][2].
-__global__ void k_ir_update(int Np, int nrhs, double2* __restrict__ x, const float2* __restrict__ d,
-                            double* __restrict__ norms) {
-    __shared__ double sd[256], sx[256];
-    const int f = blockIdx.x;
-    const size_t n = (size_t)nrhs * Np;
-    double md = 0.0, mx = 0.0;
-    for (size_t t = threadIdx.x; t < n; t += blockDim.x) {
-        size_t o = (size_t)f * n + t;
-        double2 a = x[o];
-        const float2 b = d[o];
-        a.x += (double)b.x;
-        a.y += (double)b.y;
-        x[o] = a;
-        md = fmax(md, fmax(fabs((double)b.x), fabs((double)b.y)));
-        mx = fmax(mx, fmax(fabs(a.x), fabs(a.y)));
-    }
-    sd[threadIdx.x] = md;
-    sx[threadIdx.x] = mx;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            sd[threadIdx.x] = fmax(sd[threadIdx.x], sd[threadIdx.x + s]);
-            sx[threadIdx.x] = fmax(sx[threadIdx.x], sx[threadIdx.x + s]);
-        }
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
-        norms[2 * f] = sd[0];
-        norms[2 * f + 1] = sx[0];
+        for (int i = 0; i < C::NST; i++) {
+            tc::mbar_init(&full[i], 1);
+            tc::mbar_init(&empty[i], 8);
+        }
+        for (int i = 0; i < NYB; i++) {
+            tc::mbar_init(&yfull[i], 32);
+            tc::mbar_init(&yempty[i], 8);
+        }
+        tc::mbar_init(rfull, 32);
+        tc::mbar_init(rempty, 8);
+        for (int i = 0; i < 2; i++) {
+            tc::mbar_init(&ifull[i], 1);
+            tc::mbar_init(&iempty[i], 9);
+        }
+        tc::fence_barrier_init();
+    }
+    // a last group's missing pairs stay zero
+    for (int t = threadIdx.x; t < (NYB + 1) * NQ * TB; t += TRI_THREADS) ys[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    auto wait = [&](uint64_t* bar, uint32_t parity) {  // bounded; after an error the protocol runs on, its results discarded
+        if (!tc::mbar_wait(bar, parity)) atomicExch(err, 8);
+    };
+    if (warp == 8) {
+        if (lane == 0) {
+            tc::prefetch_tensormap(&mapF);
+            tc::prefetch_tensormap(&mapD);
+            int st = 0;  // stages issued
+            for (int n = 0;; n++) {
+                if (n >= 2) wait(&iempty[n & 1], ((n >> 1) - 1) & 1);
+                const int t = atomicAdd(ctrl, 1);
+                s_item[n & 1] = t;
+                tc::mbar_arrive(&ifull[n & 1]);
+                if (t >= items) break;
+                const int k = t / nv, f = t % nv / ngroup, blk = upper_t ? k : nblk - 1 - k;
+                for (int q = 0; q < 4 * (k + 1); q++, st++) {
+                    const int s = st % C::NST, kk = q >> 2, sub = q & 3;
+                    if (st >= C::NST) wait(&empty[s], ((st / C::NST) - 1) & 1);
+                    tc::mbar_arrive_expect_tx(&full[s], (uint32_t)TRI_STAGE);
+                    uint8_t* d = base + s * TRI_STAGE;
+                    for (int p = 0; p < 2; p++)
+                        if (kk < k)
+                            tc::tma_load_4d(d + p * (TRI_STAGE / 2), &mapF, &full[s], blk * TB,
+                                            (upper_t ? kk : nblk - 1 - kk) * TB + sub * TRI_SK, p, f);
+                        else
+                            tc::tma_load_4d(d + p * (TRI_STAGE / 2), &mapD, &full[s], 0, sub * TRI_SK, p, f * nblk + blk);
+                }
+            }
+        }
+    } else if (warp == 9) {
+        int yb = 0;  // solutions loaded
+        for (int n = 0;; n++) {
+            wait(&ifull[n & 1], (n >> 1) & 1);
+            const int t = s_item[n & 1];
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&iempty[n & 1]);
+            if (t >= items) break;
+            const int k = t / nv, v = t % nv, f = v / ngroup, p0 = (v % ngroup) * NQ, nq = min(NQ, npair - p0);
+            const int blk = upper_t ? k : nblk - 1 - k;
+            const float4* X = Xall + ((size_t)f * npair + p0) * Np;
+            const int* done = ctrl + 1 + v;
+            if (n > 0) wait(rempty, (n - 1) & 1);
+            for (int q = 0; q < nq; q++)
+#pragma unroll
+                for (int e = 0; e < TB / 32; e++)
+                    cp_async_f4(rb + q * TB + 32 * e + lane, X + (size_t)q * Np + blk * TB + 32 * e + lane);
+            cp_async_arrive(rfull);
+            int have = 0;
+            for (int kk = 0; kk < k; kk++, yb++) {
+                const int b = yb % NYB;
+                if (yb >= NYB) wait(&yempty[b], ((yb / NYB) - 1) & 1);
+                if (have <= kk) {
+                    if (lane == 0) {
+                        uint32_t polls = 0;
+                        while ((have = ld_acquire_gpu(done)) <= kk && *(volatile int*)err == 0)
+                            if (++polls > TRI_WAIT_LIMIT) atomicExch(err, 8);
+                    }
+                    __syncwarp();
+                    have = __shfl_sync(0xffffffffu, have, 0);
+                }
+                const float4* xs = X + (size_t)(upper_t ? kk : nblk - 1 - kk) * TB;
+                float4* yd = ys + b * NQ * TB;
+                for (int q = 0; q < nq; q++)
+#pragma unroll
+                    for (int e = 0; e < TB / 32; e++)
+                        cp_async_f4(yd + q * TB + 32 * e + lane, xs + (size_t)q * Np + 32 * e + lane);
+                cp_async_arrive(&yfull[b]);
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+        const int ks = warp % KS, k0 = ks * (TRI_SK / KS), q0 = warp / KS * NH;  // first k of a stage, first pair
+        f32x2 ar[4][NH], ai[4][NH];
+        auto clear = [&]() {
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int c = 0; c < NH; c++) ar[r][c] = ai[r][c] = f2pack(0.f, 0.f);
+        };
+        auto barrier = [&]() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+        // the k-parts' sums, each thread its entries (pair q, row) passed to put
+        auto reduce = [&](auto put) {
+#pragma unroll
+            for (int c = 0; c < NH; c++)
+#pragma unroll
+                for (int r = 0; r < 4; r++) {  // (row 4 lane + r at 32 r + lane: consecutive 16-byte accesses)
+                    const float2 a = f2unpack(ar[r][c]), b = f2unpack(ai[r][c]);
+                    pt[(ks * NQ + q0 + c) * TB + 32 * r + lane] = make_float4(a.x, a.y, b.x, b.y);
+                }
+            barrier();
+#pragma unroll
+            for (int e = threadIdx.x; e < NQ * TB; e += 256) {
+                float4 a = pt[e];
+#pragma unroll
+                for (int h = 1; h < KS; h++) {
+                    const float4 v = pt[h * NQ * TB + e];
+                    a = make_float4(a.x + v.x, a.y + v.y, a.z + v.z, a.w + v.w);
+                }
+                const int slot = e % TB;
+                put(e / TB, 4 * (slot % 32) + slot / 32, a);
+            }
+            barrier();  // the partial sums are consumed, the entries written
+        };
+        int st = 0, yb = 0;
+        for (int n = 0;; n++) {
+            wait(&ifull[n & 1], (n >> 1) & 1);
+            const int t = s_item[n & 1];
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&iempty[n & 1]);
+            if (t >= items) break;
+            const int k = t / nv, v = t % nv, f = v / ngroup, p0 = (v % ngroup) * NQ, nq = min(NQ, npair - p0);
+            const int blk = upper_t ? k : nblk - 1 - k;
+            clear();
+            for (int kk = 0; kk < k; kk++, yb++) {
+                const int b = yb % NYB;
+                wait(&yfull[b], (yb / NYB) & 1);
+                const float4* y = ys + (b * NQ + q0) * TB;
+#pragma unroll 1
+                for (int sub = 0; sub < 4; sub++, st++) {
+                    const int s = st % C::NST;
+                    wait(&full[s], (st / C::NST) & 1);
+                    tri_stage<KS, NH, false>(reinterpret_cast<const float*>(base + s * TRI_STAGE), y + sub * TRI_SK, k0, lane, 0,
+                                         false, ar, ai);
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&empty[s]);
+                }
+                if (lane == 0) tc::mbar_arrive(&yempty[b]);
+            }
+            wait(rfull, n & 1);
+            if (k > 0) {
+                reduce([&](int q, int row, float4 a) {
+                    float4& u = rb[q * TB + row];
+                    u = make_float4(u.x - a.x, u.y - a.y, u.z - a.z, u.w - a.w);
+                });
+                clear();
+            }
+#pragma unroll 1
+            for (int sub = 0; sub < 4; sub++, st++) {
+                const int s = st % C::NST;
+                wait(&full[s], (st / C::NST) & 1);
+                tri_stage<KS, NH, true>(reinterpret_cast<const float*>(base + s * TRI_STAGE), rb + q0 * TB + sub * TRI_SK, k0, lane,
+                                    sub * TRI_SK, upper_t != 0, ar, ai);
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&empty[s]);
+            }
+            float4* X = Xall + ((size_t)f * npair + p0) * Np + (size_t)blk * TB;
+            reduce([&](int q, int row, float4 a) {
+                if (!upper_t) {  // the unit diagonal of L^-1
+                    const float4 u = rb[q * TB + row];
+                    a = make_float4(a.x + u.x, a.y + u.y, a.z + u.z, a.w + u.w);
+                }
+                if (q < nq) X[(size_t)q * Np + row] = a;
+                __threadfence();
+            });
+            if (threadIdx.x == 0) st_release_gpu(ctrl + 1 + v, k + 1);
+            if (lane == 0) tc::mbar_arrive(rempty);
+        }
+    }
+}
+
+// FP64 right-hand sides to complex64 column pairs (entering the first correction).
+__global__ void k_to_pairs(int Np, int nrhs, const double2* __restrict__ b, float4* __restrict__ r) {
+    const int f = blockIdx.z, q = blockIdx.y, np = (nrhs + 1) / 2, k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= Np) return;
+    const double2 v0 = b[((size_t)f * nrhs + 2 * q) * Np + k];
+    const double2 v1 = 2 * q + 1 < nrhs ? b[((size_t)f * nrhs + 2 * q + 1) * Np + k] : make_double2(0.0, 0.0);
+    r[((size_t)f * np + q) * Np + k] = make_float4((float)v0.x, (float)v1.x, (float)v0.y, (float)v1.y);
+}
+
+// x += d; per matrix the largest |d| and |x| (for the refinement's stopping test) into norms [F][2], zero before
+// (bits of non-negative doubles order as the values do).  A CTA per 256 rows of a column pair: one CTA a matrix took
+// 94 us for 40 matrices of order 4096 and 10 columns.
+__global__ void __launch_bounds__(256) k_ir_update(int Np, int nrhs, double2* __restrict__ x, const float4* __restrict__ d,
+                                                   unsigned long long* __restrict__ norms) {
+    __shared__ double sd[8], sx[8];
+    const int f = blockIdx.z, q = blockIdx.y, np = (nrhs + 1) / 2, k = blockIdx.x * blockDim.x + threadIdx.x;
+    double md = 0.0, mx = 0.0;
+    if (k < Np) {
+        const float4 v = d[((size_t)f * np + q) * Np + k];
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+            if (2 * q + e < nrhs) {
+                const size_t o = ((size_t)f * nrhs + 2 * q + e) * Np + k;
+                const double dx = (double)(e ? v.y : v.x), dy = (double)(e ? v.w : v.z);
+                double2 a = x[o];
+                a.x += dx;
+                a.y += dy;
+                x[o] = a;
+                md = fmax(md, fmax(fabs(dx), fabs(dy)));
+                mx = fmax(mx, fmax(fabs(a.x), fabs(a.y)));
+            }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        md = fmax(md, __shfl_xor_sync(0xffffffffu, md, o));
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if ((threadIdx.x & 31) == 0) sd[threadIdx.x >> 5] = md, sx[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; w++) {
+            md = fmax(md, sd[w]);
+            mx = fmax(mx, sx[w]);
+        }
+        atomicMax(norms + 2 * f, (unsigned long long)__double_as_longlong(md));
+        atomicMax(norms + 2 * f + 1, (unsigned long long)__double_as_longlong(mx));
     }
 }
 

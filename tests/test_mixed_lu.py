@@ -31,9 +31,30 @@ def test_lu_block_edges(n_phi, n_z, n_r):
     assert all(b < 5e-3 * a for a, b in zip(hist, hist[1:])), hist
     # the potential is solved to the rounding of the complex64 matrix, relative to its modulus: A is its real
     # part, B / omega its imaginary part (which alone may be much smaller), on one scale
+    assert _complex_error(got, ref, omegas) <= 1e-5
+
+
+def _complex_error(got, ref, omegas):
+    """The largest error of A - i B / omega and of X against their entries' scales."""
     z, r = (np.asarray(q["A"]) - 1j * np.asarray(q["B"]) / omegas[:, None, None] for q in (got, ref))
-    scale = np.maximum(np.abs(r).max(axis=0, keepdims=True), 1e-3 * np.abs(r).max())
-    assert float((np.abs(z - r) / scale).max()) <= 1e-5
-    x, r = np.asarray(got["X"]), np.asarray(ref["X"])
-    scale = np.maximum(np.abs(r).max(axis=0, keepdims=True), 1e-3 * np.abs(r).max())
-    assert float((np.abs(x - r) / scale).max()) <= 1e-5
+    pairs = [(z, r)] + ([(np.asarray(got["X"]), np.asarray(ref["X"]))] if np.asarray(ref["X"]).size else [])
+    return max(float((np.abs(a - b) / np.maximum(np.abs(b).max(axis=0, keepdims=True), 1e-3 * np.abs(b).max())).max())
+               for a, b in pairs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("freqs,headings", [(1, 0), (2, 1), (3, 3), (64, 4), (96, 6), (96, 9), (5, 13), (150, 14), (40, 26)])
+def test_sweep_columns(freqs, headings):
+    """The triangular sweeps' column pairs (odd counts, a short last group) and group sizes, from one system, whose
+    columns are spread over the SMs, to many, which keep them together: 3 blocks of 128 rows, 380 panels."""
+    from hydrobem_b200 import native as nv
+
+    v = meshes.cylinder(1.0, 0.5, 20, 9, 10)
+    omegas = np.sqrt(np.linspace(0.4, 1.2, freqs) * meshes.GRAVITY)
+    heads = 7.0 * np.arange(headings)
+    ref = nv.solve(v, omegas, heads, depth=math.inf, precision=nv.HBG_FP64)
+    got = nv.solve(v, omegas, heads, depth=math.inf, precision=nv.HBG_MIXED)
+    assert nv.last_fallback_count() == 0
+    hist = nv.last_ir_history()
+    assert all(b < 5e-3 * a for a, b in zip(hist, hist[1:])), hist
+    assert _complex_error(got, ref, omegas) <= 1e-5
