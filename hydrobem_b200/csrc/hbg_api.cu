@@ -202,6 +202,7 @@ struct DeviceCtx {
     double* tables = nullptr;
     float* t2d_f = nullptr;
     float* t1d_f = nullptr;
+    float* t1d_j = nullptr;
     Tables tab{};
 };
 
@@ -249,7 +250,11 @@ static DeviceCtx& device_ctx(int dev) {
         }
     CUDA_OK(cudaMalloc(&d.t1d_f, t1f.size() * sizeof(float)));
     CUDA_OK(cudaMemcpy(d.t1d_f, t1f.data(), t1f.size() * sizeof(float), cudaMemcpyHostToDevice));
-    d.tab = Tables{dp[0], dp[1], dp[2], dp[3], dp[4], dp[5], dp[6], dp[7], d.t2d_f, d.t1d_f};
+    std::vector<float> t1j((size_t)XT * T1D_FN * 2);  // J0, J1 of it
+    for (size_t k = 0; k < t1j.size(); k++) t1j[k] = t1f[k / 2 * 4 + k % 2];
+    CUDA_OK(cudaMalloc(&d.t1d_j, t1j.size() * sizeof(float)));
+    CUDA_OK(cudaMemcpy(d.t1d_j, t1j.data(), t1j.size() * sizeof(float), cudaMemcpyHostToDevice));
+    d.tab = Tables{dp[0], dp[1], dp[2], dp[3], dp[4], dp[5], dp[6], dp[7], d.t2d_f, d.t1d_f, d.t1d_j};
     static double glx[17][16], glw[17][16];
     memset(glx, 0, sizeof glx);
     memset(glw, 0, sizeof glw);

@@ -46,6 +46,7 @@ struct Tables {
     const double* bk;    // scaled K0, K1 tiles
     const float* t2d_f;  // t2d rounded to FP32 (the mixed form's coefficient reads)
     const float* t1d_f;  // t1d rounded to FP32
+    const float* t1d_j;  // its J0, J1 alone (half the bytes of a gather)
 };
 
 // Panels in structure-of-arrays planes (each plane N doubles, plane p at base + p N).
@@ -320,6 +321,21 @@ __device__ inline void far_series(double X, double Y, double w, double& P, doubl
 template <bool F32 = false>
 __device__ inline void bessel_j01(double X, double& j0, double& j1) {
     if (X < XT) {
+        if constexpr (F32) {  // J0, J1 of table1d_f32, from their own table
+            const int i = (int)X;
+            const float t = (float)(2.0 * (X - i) - 1.0);
+            const float2* c = reinterpret_cast<const float2*>(c_tab.t1d_j) + i * T1D_FN;
+            float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+            for (int j = T1D_FN - 1; j >= 0; j--) {
+                const float2 cc = __ldg(c + j);
+                r0 = r0 * t + cc.x;
+                r1 = r1 * t + cc.y;
+            }
+            j0 = r0;
+            j1 = r1;
+            return;
+        }
         double f[4];
         table1d_t<F32>(X, f);
         j0 = f[0];
@@ -351,11 +367,13 @@ struct Wave {
     double F, FX, FY, I, IX, IY, c;
 };
 
+// eY = exp(-Y), which the assembly has as a product of one exponential per panel; 1 / R0 by rsqrt, R0 from
+// it (FP64 roots, exponentials and divisions are a third of the assembly's instructions).
 template <bool F32 = false>
-__device__ inline Wave wave_kernel(double X, double Y) {
+__device__ inline Wave wave_kernel(double X, double Y, double eY) {
     Wave o;
-    double R0 = sqrt(X * X + Y * Y);
-    double eY = exp(-Y), j0, j1, F, FX;
+    const double R2 = X * X + Y * Y, ir = rsqrt(R2), R0 = R2 * ir;
+    double j0, j1, F, FX;
     if (X < XT && Y < YT) {
         double f[4], v, vx;
         table1d_t<F32>(X, f);
@@ -367,8 +385,8 @@ __device__ inline Wave wave_kernel(double X, double Y) {
             table2d(X, Y, v, vx);
         double lg = log(Y + R0) + (GAMMA - LOG2);
         F = -2.0 * eY * j0 * lg - PI * eY * f[2] - 2.0 * R0 * v;
-        FX = 2.0 * eY * j1 * lg - 2.0 * eY * j0 * X / (R0 * (Y + R0)) - PI * eY * f[3] - 2.0 * (X / R0) * v -
-             2.0 * R0 * vx;
+        const double xr = X * ir;
+        FX = 2.0 * eY * j1 * lg - 2.0 * eY * j0 * (xr / (Y + R0)) - PI * eY * f[3] - 2.0 * xr * v - 2.0 * R0 * vx;
     } else if (Y >= YT) {
         bessel_j01<F32>(X, j0, j1);
         double P, PX;
@@ -387,29 +405,37 @@ __device__ inline Wave wave_kernel(double X, double Y) {
     }
     o.F = F;
     o.FX = FX;
-    o.FY = -F - 2.0 / R0;
+    o.FY = -F - 2.0 * ir;
     o.c = eY * j0;
     o.I = -2.0 * PI * eY * j0;
     o.IX = 2.0 * PI * eY * j1;
     o.IY = -o.I;
     return o;
 }
-
-// real part only (green_inf.rs:647-675)
 template <bool F32 = false>
-__device__ inline void wave_real(double X, double Y, double& F, double& FX, double& FY) {
-    double R0 = sqrt(X * X + Y * Y);
+__device__ inline Wave wave_kernel(double X, double Y) {
+    return wave_kernel<F32>(X, Y, exp(-Y));
+}
+
+// real part only (green_inf.rs:647-675); eY = exp(-Y)
+template <bool F32 = false>
+__device__ inline void wave_real(double X, double Y, double eY, double& F, double& FX, double& FY) {
     if (Y >= YT) {
         double P, PX;
         far_series(X, Y, 0.0, P, PX);
         F = -2.0 * P;
         FX = -2.0 * PX;
+        FY = -F - 2.0 * rsqrt(X * X + Y * Y);
     } else {
-        Wave w = wave_kernel<F32>(X, Y);
+        const Wave w = wave_kernel<F32>(X, Y, eY);
         F = w.F;
         FX = w.FX;
+        FY = w.FY;
     }
-    FY = -F - 2.0 / R0;
+}
+template <bool F32 = false>
+__device__ inline void wave_real(double X, double Y, double& F, double& FX, double& FY) {
+    wave_real<F32>(X, Y, exp(-Y), F, FX, FY);
 }
 
 // ------------------------------------------------------------------ finite depth (green_fin.rs)
@@ -573,23 +599,28 @@ __device__ __forceinline__ Kern wave_kern(double K, const Wave& w) {
 
 // low_order.rs:627-648 pair_kernel, infinite depth
 template <bool F32 = false>
-__device__ inline Kern pair_kernel_inf(double K, double R, double z, double zeta) {
+__device__ inline Kern pair_kernel_inf(double K, double R, double z, double zeta, double eY) {
     if (R == 0.0 && z == 0.0 && zeta == 0.0) {
         Kern k = {};
         k.Wr = -2.0 * K * (GAMMA - LOG2 + log(K));
         k.Wi = -2.0 * PI * K;
         return k;
     }
-    return wave_kern(K, wave_kernel<F32>(K * R, -K * (z + zeta)));
+    return wave_kern(K, wave_kernel<F32>(K * R, -K * (z + zeta), eY));
+}
+template <bool F32 = false>
+__device__ inline Kern pair_kernel_inf(double K, double R, double z, double zeta) {
+    return pair_kernel_inf<F32>(K, R, z, zeta, exp(K * (z + zeta)));
 }
 
 // green_fin.rs:1007-1095 finite_kernel with the fin_point data of both points.
 // fz / fzeta: pointers to the plane-0 entry of the point in the fin_point planes (stride N).
 // SW: the infinite-depth wave term F3 at (K R, K v3) is supplied by the caller (*sw, when not null).
+// ih = 1 / h, eK = exp(K (z + zeta)).
 template <bool F32 = false, class TT = double, bool SW = false>
 __device__ inline Kern finite_kernel(const FdParams& fd, const TT* T1, const TT* T2, double R, double z,
                                      double zeta, const double* fz, const double* fzeta, int stride,
-                                     const Wave* sw = nullptr) {
+                                     double ih, double eK, const Wave* sw = nullptr) {
     double h = fd.h;
     double d1 = z - zeta;
     double sg = d1 > 0.0 ? 1.0 : d1 < 0.0 ? -1.0 : 0.0;
@@ -655,7 +686,7 @@ __device__ inline Kern finite_kernel(const FdParams& fd, const TT* T1, const TT*
         o.Wrz = rez;
         return o;
     }
-    double ih = 1.0 / h, ih2 = ih * ih, f1[3], f2[3];
+    double ih2 = ih * ih, f1[3], f2[3];
     if constexpr (F32) {
         phi_tiles_f32(T1, 1, R * ih, v[0] * ih, f1);
         phi_tiles_f32(T2, 2, R * ih, v[1] * ih, f2);
@@ -679,10 +710,10 @@ __device__ inline Kern finite_kernel(const FdParams& fd, const TT* T1, const TT*
                     F3X = sw->FX;
                     F3Y = sw->FY;
                 } else {
-                    wave_real<F32>(K * R, K * v[2], F3, F3X, F3Y);
+                    wave_real<F32>(K * R, K * v[2], eK, F3, F3X, F3Y);
                 }
             } else {
-                wave_real<F32>(K * R, K * v[2], F3, F3X, F3Y);
+                wave_real<F32>(K * R, K * v[2], eK, F3, F3X, F3Y);
             }
         }
         o.Wr += K * F3;

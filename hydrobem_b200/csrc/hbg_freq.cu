@@ -120,9 +120,9 @@ void launch_fin_points(const PanelsView& pv, int F, const FdParams* fd, double* 
 // low_order.rs:738-769 apply_kernel + 781-790 kind_column: (S, D-column) of panel j at x.
 __device__ __forceinline__ void apply_kernel(double rs, double rd, double dl, double dd, double area, double nx,
                                              double ny, double nz, int kindj, const double* x, const double* cj,
-                                             double K, double logc, const Kern& k, double R, bool swapped,
+                                             double K, double logc, const Kern& k, double iR, bool swapped,
                                              double2& S, double2& D) {
-    double a = R > 0.0 ? ((x[0] - cj[0]) * nx + (x[1] - cj[1]) * ny) / R : 0.0;
+    double a = ((x[0] - cj[0]) * nx + (x[1] - cj[1]) * ny) * iR;  // iR = 1 / R, 0 where R = 0
     double rz = swapped ? k.Wrz : k.WrZ;
     double iz = swapped ? k.Wiz : k.WiZ;
     S.x = rs + area * k.Wr - 2.0 * K * logc * dl;
@@ -141,8 +141,16 @@ __device__ __forceinline__ double free_term(int kind) { return kind == 1 ? -4.0 
 // unordered pair (G(x, xi) = G(xi, x), the swapped source derivative for (n, k):
 // lo_frequency.rs:399-537), the (n, k) statics read and the (n, k) entries written through shared
 // memory transposes so that every global access is coalesced along the rows.
+// Bound by instruction issue and L1 together (mixed, finite depth, per 32 pairs: 1240 instructions, of them 260 FP64,
+// and 430 L1 wavefronts, a 16-byte gather being four whatever its addresses, in 550 cycles): what counts is
+// instructions, so the exponentials are one per panel and frequency, and 1 / R and 1 / R0 are formed once.  Measured
+// (ms, before / now, the LU's working copy of A written here instead of copied: 1.6, 1.3 and 4.2 ms more): 4096
+// panels, h = 5 m, 40 frequencies 19.8 / 18.7; 12288 panels, 4 frequencies 13.1 / 12.1; 18496 panels, 5 frequencies
+// 39.5 / 36.6; the FP64 form, 4096 panels, 8 frequencies 10.3 / 10.0.  Two columns a thread with shared coefficients
+// were slower (22.9, 14.4, 41.6): more registers and instructions than the gathers they saved.
 // Output policies of the assembly: complex128 column-major N x N (the FP64 form), or two FP32 planes
 // column-major with leading dimension Np (the mixed form; entry (k, n) at n Np + k).
+// at: the offset of entry (k, n) of matrix f; a thread steps by columns of ld() elements.
 struct OutF64 {
     static constexpr bool kF32 = false;  // FP64 coefficient tables
     static constexpr int kT1 = T1_SIZE, kT2 = T2_SIZE;
@@ -151,11 +159,15 @@ struct OutF64 {
     double2* A;
     size_t stride;
     int N;
-    __device__ __forceinline__ void put(int f, int k, int n, double2 s, double2 a) const {
-        size_t o = (size_t)f * stride + (size_t)k + (size_t)n * N;
+    __device__ __forceinline__ size_t at(int f, int k, int n) const {
+        return (size_t)f * stride + (size_t)k + (size_t)n * N;
+    }
+    __device__ __forceinline__ int ld() const { return N; }
+    __device__ __forceinline__ void put(size_t o, double2 s, double2 a) const {
         S[o] = s;
         A[o] = a;
     }
+    __device__ __forceinline__ void put(int f, int k, int n, double2 s, double2 a) const { put(at(f, k, n), s, a); }
 };
 
 struct OutF32 {
@@ -166,13 +178,22 @@ struct OutF32 {
     float* A;
     size_t bstride;  // per frequency: two planes of Np * Np
     int Np;
-    __device__ __forceinline__ void put(int f, int k, int n, double2 s, double2 a) const {
-        size_t o = (size_t)f * bstride + (size_t)n * Np + k, pl = (size_t)Np * Np;
+    float* W = nullptr;  // the LU's working copy of A, written beside it (null: none)
+    __device__ __forceinline__ size_t at(int f, int k, int n) const { return (size_t)f * bstride + (size_t)n * Np + k; }
+    __device__ __forceinline__ int ld() const { return Np; }
+    __device__ __forceinline__ void put(size_t o, double2 s, double2 a) const {
+        const size_t pl = bstride / 2;
+        const float ar = (float)a.x, ai = (float)a.y;
         S[o] = (float)s.x;
         S[o + pl] = (float)s.y;
-        A[o] = (float)a.x;
-        A[o + pl] = (float)a.y;
+        A[o] = ar;
+        A[o + pl] = ai;
+        if (W) {
+            W[o] = ar;
+            W[o + pl] = ai;
+        }
     }
+    __device__ __forceinline__ void put(int f, int k, int n, double2 s, double2 a) const { put(at(f, k, n), s, a); }
 };
 
 // Symmetry sectors (SECT, G = pv.G > 1): block y = f G + g assembles the image block g of frequency f,
@@ -217,7 +238,8 @@ __global__ void __launch_bounds__(256, Out::kF32 ? 3 : 2) k_assemble(PanelsView 
     const int k = K0 + tx;
     // xk: the field point of row k; ck, nk, ak: panel g k (the source of entry (n, g k)); kept in shared
     // memory (read where used: short live ranges instead of ten doubles held across the pairs)
-    __shared__ double sKd[10][32], sNd[10][32];
+    // and exp(K z) of both depths, whose product is the wave term's exponential of a pair
+    __shared__ double sKd[11][32], sNd[11][32];
     __shared__ int sKind[32], sNKind[32];
     if (ty == 1) {  // the same for the column panels n = N0 + tx: xn, cn, nn, an
         const int nn = N0 + tx;
@@ -235,6 +257,7 @@ __global__ void __launch_bounds__(256, Out::kF32 ? 3 : 2) k_assemble(PanelsView 
         }
         for (int d = 0; d < 3; d++) sNd[d][tx] = xn[d], sNd[3 + d][tx] = cn[d], sNd[6 + d][tx] = nv3[d];
         sNd[9][tx] = an;
+        sNd[10][tx] = exp(K * cn[2]);
         sNKind[tx] = kindn;
     }
     if (ty == 0) {
@@ -252,6 +275,7 @@ __global__ void __launch_bounds__(256, Out::kF32 ? 3 : 2) k_assemble(PanelsView 
         }
         for (int d = 0; d < 3; d++) sKd[d][tx] = xk[d], sKd[3 + d][tx] = ck[d], sKd[6 + d][tx] = nk[d];
         sKd[9][tx] = ak;
+        sKd[10][tx] = exp(K * xk[2]);
         sKind[tx] = kindk;
     }
     __syncthreads();
@@ -261,6 +285,7 @@ __global__ void __launch_bounds__(256, Out::kF32 ? 3 : 2) k_assemble(PanelsView 
     const typename Out::Tile* T1 = FINITE ? tiles + (size_t)f * (Out::kT1 + Out::kT2) : nullptr;
     const typename Out::Tile* T2 = FINITE ? T1 + Out::kT1 : nullptr;
     const double* fp = FINITE ? fpt + (size_t)f * FP_PLANES * Nf : nullptr;
+    const double ih = FINITE ? 1.0 / fd->h : 0.0;
 #pragma unroll 1
     for (int i = 0; i < 4; i++) {
         const int nl = ty + 8 * i, n = N0 + nl;
@@ -275,29 +300,31 @@ __global__ void __launch_bounds__(256, Out::kF32 ? 3 : 2) k_assemble(PanelsView 
             R = sqrt(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
             zn = vN[5][nl];
         }
+        const double eK = vK[10][tx] * vN[10][nl];
         Kern w;
         if (FINITE) {
-            w = finite_kernel<Out::kF32>(*fd, T1, T2, R, xk[2], zn, fp + k, fp + n, Nf);
+            w = finite_kernel<Out::kF32>(*fd, T1, T2, R, xk[2], zn, fp + k, fp + n, Nf, ih, eK);
         } else {
-            w = pair_kernel_inf<Out::kF32>(K, R, xk[2], zn);
+            w = pair_kernel_inf<Out::kF32>(K, R, xk[2], zn, eK);
         }
+        const double iR = R > 0.0 ? 1.0 / R : 0.0;
         const double xn[3] = {vN[0][nl], vN[1][nl], vN[2][nl]}, cn[3] = {vN[3][nl], vN[4][nl], vN[5][nl]};
         const double nn3[3] = {vN[6][nl], vN[7][nl], vN[8][nl]}, an = vN[9][nl];
         const int kindn = sNKind[nl];
         // entry (k, n): the field point x_k against panel g n
-        size_t o1 = (size_t)k + (size_t)n * N;
         double2 s1, d1;
         {
+            const double* ps = stg + (size_t)k + (size_t)n * N;
             const double xk2[3] = {vK[0][tx], vK[1][tx], vK[2][tx]};
-            apply_kernel(__ldg(stg + o1), __ldg(stg + NN + o1), __ldg(stg + 2 * NN + o1), __ldg(stg + 3 * NN + o1),
-                         an, nn3[0], nn3[1], nn3[2], kindn, xk2, cn, K, logc, w, R, false, s1, d1);
+            apply_kernel(__ldg(ps), __ldg(ps + NN), __ldg(ps + 2 * NN), __ldg(ps + 3 * NN), an, nn3[0], nn3[1], nn3[2],
+                         kindn, xk2, cn, K, logc, w, iR, false, s1, d1);
         }
-        out.put(y, k, n, s1, make_double2((g == 0 && k == n ? free_term(sKind[tx]) : 0.0) - d1.x, -d1.y));
+        out.put(out.at(y, k, n), s1, make_double2((g == 0 && k == n ? free_term(sKind[tx]) : 0.0) - d1.x, -d1.y));
         if (n != k) {
             double2 s2, d2;
             const double ck[3] = {vK[3][tx], vK[4][tx], vK[5][tx]};
             apply_kernel(sT[0][tx][nl], sT[1][tx][nl], sT[2][tx][nl], sT[3][tx][nl], vK[9][tx], vK[6][tx], vK[7][tx],
-                         vK[8][tx], sKind[tx], xn, ck, K, logc, w, R, true, s2, d2);
+                         vK[8][tx], sKind[tx], xn, ck, K, logc, w, iR, true, s2, d2);
             sT[0][tx][nl] = s2.x;
             sT[1][tx][nl] = s2.y;
             sT[2][tx][nl] = -d2.x;
@@ -306,11 +333,12 @@ __global__ void __launch_bounds__(256, Out::kF32 ? 3 : 2) k_assemble(PanelsView 
     }
     __syncthreads();
     // write the (n, k) entries: n = N0 + tx (coalesced), k = K0 + ty + 8 i
+    size_t o = out.at(y, N0 + tx, K0 + ty);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < 4; i++, o += 8 * (size_t)out.ld()) {
         int n = N0 + tx, kl = ty + 8 * i, kk = K0 + kl;
         if (n < N && kk < N && (kb != nb || n > kk))
-            out.put(y, n, kk, make_double2(sT[0][kl][tx], sT[1][kl][tx]), make_double2(sT[2][kl][tx], sT[3][kl][tx]));
+            out.put(o, make_double2(sT[0][kl][tx], sT[1][kl][tx]), make_double2(sT[2][kl][tx], sT[3][kl][tx]));
     }
 }
 
@@ -407,12 +435,13 @@ __global__ void __launch_bounds__(256) k_field(PanelsView pv, const double* __re
         const double cj[3] = {pv.at(P_C, j), pv.at(P_C + 1, j), pv.at(P_C + 2, j)};
         const double dx = x[0] - cj[0], dy = x[1] - cj[1];
         const double R = sqrt(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
-        const Kern w = FINITE ? finite_kernel<false>(fdp[f], T1, T1 + T1_SIZE, R, x[2], cj[2], fqf + N + p, fqf + j, N + P)
+        const Kern w = FINITE ? finite_kernel<false>(fdp[f], T1, T1 + T1_SIZE, R, x[2], cj[2], fqf + N + p, fqf + j, N + P,
+                                                     1.0 / depth, exp(K * (x[2] + cj[2])))
                               : pair_kernel_inf<false>(K, R, x[2], cj[2]);
         const size_t o = (size_t)p + (size_t)j * P;
         double2 S, D;
         apply_kernel(stp[o], stp[NP + o], stp[2 * NP + o], stp[3 * NP + o], pv.at(P_AREA, j), pv.at(P_N, j),
-                     pv.at(P_N + 1, j), pv.at(P_N + 2, j), 0, x, cj, K, logc, w, R, false, S, D);
+                     pv.at(P_N + 1, j), pv.at(P_N + 2, j), 0, x, cj, K, logc, w, R > 0.0 ? 1.0 / R : 0.0, false, S, D);
 #pragma unroll
         for (int c = 0; c < FIELD_COLS; c++) {
             if (c >= nrhs) break;
@@ -491,12 +520,12 @@ void launch_field(const PanelsView& pv, const double* pts, int P, const double* 
 __device__ __forceinline__ bool chi_neg(int c, int g) { return __popc(c & g) & 1; }
 
 // The G image blocks M_g of each frequency (matrices f G .. f G + G - 1 of S and of A) replaced in
-// place by the sector matrices sum_g chi_c(g) M_g (lo_frequency.rs:276-346: S_c(k, n) =
+// place (A's also into W, when given) by the sector matrices sum_g chi_c(g) M_g (lo_frequency.rs:276-346: S_c(k, n) =
 // sum_g chi_c(g) S(k, g n), A_c likewise; the free term of block 0 enters every sector).  Entries
 // (k, n) < Nm of `nplanes` planes, each entry `comps` consecutive T at (n ld + k) comps; sums in FP64.
 template <typename T>
-__global__ void k_sectors(T* __restrict__ S, T* __restrict__ A, int G, int Nm, int ld, int comps, size_t plane,
-                          int nplanes, size_t mstride) {
+__global__ void k_sectors(T* __restrict__ S, T* __restrict__ A, T* __restrict__ W, int G, int Nm, int ld, int comps,
+                          size_t plane, int nplanes, size_t mstride) {
     const int f = blockIdx.y;
     const size_t per = (size_t)Nm * Nm * comps * nplanes;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < 2 * per; t += (size_t)gridDim.x * blockDim.x) {
@@ -505,25 +534,27 @@ __global__ void k_sectors(T* __restrict__ S, T* __restrict__ A, int G, int Nm, i
         const int c = (int)(e % comps);
         const size_t r = e / comps;
         const int k = (int)(r % Nm), n = (int)((r / Nm) % Nm), p = (int)(r / ((size_t)Nm * Nm));
-        T* b = M + (size_t)f * G * mstride + (size_t)p * plane + ((size_t)n * ld + k) * comps + c;
+        const size_t o = (size_t)f * G * mstride + (size_t)p * plane + ((size_t)n * ld + k) * comps + c;
+        T* b = M + o;
         double v[4];
         for (int g = 0; g < G; g++) v[g] = (double)b[(size_t)g * mstride];
         for (int cc = 0; cc < G; cc++) {
             double w = 0.0;
             for (int g = 0; g < G; g++) w += chi_neg(cc, g) ? -v[g] : v[g];
             b[(size_t)cc * mstride] = (T)w;
+            if (W && t >= per) W[o + (size_t)cc * mstride] = (T)w;  // the LU's working copy of A
         }
     }
 }
 
 void launch_sectors_f64(double2* S, double2* A, int F, int G, int Nm, size_t mat_stride, cudaStream_t s) {
-    k_sectors<double><<<dim3(296, F), 256, 0, s>>>(reinterpret_cast<double*>(S), reinterpret_cast<double*>(A), G, Nm,
-                                                    Nm, 2, 0, 1, 2 * mat_stride);
+    k_sectors<double><<<dim3(296, F), 256, 0, s>>>(reinterpret_cast<double*>(S), reinterpret_cast<double*>(A),
+                                                    nullptr, G, Nm, Nm, 2, 0, 1, 2 * mat_stride);
 }
 
-void launch_sectors_f32(float* S, float* A, int F, int G, int Nm, int Np, cudaStream_t s) {
+void launch_sectors_f32(float* S, float* A, float* W, int F, int G, int Nm, int Np, cudaStream_t s) {
     const size_t plane = (size_t)Np * Np;
-    k_sectors<float><<<dim3(296, F), 256, 0, s>>>(S, A, G, Nm, Np, 1, plane, 2, 2 * plane);
+    k_sectors<float><<<dim3(296, F), 256, 0, s>>>(S, A, W, G, Nm, Np, 1, plane, 2, 2 * plane);
 }
 
 // Right-hand-side vectors projected on the sectors (lo_frequency.rs:875-884): up[f G + c][col][n] =
@@ -618,9 +649,9 @@ void launch_tiles_f32(int F, const double* tiles, float* tiles_f, cudaStream_t s
 }
 
 void launch_assemble_f32(const PanelsView& pv, const double* st, int F, const FreqInfo* fi, const FdParams* fd,
-                         const float* tiles, const double* fpt, bool finite, float* S, float* A, int Np,
+                         const float* tiles, const double* fpt, bool finite, float* S, float* A, float* W, int Np,
                          cudaStream_t s) {
-    assemble(pv, st, F, fi, fd, tiles, fpt, finite, OutF32{S, A, 2 * (size_t)Np * Np, Np}, s);
+    assemble(pv, st, F, fi, fd, tiles, fpt, finite, OutF32{S, A, 2 * (size_t)Np * Np, Np, W}, s);
 }
 
 // ------------------------------------------------------------------ boundary values

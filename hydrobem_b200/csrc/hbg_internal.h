@@ -275,14 +275,14 @@ void launch_assemble_f64(const PanelsView& pv, const double* st, int F, const Fr
                          const double* tiles, const double* fpt, bool finite, double2* S, double2* A,
                          size_t mat_stride, cudaStream_t s);
 void launch_assemble_f32(const PanelsView& pv, const double* st, int F, const FreqInfo* fi, const FdParams* fd,
-                         const float* tiles, const double* fpt, bool finite, float* S, float* A, int Np,
+                         const float* tiles, const double* fpt, bool finite, float* S, float* A, float* W, int Np,
                          cudaStream_t s);
 void launch_tiles_f32(int F, const double* tiles, float* tiles_f, cudaStream_t s);
 // symmetry sectors: the image blocks of F frequencies into their sector matrices (in place), the
 // right-hand sides projected on the sectors up[F G][nrhs][ldp], the potentials of every panel
 // phi[F][nrhs][G Nm] from the sector solutions x[F G][nrhs][ldx]
 void launch_sectors_f64(double2* S, double2* A, int F, int G, int Nm, size_t mat_stride, cudaStream_t s);
-void launch_sectors_f32(float* S, float* A, int F, int G, int Nm, int Np, cudaStream_t s);
+void launch_sectors_f32(float* S, float* A, float* W, int F, int G, int Nm, int Np, cudaStream_t s);
 void launch_project(const double2* u, double2* up, int F, int G, int Nm, int nrhs, int ldp, cudaStream_t s);
 void launch_recombine(const double2* x, double2* phi, int F, int G, int Nm, int nrhs, int ldx, cudaStream_t s);
 // the wave-term network inside the mixed assembly: its parameters followed by the outputs' means and

@@ -516,15 +516,16 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             if (sg)
                 launch_assemble_f32_sg(pv, st, nb, dfi, dfd, tiles_f, fpt, fin, S32, A32, Np, sg_img, sg_count, err, s);
             else
-                launch_assemble_f32(pv, st, nb, dfi, dfd, tiles_f, fpt, fin, S32, A32, Np, s);
+                launch_assemble_f32(pv, st, nb, dfi, dfd, tiles_f, fpt, fin, S32, A32, G > 1 ? nullptr : W, Np, s);
             if (G > 1) {
-                launch_sectors_f32(S32, A32, nb, G, Nm, Np, s);
+                launch_sectors_f32(S32, A32, W, nb, G, Nm, Np, s);
                 (*launches)++;
             }
             // algorithmic bytes per pair: 4 FP64 statics read (32 B), S and A written as complex64 (16 B)
             P.end(KF_ASSEMBLE, 48.0 * (double)Nm * N * nb, s);
-            if (Np > Nm) k_pad_identity<<<dim3(64, ns), 256, 0, s>>>(A32, Nm, Np, MB);
-            cudaMemcpyAsync(W, A32, MB * ns * 4, cudaMemcpyDeviceToDevice, s);
+            if (Np > Nm) k_pad_identity<<<dim3(64, ns), 256, 0, s>>>(A32, W, Nm, Np, MB);
+            if (sg && G == 1)  // (the others write the LU's working copy of A beside it)
+                cudaMemcpyAsync(W, A32, MB * ns * 4, cudaMemcpyDeviceToDevice, s);
             P.begin(s);
             launch_boundary(pv, nb, dfi, H, dheads, depth, opt.gravity, u, phiI, s);
             P.end(KF_BOUNDARY, 0.0, s);

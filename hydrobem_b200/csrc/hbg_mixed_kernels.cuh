@@ -1474,11 +1474,10 @@ __global__ void __launch_bounds__(256) k_ir_update(int Np, int nrhs, double2* __
     }
 }
 
-// The padding rows and columns N..Np of the planar matrices: identity (zero elsewhere).
-__global__ void k_pad_identity(float* __restrict__ W, int N, int Np, size_t bstride) {
+// The padding rows and columns N..Np of the planar matrices A and W: identity (zero elsewhere).
+__global__ void k_pad_identity(float* __restrict__ A, float* __restrict__ W, int N, int Np, size_t bstride) {
     const int f = blockIdx.y;
-    float* Wr = W + (size_t)f * bstride;
-    float* Wi = Wr + (size_t)Np * Np;
+    float* Mr[2] = {A + (size_t)f * bstride, W + (size_t)f * bstride};
     const size_t npad = (size_t)(Np - N);
     const size_t total = 2 * npad * Np;  // the last npad columns and the last npad rows
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -1492,8 +1491,11 @@ __global__ void k_pad_identity(float* __restrict__ W, int N, int Np, size_t bstr
             c = u % Np;
         }
         size_t o = c * Np + r;
-        Wr[o] = (r == c) ? 1.f : 0.f;
-        Wi[o] = 0.f;
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            Mr[m][o] = (r == c) ? 1.f : 0.f;
+            Mr[m][o + (size_t)Np * Np] = 0.f;
+        }
     }
 }
 

@@ -613,22 +613,23 @@ __global__ void __launch_bounds__(256, 1) k_assemble_sg(PanelsView pv, const dou
             if (FINITE) {
                 if (inb) {
                     const Wave sw = sg_wave(X, Y, o6);
-                    w = finite_kernel<true, float, true>(*fd, T1, T2, R, xk[2], xn[2], fp + k, fp + n, N, &sw);
+                    w = finite_kernel<true, float, true>(*fd, T1, T2, R, xk[2], xn[2], fp + k, fp + n, N, 1.0 / fd->h, 0.0, &sw);
                 } else {
-                    w = finite_kernel<true>(*fd, T1, T2, R, xk[2], xn[2], fp + k, fp + n, N);
+                    w = finite_kernel<true>(*fd, T1, T2, R, xk[2], xn[2], fp + k, fp + n, N, 1.0 / fd->h, exp(K * (xk[2] + xn[2])));
                 }
             } else {
                 w = inb ? wave_kern(K, sg_wave(X, Y, o6)) : pair_kernel_inf<true>(K, R, xk[2], xn[2]);
             }
+            const double iR = R > 0.0 ? 1.0 / R : 0.0;
             size_t o1 = (size_t)k + (size_t)n * N;
             double2 s1, d1;
             apply_kernel(__ldg(st + o1), __ldg(st + NN + o1), __ldg(st + 2 * NN + o1), __ldg(st + 3 * NN + o1), an,
-                         nn3[0], nn3[1], nn3[2], kindn, xk, xn, K, logc, w, R, false, s1, d1);
+                         nn3[0], nn3[1], nn3[2], kindn, xk, xn, K, logc, w, iR, false, s1, d1);
             out.put(f, k, n, s1, make_double2((k == n ? free_term(kindk) : 0.0) - d1.x, -d1.y));
             if (n != k) {
                 double2 s2, d2;
                 apply_kernel(sT[0][tx][nl], sT[1][tx][nl], sT[2][tx][nl], sT[3][tx][nl], ak, nk[0], nk[1], nk[2],
-                             kindk, xn, xk, K, logc, w, R, true, s2, d2);
+                             kindk, xn, xk, K, logc, w, iR, true, s2, d2);
                 sT[0][tx][nl] = s2.x;
                 sT[1][tx][nl] = s2.y;
                 sT[2][tx][nl] = -d2.x;
