@@ -325,19 +325,53 @@ __device__ __forceinline__ int log_order(const PanelRegs& p, const double* image
     return 0;
 }
 
-__device__ inline void log_gauss(const PanelRegs& p, const double* image, int order, double& L, double& Ld) {
+// The points of the panel's order-4 rule (x, y, z and weight), formed once a panel: log_point4 of lane e < 16.
+struct LogPoint {
+    double x[3], w;
+};
+__device__ __forceinline__ LogPoint log_point4(const PanelRegs& p, int e) {
+    double m[4][3], jac;
+    panel_map(p, m);
+    LogPoint q;
+    bilinear(m, c_glx[4][e / 4], c_glx[4][e % 4], q.x, jac);
+    q.w = c_glw[4][e / 4] * c_glw[4][e % 4] * jac;
+    return q;
+}
+// log_gauss of order 4 on those points
+__device__ __forceinline__ void log_gauss4(const LogPoint* lp, const PanelRegs& p, const double* image, double& L, double& Ld) {
+    double l = 0.0, ld = 0.0;
+#pragma unroll 2
+    for (int e = 0; e < 16; e++) {
+        double psi, dpsi;
+        psi_terms(lp[e].x, image, p.n, psi, dpsi);
+        l += lp[e].w * psi;
+        ld += lp[e].w * dpsi;
+    }
+    L = l;
+    Ld = ld;
+}
+
+// The Gauss rule of order n x n (5 to 10) at one image by a warp: the points spread over the lanes, the sums in every
+// lane.  (A lane of its own for each image ran the orders of a warp's images one after another, up to
+// 25 + 36 + 64 + 100 points of ~150 dependent FP64 instructions: 177 us for the whole of an 84-panel hull.)
+__device__ __forceinline__ void log_gauss_warp(const PanelRegs& p, const double* image, int order, int lane, double& L,
+                                               double& Ld) {
     double m[4][3];
     panel_map(p, m);
     double l = 0.0, ld = 0.0;
-    for (int i = 0; i < order; i++)
-        for (int j = 0; j < order; j++) {
-            double xi[3], jac, psi, dpsi;
-            bilinear(m, c_glx[order][i], c_glx[order][j], xi, jac);
-            psi_terms(xi, image, p.n, psi, dpsi);
-            double ww = c_glw[order][i] * c_glw[order][j] * jac;
-            l += ww * psi;
-            ld += ww * dpsi;
-        }
+    for (int e = lane; e < order * order; e += 32) {
+        const int i = e / order, j = e - i * order;
+        double xi[3], jac, psi, dpsi;
+        bilinear(m, c_glx[order][i], c_glx[order][j], xi, jac);
+        psi_terms(xi, image, p.n, psi, dpsi);
+        double ww = c_glw[order][i] * c_glw[order][j] * jac;
+        l += ww * psi;
+        ld += ww * dpsi;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, o);
+        ld += __shfl_xor_sync(0xffffffffu, ld, o);
+    }
     L = l;
     Ld = ld;
 }
@@ -348,45 +382,52 @@ __device__ inline void log_gauss(const PanelRegs& p, const double* image, int or
 // The rule's error falls as (radius / distance)^6, below FP32 rounding at 20 radii.
 constexpr double MIX_FAR = 20.0;
 
-__device__ __forceinline__ void rankine_gauss_f32(const PanelsView& pv, int j, const PanelRegs& p, const double* x,
-                                                  double& S, double& D) {
+// The images of a field point differ in z alone, so the horizontal differences of a Gauss point are formed once for
+// all of them (bit i of any: some lane of the warp needs image i); the rule's points and weights in shared memory.
+template <int NI>
+__device__ __forceinline__ void rankine_gauss_f32(const double (*g)[3], const float* gw, const PanelRegs& p, const double* x,
+                                                  const double (&z)[NI], unsigned any, double (&S)[NI], double (&D)[NI]) {
     const float n0 = (float)p.n[0], n1 = (float)p.n[1], n2 = (float)p.n[2];
-    float s = 0.f, dd = 0.f;
+    float s[NI], dd[NI];
 #pragma unroll
+    for (int i = 0; i < NI; i++) s[i] = dd[i] = 0.f;
+#pragma unroll 3
     for (int k = 0; k < 9; k++) {
-        const float r0 = (float)(x[0] - pv.at(P_GX + 3 * k, j));
-        const float r1 = (float)(x[1] - pv.at(P_GX + 3 * k + 1, j));
-        const float r2 = (float)(x[2] - pv.at(P_GX + 3 * k + 2, j));
-        const float w = (float)pv.at(P_GW + k, j);
-        const float ir = rsqrtf(__fmaf_rn(r0, r0, __fmaf_rn(r1, r1, r2 * r2)));
-        const float wi = w * ir;
-        s += wi;
-        dd = __fmaf_rn(wi * ir * ir, __fmaf_rn(n0, r0, __fmaf_rn(n1, r1, n2 * r2)), dd);
+        const float r0 = (float)(x[0] - g[k][0]), r1 = (float)(x[1] - g[k][1]);
+        const double gz = g[k][2];
+        const float w = gw[k];
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+            if (!(any >> i & 1)) continue;
+            const float r2 = (float)(z[i] - gz);
+            const float ir = rsqrtf(__fmaf_rn(r0, r0, __fmaf_rn(r1, r1, r2 * r2)));
+            const float wi = w * ir;
+            s[i] += wi;
+            dd[i] = __fmaf_rn(wi * ir * ir, __fmaf_rn(n0, r0, __fmaf_rn(n1, r1, n2 * r2)), dd[i]);
+        }
     }
-    S = s;
-    D = dd;
+#pragma unroll
+    for (int i = 0; i < NI; i++) S[i] = s[i], D[i] = dd[i];
 }
 
 // log_gauss with the integrand log(R - dz) and its normal derivative in FP32 (positions, weights and
 // sums in FP64): R - dz = R + |dz| for an image above the panel, so no cancellation.
-__device__ inline void log_gauss_f32(const PanelRegs& p, const double* image, int order, double& L, double& Ld) {
-    double m[4][3];
-    panel_map(p, m);
+__device__ __forceinline__ void log_gauss4_f32(const LogPoint* lp, const PanelRegs& p, const double* image, double& L,
+                                               double& Ld) {
     const float n0 = (float)p.n[0], n1 = (float)p.n[1], n2 = (float)p.n[2];
     double l = 0.0, ld = 0.0;
-    for (int i = 0; i < order; i++)
-        for (int j = 0; j < order; j++) {
-            double xi[3], jac;
-            bilinear(m, c_glx[order][i], c_glx[order][j], xi, jac);
-            const float d0 = (float)(xi[0] - image[0]), d1 = (float)(xi[1] - image[1]), d2 = (float)(xi[2] - image[2]);
-            const float R = sqrtf(__fmaf_rn(d0, d0, __fmaf_rn(d1, d1, d2 * d2)));
-            const float den = R - d2;
-            const float psi = logf(den);
-            const float dpsi = (__fmaf_rn(d0, n0, __fmaf_rn(d1, n1, d2 * n2)) / R - n2) / den;
-            const double ww = c_glw[order][i] * c_glw[order][j] * jac;
-            l += ww * (double)psi;
-            ld += ww * (double)dpsi;
-        }
+#pragma unroll 4
+    for (int e = 0; e < 16; e++) {
+        const double* xi = lp[e].x;
+        const float d0 = (float)(xi[0] - image[0]), d1 = (float)(xi[1] - image[1]), d2 = (float)(xi[2] - image[2]);
+        const float R = sqrtf(__fmaf_rn(d0, d0, __fmaf_rn(d1, d1, d2 * d2)));
+        const float den = R - d2;
+        const float psi = logf(den);
+        const float dpsi = (__fmaf_rn(d0, n0, __fmaf_rn(d1, n1, d2 * n2)) / R - n2) / den;
+        const double ww = lp[e].w;
+        l += ww * (double)psi;
+        ld += ww * (double)dpsi;
+    }
     L = l;
     Ld = ld;
 }
@@ -428,30 +469,16 @@ __device__ inline void rankine_gauss_tier(const PanelRegs& p, const float* __res
     D = d;
 }
 
-// Rankine integrals at x: with the tiers, panel_integrals.rs:359-363 rankine_any of the production mode
-// (the tiers, or the closed forms within 2 radii); the mixed form's own rule otherwise (the closed
-// forms, the FP32 3 x 3 rule beyond MIX_FAR radii); the FP64 form the closed forms.
-template <bool MIXED>
-__device__ __forceinline__ void rankine_at(const PanelsView& pv, int j, const PanelRegs& p, const double* x, double& S,
-                                           double& D) {
-    if constexpr (MIXED) {
-        const double t0 = x[0] - p.c[0], t1 = x[1] - p.c[1], t2 = x[2] - p.c[2];
-        if (pv.tiers) {  // the production rule
-            const double rc[3] = {t0, t1, t2};
-            const int t = rankine_tier(norm3(rc) / p.radius);
-            if (t >= 0) {
-                rankine_gauss_tier(p, pv.tiers + (size_t)j * TIER_FLOATS, x, t, S, D);
-                return;
-            }
-        } else {  // the mixed form's own rule: the closed forms within MIX_FAR radii
-            const double far = MIX_FAR * p.radius;
-            if (t0 * t0 + t1 * t1 + t2 * t2 > far * far) {
-                rankine_gauss_f32(pv, j, p, x, S, D);
-                return;
-            }
-        }
-    }
-    rankine(pv, j, p, x, S, D);
+// Rankine integrals at x by the production rule, panel_integrals.rs:359-363 rankine_any: the tiers, or the closed forms
+// within 2 radii.
+__device__ __forceinline__ void rankine_prod(const PanelsView& pv, int j, const PanelRegs& p, const double* x, double& S,
+                                             double& D) {
+    const double rc[3] = {x[0] - p.c[0], x[1] - p.c[1], x[2] - p.c[2]};
+    const int t = rankine_tier(norm3(rc) / p.radius);
+    if (t >= 0)
+        rankine_gauss_tier(p, pv.tiers + (size_t)j * TIER_FLOATS, x, t, S, D);
+    else
+        rankine(pv, j, p, x, S, D);
 }
 
 // panel_integrals.rs:380-392: in the production mode the log integral of an image farther than 12 radii
@@ -508,77 +535,136 @@ __device__ inline double log_in_plane(const PanelRegs& p, const double* x) {
 // MIXED: the mixed form's variant (far Rankine points and the order-4 log rule in FP32, above; with
 // pv.tiers the reference's production rule instead, rows in float32); the FP64 form runs the reference's
 // double-precision arithmetic to the bit.
-template <bool MIXED>
-__global__ void __launch_bounds__(256, 2) k_statics(PanelsView pv, double depth, int logint, double tol,
+// Bound by instruction issue and the conversions' pipe (per 32 pairs of the mixed form, infinite depth: 1800
+// instructions, of them 440 FP64 and 150 conversions and reciprocals, before; FP64 closed forms near, the 3 x 3 and
+// order-4 rules far).  Three CTAs an SM (80 registers, some spills) against two: 18496 panels 32.6 / 39.3 ms.  Measured, ms
+// before / now: mixed 4096 panels, h = 5 m 4.2 / 2.6, 12288 panels 13.7 / 9.8, 18496 panels 50.0 / 33.5, FP64 4096
+// panels 7.4 / 6.4; 84 panels 0.18 / 0.035, with the adaptive pairs 0.46 / 0.11.
+// A warp has one panel; what depends on the panel alone (its data, the 3 x 3 rule, the points of the order-4 log rule
+// with their FP64 bilinear map and Jacobian) is formed once by the warp, in shared memory.
+template <bool MIXED, bool FINITE>
+__global__ void __launch_bounds__(256, 3) k_statics(PanelsView pv, double depth, int logint, double tol, int rows,
                                                  double* __restrict__ st, int32_t* __restrict__ work,
                                                  int32_t* __restrict__ nwork, int work_cap) {
+    constexpr int NI = FINITE ? 6 : 2;  // the point and its images
     // rows: the sector's panels (or the field points); columns: all panels
     const int N = pv.N, Nr = pv.rows ? pv.nrows : N / pv.G;
-    int k = blockIdx.x * 32 + threadIdx.x;
+    int k = blockIdx.x * rows + threadIdx.x;  // a warp's first `rows` lanes hold a row each
     int j = blockIdx.y * 8 + threadIdx.y;
     // the panel of each warp (36 values every lane of the warp reads) in shared memory rather than in
     // 72 registers of every lane
     __shared__ PanelRegs sp[8];
-    if (threadIdx.x == 0 && j < N) load_panel(pv, j, sp[threadIdx.y]);
-    __syncthreads();
-    if (k >= Nr || j >= N) return;
+    __shared__ LogPoint slp[8][16];
+    __shared__ double sg[MIXED ? 8 : 1][9][3];
+    __shared__ float sgw[MIXED ? 8 : 1][9];
+    if (j >= N) return;  // (a whole warp)
+    if (threadIdx.x == 0) load_panel(pv, j, sp[threadIdx.y]);
+    __syncwarp();
     const PanelRegs& p = sp[threadIdx.y];
+    if (threadIdx.x < 16) slp[threadIdx.y][threadIdx.x] = log_point4(p, threadIdx.x);
+    if (MIXED && threadIdx.x < 9) {
+        for (int d = 0; d < 3; d++) sg[threadIdx.y][threadIdx.x][d] = pv.at(P_GX + 3 * threadIdx.x + d, j);
+        sgw[threadIdx.y][threadIdx.x] = (float)pv.at(P_GW + threadIdx.x, j);
+    }
+    __syncwarp();
+    const LogPoint* lp = slp[threadIdx.y];
+    const bool live = (int)threadIdx.x < rows && k < Nr;
+    if (!live) k = min(k, Nr - 1);
     double x[3];
     for (int d = 0; d < 3; d++) x[d] = pv.rows ? pv.rows[3 * k + d] : pv.at(P_C + d, k);
     double xb[3] = {x[0], x[1], -x[2]};
-    double s0, d0, sb, db;
-    rankine_at<MIXED>(pv, j, p, x, s0, d0);
-    rankine_at<MIXED>(pv, j, p, xb, sb, db);
-    double sr = s0 + sb, dr = d0 + db;
-    if (depth > 0.0) {
-        double h = depth;
-        double p1[3] = {x[0], x[1], -x[2] - 2.0 * h}, p3[3] = {x[0], x[1], x[2] + 2.0 * h};
-        double p4[3] = {x[0], x[1], x[2] - 2.0 * h}, p5[3] = {x[0], x[1], -x[2] - 4.0 * h};
-        double s2, d2, s4, d4, s5, d5, s6, d6;
-        rankine_at<MIXED>(pv, j, p, p1, s2, d2);
-        rankine_at<MIXED>(pv, j, p, p3, s4, d4);
-        if (MIXED && pv.tiers) {  // production: the two deep images by the 3 x 3 rule beyond 12 radii
-            rankine(pv, j, p, p4, s5, d5, 12.0);  // (lo_static.rs:82-88)
-            rankine(pv, j, p, p5, s6, d6, 12.0);
-        } else {
-            rankine_at<MIXED>(pv, j, p, p4, s5, d5);
-            rankine_at<MIXED>(pv, j, p, p5, s6, d6);
+    const double h = depth;
+    double z[NI], S[NI], D[NI];
+    z[0] = x[2];
+    z[1] = -x[2];
+    if constexpr (FINITE) {
+        z[2] = -x[2] - 2.0 * h;
+        z[3] = x[2] + 2.0 * h;
+        z[4] = x[2] - 2.0 * h;
+        z[5] = -x[2] - 4.0 * h;
+    }
+    if (MIXED && !pv.tiers) {  // the mixed form's own rule: the closed forms within MIX_FAR radii
+        const double far = MIX_FAR * p.radius, t0 = x[0] - p.c[0], t1 = x[1] - p.c[1];
+        unsigned mine = 0, any = 0;
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+            const double t2 = z[i] - p.c[2];
+            const bool f = t0 * t0 + t1 * t1 + t2 * t2 > far * far;
+            mine |= (unsigned)f << i;
+            any |= (unsigned)(__any_sync(0xffffffffu, f) != 0) << i;
         }
-        sr += (s2 + s4) + s5 + s6;
-        dr += (d2 + d4) + d5 + d6;
+        rankine_gauss_f32<NI>(sg[threadIdx.y], sgw[threadIdx.y], p, x, z, any, S, D);
+#pragma unroll
+        for (int i = 0; i < NI; i++)
+            if (live && !(mine >> i & 1)) {
+                const double xi[3] = {x[0], x[1], z[i]};
+                rankine(pv, j, p, xi, S[i], D[i]);
+            }
+    } else if (live) {
+#pragma unroll
+        for (int i = 0; i < NI; i++) {
+            const double xi[3] = {x[0], x[1], z[i]};
+            if (!MIXED)
+                rankine(pv, j, p, xi, S[i], D[i]);
+            else if (i >= 4)  // production: the two deep images by the 3 x 3 rule beyond 12 radii
+                rankine(pv, j, p, xi, S[i], D[i], 12.0);  // (lo_static.rs:82-88)
+            else
+                rankine_prod(pv, j, p, xi, S[i], D[i]);
+        }
+    }
+    double sr = S[0] + S[1], dr = D[0] + D[1];
+    if constexpr (FINITE) {
+        sr += (S[2] + S[3]) + S[4] + S[5];
+        dr += (D[2] + D[3]) + D[4] + D[5];
     }
     const bool prod = MIXED && pv.tiers;  // the production rows are stored in float32
     size_t NN = (size_t)Nr * N, o = (size_t)k + (size_t)j * Nr;
-    st[o] = prod ? to_f32(sr) : sr;
-    st[NN + o] = prod ? to_f32(dr) : dr;
+    if (live) {
+        st[o] = prod ? to_f32(sr) : sr;
+        st[NN + o] = prod ? to_f32(dr) : dr;
+    }
     double dl = 0.0, dd = 0.0;
-    bool use_log = logint && log_pair(p, x, tol);
-    if (use_log && pv.kind[j] == 1 && x[2] == 0.0) {
-        double L = log_in_plane(p, x);
+    const bool use_log = live && logint && log_pair(p, x, tol);
+    const bool plane = use_log && pv.kind[j] == 1 && x[2] == 0.0;
+    int order = 4;
+    bool far3 = false;
+    if (use_log && !plane) {
+        const double tb[3] = {xb[0] - p.c[0], xb[1] - p.c[1], xb[2] - p.c[2]};
+        far3 = prod && norm3(tb) > 12.0 * p.radius;
+        order = far3 ? 3 : log_order(p, xb);
+    }
+    // the near images one after another, each by the whole warp
+    double L = 0.0, Ld = 0.0;
+    for (unsigned near = __ballot_sync(0xffffffffu, order > 4); near; near &= near - 1) {
+        const int src = __ffs(near) - 1;
+        const double image[3] = {__shfl_sync(0xffffffffu, xb[0], src), __shfl_sync(0xffffffffu, xb[1], src),
+                                 __shfl_sync(0xffffffffu, xb[2], src)};
+        double l, ld;
+        log_gauss_warp(p, image, __shfl_sync(0xffffffffu, order, src), threadIdx.x, l, ld);
+        if ((int)threadIdx.x == src) L = l, Ld = ld;
+    }
+    if (!live) return;
+    if (plane) {
+        const double Lp = log_in_plane(p, x);
         double t[3] = {p.c[0] - x[0], p.c[1] - x[1], p.c[2] - x[2]};
         double Rr = norm3(t);
-        dl = Rr > 0.0 ? L - p.area * log(Rr) : L;
+        dl = Rr > 0.0 ? Lp - p.area * log(Rr) : Lp;
+    } else if (use_log && order > 0) {
+        double psi, dpsi;
+        if (far3)
+            log_far_3x3(pv, j, p, xb, L, Ld);
+        else if (order == 4 && MIXED && !prod)
+            log_gauss4_f32(lp, p, xb, L, Ld);
+        else if (order == 4)
+            log_gauss4(lp, p, xb, L, Ld);
+        psi_terms(p.c, xb, p.n, psi, dpsi);
+        dl = L - p.area * psi;
+        dd = Ld - p.area * dpsi;
     } else if (use_log) {
-        const double tb[3] = {xb[0] - p.c[0], xb[1] - p.c[1], xb[2] - p.c[2]};
-        const bool far3 = prod && norm3(tb) > 12.0 * p.radius;
-        int order = far3 ? 3 : log_order(p, xb);
-        if (order > 0) {
-            double L, Ld, psi, dpsi;
-            if (far3)
-                log_far_3x3(pv, j, p, xb, L, Ld);
-            else if (MIXED && !prod && order == 4)
-                log_gauss_f32(p, xb, order, L, Ld);
-            else
-                log_gauss(p, xb, order, L, Ld);
-            psi_terms(p.c, xb, p.n, psi, dpsi);
-            dl = L - p.area * psi;
-            dd = Ld - p.area * dpsi;
-        } else {
-            int slot = atomicAdd(nwork, 1);
-            if (slot < work_cap) {
-                work[2 * slot] = k;
-                work[2 * slot + 1] = j;
-            }
+        int slot = atomicAdd(nwork, 1);
+        if (slot < work_cap) {
+            work[2 * slot] = k;
+            work[2 * slot + 1] = j;
         }
     }
     st[2 * NN + o] = prod ? to_f32(dl) : dl;
@@ -601,11 +687,13 @@ __device__ inline void log_cell(const double m[4][3], const double* image, const
         }
 }
 
-// The adaptive pairs: quadrisection to 1e-13 of the integrals' scale, at most 14 levels, cells
-// taken in the depth-first order of panel_integrals.rs:100-120.  One warp per pair: at each level
-// the 32 lanes evaluate the 4 sub-cells x 16 Gauss points (two points a lane), reduce them per
-// sub-cell by shuffles, and lane 0 keeps the depth-first stack in shared memory.
-constexpr int AD_WARPS = 4, AD_STACK = 48;
+// The adaptive pairs: quadrisection to 1e-13 of the integrals' scale, at most 14 levels
+// (panel_integrals.rs:100-120).  One CTA per pair: the cells wait on a stack in shared memory, each round the
+// AD_WARPS topmost are taken, a warp each (the 32 lanes evaluate the 4 sub-cells x 16 Gauss points, two a lane, and
+// reduce them per sub-cell by shuffles), and those to be split push their sub-cells.  A cell's decision depends on
+// its own sums alone, so the cells are those of the reference's depth-first order; their sums are added per warp,
+// then over the warps in order.  (One warp a pair took 0.29-0.39 ms for the few pairs of a small hull.)
+constexpr int AD_WARPS = 8, AD_STACK = AD_WARPS * 48;
 
 struct AdCell {
     double u0, u1, v0, v1, p0, p1;
@@ -623,13 +711,22 @@ __device__ __forceinline__ void log_point(const double m[4][3], const double* im
     b = ww * dpsi;
 }
 
-// One adaptive pair (worklist entry t) by the calling warp; stk: the warp's stack in shared memory.
-__device__ void adaptive_pair(const PanelsView& pv, const int32_t* __restrict__ work, int t, double* __restrict__ st,
-                              AdCell* stk, int lane) {
-    const int N = pv.N;
-    const int k = work[2 * t], j = work[2 * t + 1];
+struct AdShared {
+    AdCell stk[AD_STACK];
     PanelRegs p;
-    load_panel(pv, j, p);
+    double acc[AD_WARPS][2];
+    int split[AD_WARPS];
+    int entry;
+};
+
+// One adaptive pair (worklist entry t) by the calling CTA.
+__device__ void adaptive_pair(const PanelsView& pv, const int32_t* __restrict__ work, int t, double* __restrict__ st,
+                              AdShared& sh) {
+    const int N = pv.N, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k = work[2 * t], j = work[2 * t + 1];
+    if (threadIdx.x == 0) load_panel(pv, j, sh.p);
+    __syncthreads();
+    const PanelRegs& p = sh.p;
     double xb[3];
     for (int d = 0; d < 3; d++) xb[d] = pv.rows ? pv.rows[3 * k + d] : pv.at(P_C + d, k);
     xb[2] = -xb[2];
@@ -640,59 +737,67 @@ __device__ void adaptive_pair(const PanelsView& pv, const int32_t* __restrict__ 
     double dmin = fmax(dist - p.radius, 1e-3 * p.radius);
     double scale = fabs(log(dist + p.radius)) + 1.0;
     double tol_l = 1e-13 * p.area * scale, tol_d = 1e-13 * p.area / dmin;
-    // the whole square by one 4 x 4 cell (lanes 0..15 one point each)
-    double wa = 0.0, wb = 0.0;
-    if (lane < 16) log_point(m, xb, p.n, -1.0, 1.0, -1.0, 1.0, lane / 4, lane % 4, wa, wb);
-    for (int o = 16; o > 0; o >>= 1) {
-        wa += __shfl_xor_sync(0xffffffffu, wa, o);
-        wb += __shfl_xor_sync(0xffffffffu, wb, o);
+    if (warp == 0) {  // the whole square by one 4 x 4 cell (lanes 0..15 one point each)
+        double wa = 0.0, wb = 0.0;
+        if (lane < 16) log_point(m, xb, p.n, -1.0, 1.0, -1.0, 1.0, lane / 4, lane % 4, wa, wb);
+        for (int o = 16; o > 0; o >>= 1) {
+            wa += __shfl_xor_sync(0xffffffffu, wa, o);
+            wb += __shfl_xor_sync(0xffffffffu, wb, o);
+        }
+        if (lane == 0) sh.stk[0] = AdCell{-1.0, 1.0, -1.0, 1.0, wa, wb, 0};
     }
-    int sp = 0;
-    if (lane == 0) stk[0] = AdCell{-1.0, 1.0, -1.0, 1.0, wa, wb, 0};
-    sp = 1;
-    __syncwarp();
+    int sp = 1;
     double acc0 = 0.0, acc1 = 0.0;
+    __syncthreads();
     while (sp > 0) {
-        AdCell c = stk[sp - 1];
-        sp--;
-        __syncwarp();
-        const double um = 0.5 * (c.u0 + c.u1), vm = 0.5 * (c.v0 + c.v1);
-        const double us0[4] = {c.u0, um, um, c.u0}, us1[4] = {um, c.u1, c.u1, um};
-        const double vs0[4] = {c.v0, c.v0, vm, vm}, vs1[4] = {vm, vm, c.v1, c.v1};
-        // lane l: point l of sub-cells (l / 16) and (l / 16) + 2
-        const int sa = lane >> 4, q = lane & 15;
-        double a0, b0, a1, b1;
-        log_point(m, xb, p.n, us0[sa], us1[sa], vs0[sa], vs1[sa], q / 4, q % 4, a0, b0);
-        log_point(m, xb, p.n, us0[sa + 2], us1[sa + 2], vs0[sa + 2], vs1[sa + 2], q / 4, q % 4, a1, b1);
-        for (int o = 8; o > 0; o >>= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            b0 += __shfl_xor_sync(0xffffffffu, b0, o);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-            b1 += __shfl_xor_sync(0xffffffffu, b1, o);
+        const int take = min(sp, AD_WARPS);
+        sp -= take;
+        bool split = false;
+        AdCell c;
+        double a0, b0, a1, b1, um, vm;
+        if (warp < take) {
+            c = sh.stk[sp + take - 1 - warp];
+            um = 0.5 * (c.u0 + c.u1), vm = 0.5 * (c.v0 + c.v1);
+            // lane l: point l % 16 of sub-cells (l / 16) and (l / 16) + 2, in the order (u0, v0), (um, v0), (um, vm), (u0, vm)
+            const int sa = lane >> 4, q = lane & 15;
+            const double ua = sa ? um : c.u0, ub = sa ? c.u1 : um;
+            log_point(m, xb, p.n, ua, ub, c.v0, vm, q / 4, q % 4, a0, b0);
+            log_point(m, xb, p.n, sa ? c.u0 : um, sa ? um : c.u1, vm, c.v1, q / 4, q % 4, a1, b1);
+            for (int o = 8; o > 0; o >>= 1) {
+                a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+                b0 += __shfl_xor_sync(0xffffffffu, b0, o);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+                b1 += __shfl_xor_sync(0xffffffffu, b1, o);
+            }
+            // the sums of sub-cells 0, 1 (lanes 0, 16 of a0, b0) and 2, 3
+            const double s0 = __shfl_sync(0xffffffffu, a0, 0) + __shfl_sync(0xffffffffu, a0, 16) +
+                              __shfl_sync(0xffffffffu, a1, 0) + __shfl_sync(0xffffffffu, a1, 16);
+            const double s1 = __shfl_sync(0xffffffffu, b0, 0) + __shfl_sync(0xffffffffu, b0, 16) +
+                              __shfl_sync(0xffffffffu, b1, 0) + __shfl_sync(0xffffffffu, b1, 16);
+            split = !(c.depth >= 14 || (fabs(s0 - c.p0) <= tol_l && fabs(s1 - c.p1) <= tol_d));
+            if (split && sp + 4 * AD_WARPS > AD_STACK) split = false;  // (the stack holds more than 14 levels need)
+            if (!split) acc0 += s0, acc1 += s1;
         }
-        double cc[4][2];
-        cc[0][0] = __shfl_sync(0xffffffffu, a0, 0);
-        cc[0][1] = __shfl_sync(0xffffffffu, b0, 0);
-        cc[1][0] = __shfl_sync(0xffffffffu, a0, 16);
-        cc[1][1] = __shfl_sync(0xffffffffu, b0, 16);
-        cc[2][0] = __shfl_sync(0xffffffffu, a1, 0);
-        cc[2][1] = __shfl_sync(0xffffffffu, b1, 0);
-        cc[3][0] = __shfl_sync(0xffffffffu, a1, 16);
-        cc[3][1] = __shfl_sync(0xffffffffu, b1, 16);
-        const double s0 = cc[0][0] + cc[1][0] + cc[2][0] + cc[3][0];
-        const double s1 = cc[0][1] + cc[1][1] + cc[2][1] + cc[3][1];
-        if (c.depth >= 14 || (fabs(s0 - c.p0) <= tol_l && fabs(s1 - c.p1) <= tol_d) || sp + 4 > AD_STACK) {
-            acc0 += s0;
-            acc1 += s1;
-            continue;
+        if (lane == 0) sh.split[warp] = split;
+        __syncthreads();  // the cells are taken, the decisions known
+        int at = sp, total = 0;
+#pragma unroll
+        for (int w = 0; w < AD_WARPS; w++) {
+            if (w < warp) at += 4 * sh.split[w];
+            total += sh.split[w];
         }
-        if (lane == 0)
-            for (int qq = 3; qq >= 0; qq--)
-                stk[sp + 3 - qq] = AdCell{us0[qq], us1[qq], vs0[qq], vs1[qq], cc[qq][0], cc[qq][1], c.depth + 1};
-        sp += 4;
-        __syncwarp();
+        if (split && (lane & 15) == 0) {  // lanes 0 and 16 hold the sums of sub-cells 0, 2 and 1, 3
+            const int sa = lane >> 4;
+            sh.stk[at + 3 - sa] = AdCell{sa ? um : c.u0, sa ? c.u1 : um, c.v0, vm, a0, b0, c.depth + 1};
+            sh.stk[at + 1 - sa] = AdCell{sa ? c.u0 : um, sa ? um : c.u1, vm, c.v1, a1, b1, c.depth + 1};
+        }
+        sp += 4 * total;
+        __syncthreads();
     }
-    if (lane == 0) {
+    if (lane == 0) sh.acc[warp][0] = acc0, sh.acc[warp][1] = acc1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < AD_WARPS; w++) acc0 += sh.acc[w][0], acc1 += sh.acc[w][1];
         double psi, dpsi;
         psi_terms(p.c, xb, p.n, psi, dpsi);
         const int Nr = pv.rows ? pv.nrows : N / pv.G;
@@ -703,14 +808,11 @@ __device__ void adaptive_pair(const PanelsView& pv, const int32_t* __restrict__ 
     }
 }
 
-// One warp per worklist entry, the entry count given by the host.
+// One CTA per worklist entry, the entry count given by the host.
 __global__ void __launch_bounds__(AD_WARPS * 32) k_statics_adaptive(PanelsView pv, const int32_t* __restrict__ work,
                                                                     int nwork, double* __restrict__ st) {
-    __shared__ AdCell stack[AD_WARPS][AD_STACK];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * AD_WARPS + warp;
-    if (t >= nwork) return;
-    adaptive_pair(pv, work, t, st, stack[warp], lane);
+    __shared__ AdShared sh;
+    if ((int)blockIdx.x < nwork) adaptive_pair(pv, work, blockIdx.x, st, sh);
 }
 
 // The same with the entry count in device memory (q[0], capped at work_cap) and the entries taken
@@ -720,17 +822,16 @@ __global__ void __launch_bounds__(AD_WARPS * 32) k_statics_adaptive_q(PanelsView
                                                                       int32_t* q, int work_cap,
                                                                       const int32_t* __restrict__ bad, int32_t clean,
                                                                       double* __restrict__ st) {
-    __shared__ AdCell stack[AD_WARPS][AD_STACK];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ AdShared sh;
     if (*bad != clean) return;
     const int nwork = min(*(volatile int32_t*)q, work_cap);
     for (;;) {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(q + 1, 1);
-        t = __shfl_sync(0xffffffffu, t, 0);
+        if (threadIdx.x == 0) sh.entry = atomicAdd(q + 1, 1);
+        __syncthreads();
+        const int t = sh.entry;
         if (t >= nwork) return;
-        adaptive_pair(pv, work, t, st, stack[warp], lane);
-        __syncwarp();
+        adaptive_pair(pv, work, t, st, sh);
+        __syncthreads();  // (the next entry overwrites the shared data)
     }
 }
 
@@ -740,17 +841,27 @@ void launch_panel_geometry(int N, const double* verts, const int32_t* kind, doub
     k_panel_geometry<<<(N + 127) / 128, 128, 0, s>>>(N, verts, kind, planes, bad, tiers, orig);
 }
 
+// Pairs up to which a warp takes four rows instead of 32.  Measured, us with 4 / 32 rows: 84 panels 35 / 56; 512 panels
+// 388 / 97 (eight rows 210): a warp costs the same with few rows, so they pay only while the device is nearly empty.
+constexpr double STATICS_SMALL = 1.6e4;
+
 void launch_statics(const PanelsView& pv, double depth, int logint, double tol, double* st, int32_t* work,
                     int32_t* nwork, int work_cap, cudaStream_t s, bool mixed) {
-    dim3 grid(((pv.rows ? pv.nrows : pv.N / pv.G) + 31) / 32, (pv.N + 7) / 8);
+    // few panels: fewer rows a warp, so that its near images (a warp's work each) are spread over the device
+    const int Nr = pv.rows ? pv.nrows : pv.N / pv.G;
+    const int rows = (double)Nr * pv.N < STATICS_SMALL ? 4 : 32;
+    dim3 grid((Nr + rows - 1) / rows, (pv.N + 7) / 8);
+    auto go = [&](auto kernel) {
+        kernel<<<grid, dim3(32, 8), 0, s>>>(pv, depth, logint, tol, rows, st, work, nwork, work_cap);
+    };
     if (mixed)
-        k_statics<true><<<grid, dim3(32, 8), 0, s>>>(pv, depth, logint, tol, st, work, nwork, work_cap);
+        depth > 0.0 ? go(k_statics<true, true>) : go(k_statics<true, false>);
     else
-        k_statics<false><<<grid, dim3(32, 8), 0, s>>>(pv, depth, logint, tol, st, work, nwork, work_cap);
+        depth > 0.0 ? go(k_statics<false, true>) : go(k_statics<false, false>);
 }
 
 void launch_statics_adaptive(const PanelsView& pv, const int32_t* work, int nwork, double* st, cudaStream_t s) {
-    if (nwork > 0) k_statics_adaptive<<<(nwork + AD_WARPS - 1) / AD_WARPS, AD_WARPS * 32, 0, s>>>(pv, work, nwork, st);
+    if (nwork > 0) k_statics_adaptive<<<nwork, AD_WARPS * 32, 0, s>>>(pv, work, nwork, st);
 }
 
 void launch_statics_adaptive_q(const PanelsView& pv, const int32_t* work, int32_t* q, int work_cap,
