@@ -6,6 +6,7 @@
 // Matrices are column-major complex128 (entry (i, j) at i + j N), matrix f at A + f * stride.
 // ipiv[f * N + i] is the 0-based row swapped with row i at step i (LAPACK's layout).
 #include <atomic>
+#include <type_traits>
 
 #include "hbg_device.cuh"
 #include "hbg_internal.h"
@@ -125,6 +126,224 @@ __global__ void __launch_bounds__(512) k_lu_base(int N, int c0, int w, int pk0, 
     }
 }
 
+// ------------------------------------------------------------------ strip in registers
+// The same for strips of up to W columns while the rows fit a cluster of up to eight CTAs, a row a thread: the
+// row's entries stay in registers, shifted down a column a step (so that every register index is constant and the loop
+// body short), its multipliers in shared memory.  Per column each warp finds
+// its candidate (two 32-bit reductions: the upper word of |a|^2, so a pivot is within 1e-6 of the largest modulus, and
+// the first position) and puts its row and reciprocal into shared memory, its claim into every CTA's; a cluster
+// barrier; every CTA takes the winner's row over, and updates.  Rows change places in `pos` alone and are written to
+// their places at the end, where the panel's other columns are permuted too.  Bound by that chain of dependent
+// instructions, ~1.1 us a column in one CTA, ~2 in clusters: a strip of 32 columns takes 41 / 64 / 79 us with 84 / 645 /
+// 1007 rows where one of 8 columns with its rows in global memory took 18 / 23 / 28, and 64 with 4096, and a panel now
+// needs three products between its strips instead of fifteen.  Whole LU, ms, before / now: 9 systems of order 645 3.28
+// / 2.21, 21 of order 1007 6.8 / 4.75, 8 of order 4096 64.8 / 58.9.
+constexpr int LU_CLUSTER = 8;  // the portable limit
+template <int W>
+struct LuStrip {
+    static constexpr int T = W == 32 ? 256 : 512, NW = T / 32;  // threads (rows) of a CTA, its warps
+    static constexpr int MAXROWS = T * LU_CLUSTER;
+    struct __align__(16) Slot {
+        unsigned key;  // upper word of |a|^2, plus one (0: no candidate)
+        int pos, src, low;  // low: nonzero if |a|^2 is above zero
+    };
+    struct Shared {
+        double2 L[W][T];  // multipliers
+        double2 row[2][NW][W + 1];  // the candidates' rows, the reciprocal of the diagonal before it
+        double2 prow[2][W + 1];     // the winner's, taken over from another CTA
+        Slot slot[2][LU_CLUSTER * NW];
+        int from[2 * W], to[2 * W];  // the moved rows (those of CTA 0 count)
+        int moved;
+    };
+};
+
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ unsigned cluster_size() {
+    unsigned r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync(unsigned size) {
+    if (size == 1) {
+        __syncthreads();
+    } else {
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+// the address of this CTA's shared variable in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, unsigned rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store16(uint32_t a, const void* v) {
+    const uint4 q = *static_cast<const uint4*>(v);
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
+}
+
+template <int W>
+__global__ void __launch_bounds__(LuStrip<W>::T) k_lu_strip(int N, int c0, int w, int pk0, int pnb,
+                                                            double2* __restrict__ Aall, size_t stride,
+                                                            int32_t* __restrict__ ipiv, int32_t* __restrict__ info) {
+    using S = LuStrip<W>;
+    constexpr int T = S::T, NW = S::NW;
+    extern __shared__ __align__(16) unsigned char strip_raw[];
+    typename S::Shared& sh = *reinterpret_cast<typename S::Shared*>(strip_raw);
+    const unsigned C = cluster_size(), rank = cluster_rank();
+    const int f = blockIdx.x / C, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double2* A = Aall + (size_t)f * stride;
+    const int orig = c0 + (int)rank * T + tid;
+    bool active = orig < N;
+    int pos = active ? orig : 0x7fffffff;
+    if (tid == 0) sh.moved = 0;
+    double2 a[W];
+#pragma unroll
+    for (int c = 0; c < W; c++)
+        a[c] = active && c < w ? A[(size_t)orig + (size_t)(c0 + c) * N] : make_double2(0.0, 0.0);
+    cluster_sync(C);  // every CTA of the cluster runs before another one writes to it
+    auto step = [&](int j, auto width) {
+        constexpr int R = decltype(width)::value;  // columns still held, at most
+        const int col = c0 + j, par = j & 1;
+        // ---- the warp's candidate: largest modulus, first position on a tie
+        {
+            const double m2 = cabs2(a[0]);
+            // (in flight beside the search)
+            const double im2 = m2 > 0.0 ? 1.0 / m2 : 0.0;
+            const double2 rcp = make_double2(a[0].x * im2, -a[0].y * im2);
+            const unsigned key = active && m2 == m2 ? (unsigned)__double2hiint(m2) + 1 : 0;
+            const unsigned mk = __reduce_max_sync(0xffffffffu, key);
+            const unsigned mp = __reduce_min_sync(0xffffffffu, key == mk ? (unsigned)pos : 0x7fffffffu);
+            if (key == mk && pos == (int)mp) {  // one lane (in a warp without candidates its row is never taken)
+                double2* q = sh.row[par][warp];
+                q[0] = rcp;
+#pragma unroll
+                for (int c = 0; c < R; c++) q[1 + c] = a[c];
+                typename S::Slot v{mk, (int)mp, (int)(rank * T) + tid, m2 > 0.0};
+                typename S::Slot* o = &sh.slot[par][rank * NW + warp];
+                if (C == 1)
+                    *o = v;
+                else
+                    for (unsigned c = 0; c < C; c++) cluster_store16(cluster_addr(o, c), &v);
+            }
+        }
+        cluster_sync(C);
+        // ---- the column's pivot
+        typename S::Slot best{0, 0x7fffffff, 0, 0};
+        for (int e = lane; e < (int)C * NW; e += 32) {
+            const typename S::Slot v = sh.slot[par][e];
+            if (v.key > best.key || (v.key == best.key && v.key && v.pos < best.pos)) best = v;
+        }
+        const unsigned mk = __reduce_max_sync(0xffffffffu, best.key);
+        const unsigned mp = __reduce_min_sync(0xffffffffu, best.key == mk ? (unsigned)best.pos : 0x7fffffffu);
+        const int from = __ffs(__ballot_sync(0xffffffffu, best.key == mk && best.pos == (int)mp)) - 1;
+        const int src = __shfl_sync(0xffffffffu, best.src, from), low = __shfl_sync(0xffffffffu, best.low, from);
+        const bool none = mk == 0;  // every modulus a NaN: the row at the diagonal, its reciprocal zero
+        const int p = none ? col : (int)mp;
+        const bool mine = none ? pos == col : (int)(rank * T) + tid == src;
+        if (rank == 0 && tid == 0) {
+            ipiv[(size_t)f * N + col] = p;
+            if (!low && info[f] == 0) info[f] = col + 1;  // not above zero
+        }
+        const double2* prow = sh.row[par][(src % T) >> 5];
+        if (C > 1) {
+            if (tid <= R) {
+                uint4 v;
+                const uint32_t q = cluster_addr(&sh.row[par][(src % T) >> 5][tid], src / T);
+                asm volatile("ld.shared::cluster.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                             : "r"(q)
+                             : "memory");
+                *reinterpret_cast<uint4*>(&sh.prow[par][tid]) = v;
+            }
+            prow = sh.prow[par];
+            __syncthreads();
+        }
+        if (mine)
+            active = false, pos = col;
+        else if (pos == col)
+            pos = p;
+        // the pivot row is at its place: the row of U from the diagonal on, by the last CTA's last warp
+        if (rank == C - 1 && warp == NW - 1 && lane < w - j) A[(size_t)col + (size_t)(col + lane) * N] = prow[1 + lane];
+        // ---- multiplier and update
+        if (!__any_sync(0xffffffffu, active)) return;
+        const double2 l = none ? make_double2(0.0, 0.0) : cmul(a[0], prow[0]);
+        if (active) sh.L[j][tid] = l;
+#pragma unroll
+        for (int c = 0; c + 1 < R; c++) a[c] = csub(a[c + 1], cmul(l, prow[c + 2]));
+    };
+    // (half of the columns held from the middle on; more bodies cost more instruction fetches than they save)
+    int j = 0;
+    for (; j < min(w, W / 2); j++) step(j, std::integral_constant<int, W>());
+    for (; j < w; j++) step(j, std::integral_constant<int, W / 2>());
+    // ---- the rows to their places, the moved ones listed for the panel's other columns
+    const bool has = orig < N;
+    if (has)  // its multipliers (of a pivot row those before its diagonal)
+        for (int c = 0, n = min(w, pos - c0); c < n; c++) A[(size_t)pos + (size_t)(c0 + c) * N] = sh.L[c][tid];
+    if (has && pos != orig) {
+        uint32_t n0 = cluster_addr(&sh.moved, 0), e;
+        asm volatile("atom.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(e) : "r"(n0) : "memory");
+        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(cluster_addr(&sh.from[e], 0)), "r"(orig) : "memory");
+        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(cluster_addr(&sh.to[e], 0)), "r"(pos) : "memory");
+    }
+    cluster_sync(C);
+    int nm;
+    asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(nm) : "r"(cluster_addr(&sh.moved, 0)) : "memory");
+    if (rank != 0) {
+        for (int e = tid; e < nm; e += T) {
+            asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(sh.from[e]) : "r"(cluster_addr(&sh.from[e], 0)) : "memory");
+            asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(sh.to[e]) : "r"(cluster_addr(&sh.to[e], 0)) : "memory");
+        }
+    }
+    cluster_sync(C);  // (CTA 0's list may go)
+    if (nm == 0) return;
+    constexpr int V = 4;  // entries a thread holds across the barrier
+    const int per = V * T / nm, ncol = pnb - w;  // whole columns a pass
+    for (int b = (int)rank * per; b < ncol; b += (int)C * per) {
+        const int n = min(per, ncol - b) * nm;
+        double2 v[V];
+        size_t at[V];
+#pragma unroll
+        for (int q = 0; q < V; q++) {
+            const int e = tid + q * T;
+            if (e < n) {
+                int col = pk0 + b + e / nm;
+                if (col >= c0) col += w;
+                at[q] = (size_t)sh.to[e % nm] + (size_t)col * N;
+                v[q] = A[(size_t)sh.from[e % nm] + (size_t)col * N];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < V; q++)
+            if (tid + q * T < n) A[at[q]] = v[q];
+    }
+}
+
+template <int W>
+static void launch_lu_strip(int N, int F, int c0, int w, int pk0, int pnb, double2* A, size_t stride, int32_t* ipiv,
+                            int32_t* info, cudaStream_t s) {
+    using S = LuStrip<W>;
+    int C = 1;
+    while (C * S::T < N - c0) C *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(F * C);
+    cfg.blockDim = dim3(S::T);
+    cfg.dynamicSmemBytes = sizeof(typename S::Shared);
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_lu_strip<W>, N, c0, w, pk0, pnb, A, stride, ipiv, info);
+}
+
 // ------------------------------------------------------------------ row interchanges
 // The swaps of rows r0 .. r1 - 1 (in order, LAPACK's zlaswp) on the columns [ca, cb) and [cc, cd), one
 // thread per column.
@@ -146,6 +365,11 @@ __global__ void k_lu_laswp(int N, int r0, int r1, int ca, int cb, int cc, int cd
     }
 }
 
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool ok) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gmem), "r"(ok ? 16 : 0) : "memory");
+}
+
 // ------------------------------------------------------------------ triangular solves of a block row
 // B := L^-1 B (lower: L the unit lower n1 x n1 block of the factor at (c0, c0)) or B := U^-1 B (upper: U
 // the upper block, diagonal included), B the rows c0 .. c0 + n1 - 1, columns [cb, ce) of the matrix X
@@ -164,13 +388,16 @@ __global__ void __launch_bounds__(512) k_lu_trsm(int N, int c0, int n1, int cb, 
     // upper: column p holds rows 0 .. p at uoff(p) + r
     auto loff = [n1](int p) { return p * (2 * n1 - p - 1) / 2; };
     auto uoff = [](int p) { return p * (p + 1) / 2; };
+    // (cp.async: all of the triangle in flight at once; loads through registers took 8 us of latencies)
     if (UPPER) {
         for (int p = warp; p < n1; p += nw)
-            for (int r = lane; r <= p; r += 32) Lc[uoff(p) + r] = L[(size_t)(c0 + r) + (size_t)(c0 + p) * N];
+            for (int r = lane; r <= p; r += 32) cp_async16(Lc + uoff(p) + r, L + (size_t)(c0 + r) + (size_t)(c0 + p) * N, true);
     } else {
         for (int p = warp; p < n1 - 1; p += nw)
-            for (int r = p + 1 + lane; r < n1; r += 32) Lc[loff(p) + r - p - 1] = L[(size_t)(c0 + r) + (size_t)(c0 + p) * N];
+            for (int r = p + 1 + lane; r < n1; r += 32)
+                cp_async16(Lc + loff(p) + r - p - 1, L + (size_t)(c0 + r) + (size_t)(c0 + p) * N, true);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     for (int col0 = cb + (blockIdx.x * nw + warp) * CPW; col0 < ce; col0 += gridDim.x * nw * CPW) {
         double2 x[CPW][NQ];
@@ -284,11 +511,6 @@ struct ZgTile {
 };
 constexpr int ZG_NARROW = 1024;  // products of at most this many columns take the 32-column tiles
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool ok) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(gmem), "r"(ok ? 16 : 0) : "memory");
-}
-
 template <int WN>
 __global__ void __launch_bounds__(128 * WN, 4 / WN) k_lu_zgemm(int N, const double2* Aall, size_t astride, double2* Call,
                                                              size_t cstride, int r0, int c0, int k0, int M, int n, int K) {
@@ -391,8 +613,8 @@ static void lu_zgemm_attributes() {
 
 // The tile width of a product of n columns, autotuned per device: when the device is first used
 // (before any solve's work is queued on it) both widths are timed on a product of each width bucket
-// n <= 8, 16, ..., 2048 and 4096 (2048 rows, K = min(n, 128), four matrices, the best of three launches
-// each, on scratch buffers freed afterwards) and the 64-column tile is taken where it is at least 2 %
+// n <= 8, 16, ..., 2048 and 4096 (2048 rows, K = min(n, 128), four matrices, the best of three launches,
+// twelve of the short ones, on scratch buffers freed afterwards) and the 64-column tile is taken where it is at least 2 %
 // faster.  Until then, or if the timing cannot run, products of at most ZG_NARROW columns take the
 // 32-column tile (the choice the measurements on the benchmark's shapes gave).
 constexpr int ZG_TUNE_BUCKETS = 10;
@@ -458,7 +680,7 @@ void lu_tune_device(int dev) {
             for (int w = 0; w < 2; w++) {
                 float best = 1e30f;
                 launch_lu_zgemm_wn(w == 1, N, F, A, astride, C, cstride, KMAX, 0, 0, M, n, K, s);
-                for (int r = 0; r < 3 && ok; r++) {
+                for (int r = 0; r < (n <= 64 ? 12 : 3) && ok; r++) {  // (the short ones are near the events' resolution)
                     cudaEventRecord(e0, s);
                     launch_lu_zgemm_wn(w == 1, N, F, A, astride, C, cstride, KMAX, 0, 0, M, n, K, s);
                     cudaEventRecord(e1, s);
@@ -584,16 +806,23 @@ struct LuF64 {
     // the right half; the strips swap their rows across the whole panel, so no interchanges between)
     int pk0 = 0, pnb = 0;
     void panel(int c0, int w) {
-        if (w <= LU_BASE) {
+        // strips of 32 or 16 columns in registers while their rows fit a cluster, else of 8 in global memory
+        const int rows = N - c0, base = rows <= LuStrip<32>::MAXROWS ? 32 : rows <= LuStrip<16>::MAXROWS ? 16 : LU_BASE;
+        if (w <= base) {
             KernelProfiler& P = profiler();
             const double m = N - c0;
             P.begin(sp);
-            k_lu_base<<<F, 512, 0, sp>>>(N, c0, w, pk0, pnb, A, stride, ipiv, info);
+            if (base == 32)
+                launch_lu_strip<32>(N, F, c0, w, pk0, pnb, A, stride, ipiv, info, sp);
+            else if (base == 16)
+                launch_lu_strip<16>(N, F, c0, w, pk0, pnb, A, stride, ipiv, info, sp);
+            else
+                k_lu_base<<<F, 512, 0, sp>>>(N, c0, w, pk0, pnb, A, stride, ipiv, info);
             P.end(KF_LU_PANEL, (double)F * 8.0 * (m * w * w - (double)w * w * w / 3.0), sp);
             (*launches)++;
             return;
         }
-        const int n1 = w / 2 / LU_BASE * LU_BASE > 0 ? w / 2 / LU_BASE * LU_BASE : w / 2, n2 = w - n1;
+        const int n1 = w / 2 / base * base > 0 ? w / 2 / base * base : base, n2 = w - n1;
         panel(c0, n1);
         trsm(sp, c0, n1, c0 + n1, c0 + w);
         gemm(sp, c0 + n1, c0 + n1, c0, N - c0 - n1, n2, n1);
@@ -649,6 +878,8 @@ void lu_f64_schedule(int groups, int lookahead) {
 
 static void lu_f64_attributes() {
     lu_zgemm_attributes();
+    cudaFuncSetAttribute(k_lu_strip<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LuStrip<32>::Shared));
+    cudaFuncSetAttribute(k_lu_strip<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LuStrip<16>::Shared));
     cudaFuncSetAttribute(k_lu_trsm<4, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(double2) * LU_NB * (LU_NB - 1) / 2));
     cudaFuncSetAttribute(k_lu_trsm<4, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
