@@ -841,7 +841,8 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
     // ---- frequency batches
     // per frequency: G systems (S, A, right-hand sides, solutions, pivots), the boundary values and incident
     // wave of every panel, with sectors the projected right-hand sides and the recombined potentials
-    size_t per_freq = G * (2 * NN * sizeof(double2) + (size_t)2 * nrhs * Nm * sizeof(double2) + (size_t)Nm * 4 + 4) +
+    size_t per_freq = G * (2 * NN * sizeof(double2) + (size_t)2 * nrhs * Nm * sizeof(double2) + (size_t)Nm * 4 + 4 +
+                           rhs_f64_scratch(Nm, 1, nrhs)) +
                       (size_t)(nrhs + H) * N * sizeof(double2) + (G > 1 ? (size_t)2 * nrhs * N * sizeof(double2) : 0) +
                       (fin ? (size_t)(T1_SIZE + T2_SIZE) * 8 + (size_t)FP_PLANES * N * 8 +
                                                               (size_t)6912 * 3 * 8
@@ -884,6 +885,8 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
     dA.alloc(sizeof(double2) * NN * BS);
     du.alloc(sizeof(double2) * (size_t)nrhs * N * B);
     drhs.alloc(sizeof(double2) * (size_t)nrhs * Nm * BS);
+    WsBuf dpart(ws, WS_PART);
+    dpart.alloc(rhs_f64_scratch(Nm, (int)BS, nrhs));
     dX.alloc(sizeof(double2) * (size_t)nrhs * Nm * BS);
     if (G > 1) {
         dup.alloc(sizeof(double2) * (size_t)nrhs * Nm * BS);
@@ -964,7 +967,7 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
                 urhs = dup.as<double2>();
             }
             P.begin(s);
-            launch_rhs_f64(Nm, ns, nrhs, dS.as<double2>(), NN, urhs, drhs.as<double2>(), s);
+            launch_rhs_f64(Nm, ns, nrhs, dS.as<double2>(), NN, urhs, drhs.as<double2>(), dpart.as<double2>(), s);
             // S read once (16 B per entry)
             P.end(KF_RHS, 16.0 * (double)NN * ns, s);
             g_launches += 3 + 2 * (G > 1);

@@ -708,53 +708,88 @@ void launch_boundary(const PanelsView& pv, int F, const FreqInfo* fi, int H, con
 }
 
 // ------------------------------------------------------------------ right-hand sides -S u
-// One thread per row k holds the nrhs sums; S is read once, column by column (coalesced along k),
-// u staged in shared memory (lo_frequency.rs:875-892: the product S U with U = -u).
+// (lo_frequency.rs:875-892: the product S U with U = -u.)  One thread per row k and a chunk of columns of S holds the
+// nrhs partial sums: S is read once, eight columns in flight a thread (coalesced along k), u staged in shared
+// memory; k_rhs_sum adds the chunks in order.  One thread for all columns of its row left the device to a few
+// latency-bound CTAs: 0.47 ms for 9 systems of order 645, 3.0 for 8 of order 4096, now 0.09 and 0.98.
+// Columns of a chunk: 128, more where that would be over 16 chunks (a large matrix has rows enough to fill the device).
+static int rhs_chunk(int N) { return std::max(128, (N + 511) / 512 * 32); }
 template <int NR>
-__global__ void __launch_bounds__(128) k_rhs_f64(int N, int nrhs, const double2* __restrict__ S, size_t mat_stride,
-                                                 const double2* __restrict__ u, double2* __restrict__ rhs) {
-    constexpr int CH = 32;
+__global__ void __launch_bounds__(128) k_rhs_f64(int N, int nrhs, int chunk, const double2* __restrict__ S, size_t mat_stride,
+                                                 const double2* __restrict__ u, double2* __restrict__ part) {
+    constexpr int CH = 32, AHEAD = 8;
     __shared__ double2 su[CH][NR];
-    int f = blockIdx.y;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int f = blockIdx.y, z = blockIdx.z;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const double2* Sf = S + (size_t)f * mat_stride;
     const double2* uf = u + (size_t)f * nrhs * N;
+    const int nbeg = z * chunk, nend = min(N, nbeg + chunk);
     double2 acc[NR];
 #pragma unroll
     for (int c = 0; c < NR; c++) acc[c] = make_double2(0.0, 0.0);
-    for (int n0 = 0; n0 < N; n0 += CH) {
+    for (int n0 = nbeg; n0 < nend; n0 += CH) {
         __syncthreads();
         for (int t = threadIdx.x; t < CH * NR; t += blockDim.x) {
             int nn = t % CH, c = t / CH;
-            su[nn][c] = (n0 + nn < N && c < nrhs) ? uf[(size_t)c * N + n0 + nn] : make_double2(0.0, 0.0);
+            su[nn][c] = (n0 + nn < nend && c < nrhs) ? uf[(size_t)c * N + n0 + nn] : make_double2(0.0, 0.0);
         }
         __syncthreads();
         if (k < N) {
-            int lim = min(CH, N - n0);
-            for (int nn = 0; nn < lim; nn++) {
-                double2 s = Sf[(size_t)k + (size_t)(n0 + nn) * N];
+            const int lim = min(CH, nend - n0);
+            const double2* Sk = Sf + (size_t)k + (size_t)n0 * N;
+            for (int q = 0; q < lim; q += AHEAD) {
+                double2 s[AHEAD];
 #pragma unroll
-                for (int c = 0; c < NR; c++) {
-                    double2 v = su[nn][c];
-                    acc[c].x += s.x * v.x - s.y * v.y;
-                    acc[c].y += s.x * v.y + s.y * v.x;
-                }
+                for (int e = 0; e < AHEAD; e++) s[e] = q + e < lim ? __ldg(Sk + (size_t)(q + e) * N) : make_double2(0.0, 0.0);
+#pragma unroll
+                for (int e = 0; e < AHEAD; e++)
+#pragma unroll
+                    for (int c = 0; c < NR; c++) {
+                        const double2 v = su[min(q + e, CH - 1)][c];
+                        acc[c].x = fma(-s[e].y, v.y, fma(s[e].x, v.x, acc[c].x));
+                        acc[c].y = fma(s[e].y, v.x, fma(s[e].x, v.y, acc[c].y));
+                    }
             }
         }
     }
     if (k < N)
-        for (int c = 0; c < nrhs && c < NR; c++) rhs[((size_t)f * nrhs + c) * N + k] = make_double2(-acc[c].x, -acc[c].y);
+        for (int c = 0; c < nrhs && c < NR; c++) part[(((size_t)z * gridDim.y + f) * nrhs + c) * N + k] = acc[c];
+}
+
+__global__ void k_rhs_sum(size_t n, int nz, const double2* __restrict__ part, double2* __restrict__ rhs) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    double re = 0.0, im = 0.0;
+    for (int z = 0; z < nz; z++) {
+        const double2 v = part[(size_t)z * n + t];
+        re += v.x;
+        im += v.y;
+    }
+    rhs[t] = make_double2(-re, -im);
+}
+
+size_t rhs_f64_scratch(int N, int F, int nrhs) {
+    const int chunk = rhs_chunk(N);
+    return sizeof(double2) * ((N + chunk - 1) / chunk) * (size_t)F * nrhs * N;
 }
 
 void launch_rhs_f64(int N, int F, int nrhs, const double2* S, size_t mat_stride, const double2* u, double2* rhs,
-                    cudaStream_t s) {
-    dim3 grid((N + 127) / 128, F);
-    if (nrhs <= 8)
-        k_rhs_f64<8><<<grid, 128, 0, s>>>(N, nrhs, S, mat_stride, u, rhs);
+                    double2* scratch, cudaStream_t s) {
+    const int chunk = rhs_chunk(N), nz = (N + chunk - 1) / chunk;
+    dim3 grid((N + 127) / 128, F, nz);
+    auto go = [&](auto kernel) { kernel<<<grid, 128, 0, s>>>(N, nrhs, chunk, S, mat_stride, u, scratch); };
+    if (nrhs <= 6)
+        go(k_rhs_f64<6>);
+    else if (nrhs <= 8)
+        go(k_rhs_f64<8>);
+    else if (nrhs <= 10)
+        go(k_rhs_f64<10>);
     else if (nrhs <= 16)
-        k_rhs_f64<16><<<grid, 128, 0, s>>>(N, nrhs, S, mat_stride, u, rhs);
+        go(k_rhs_f64<16>);
     else
-        k_rhs_f64<32><<<grid, 128, 0, s>>>(N, nrhs, S, mat_stride, u, rhs);
+        go(k_rhs_f64<32>);
+    const size_t n = (size_t)F * nrhs * N;
+    k_rhs_sum<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, nz, scratch, rhs);
 }
 
 // ------------------------------------------------------------------ forces

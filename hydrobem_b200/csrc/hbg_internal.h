@@ -302,8 +302,10 @@ inline long long& last_surrogate_pairs() {
 void launch_boundary(const PanelsView& pv, int F, const FreqInfo* fi, int H, const double* heads, double depth,
                      double grav, double2* u, double2* phiI, cudaStream_t s);
 // rhs[F][nrhs][N] = -S u
+// (scratch: rhs_f64_scratch bytes)
 void launch_rhs_f64(int N, int F, int nrhs, const double2* S, size_t mat_stride, const double2* u, double2* rhs,
-                    cudaStream_t s);
+                    double2* scratch, cudaStream_t s);
+size_t rhs_f64_scratch(int N, int F, int nrhs);
 // field points: the fin-point planes of the panels then the P points ([F][FP_PLANES][N + P]); the elevation
 // or p / (rho g) at each point, radiation [F][P][D], incident, scattered and total [F][P][H]
 void launch_field_fin(const PanelsView& pv, const double* pts, int P, int F, const FdParams* fd, double* fq,

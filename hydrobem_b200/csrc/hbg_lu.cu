@@ -15,6 +15,10 @@ namespace hbg {
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// x - a b by two dependent multiply-adds a component
+__device__ __forceinline__ double2 cfms(double2 x, double2 a, double2 b) {
+    return make_double2(fma(a.y, b.y, fma(-a.x, b.x, x.x)), fma(-a.y, b.x, fma(-a.x, b.y, x.y)));
+}
 __device__ __forceinline__ double cabs2(double2 a) { return a.x * a.x + a.y * a.y; }
 
 // Blocking of the factorization: panels of LU_NB columns, each factored recursively (halves) down to
@@ -274,7 +278,7 @@ __global__ void __launch_bounds__(LuStrip<W>::T) k_lu_strip(int N, int c0, int w
         const double2 l = none ? make_double2(0.0, 0.0) : cmul(a[0], prow[0]);
         if (active) sh.L[j][tid] = l;
 #pragma unroll
-        for (int c = 0; c + 1 < R; c++) a[c] = csub(a[c + 1], cmul(l, prow[c + 2]));
+        for (int c = 0; c + 1 < R; c++) a[c] = cfms(a[c + 1], l, prow[c + 2]);
     };
     // (half of the columns held from the middle on; more bodies cost more instruction fetches than they save)
     int j = 0;
@@ -425,7 +429,7 @@ __global__ void __launch_bounds__(512) k_lu_trsm(int N, int c0, int n1, int cb, 
                         if (r > p && r < n1) {
                             const double2 l = Lc[base + r];
 #pragma unroll
-                            for (int c = 0; c < CPW; c++) x[c][q] = csub(x[c][q], cmul(l, xp[c]));
+                            for (int c = 0; c < CPW; c++) x[c][q] = cfms(x[c][q], l, xp[c]);
                         }
                     }
                 }
@@ -451,7 +455,7 @@ __global__ void __launch_bounds__(512) k_lu_trsm(int N, int c0, int n1, int cb, 
                         if (r < p) {
                             const double2 u = Lc[uoff(p) + r];
 #pragma unroll
-                            for (int c = 0; c < CPW; c++) x[c][q] = csub(x[c][q], cmul(u, xp[c]));
+                            for (int c = 0; c < CPW; c++) x[c][q] = cfms(x[c][q], u, xp[c]);
                         }
                     }
                 }
@@ -467,10 +471,10 @@ __global__ void __launch_bounds__(512) k_lu_trsm(int N, int c0, int n1, int cb, 
     }
 }
 
-template <bool UPPER>
-static void launch_lu_trsm(int N, int F, int c0, int n1, int cb, int ce, const double2* L, size_t lstride, double2* X,
-                           size_t xstride, cudaStream_t s) {
-    constexpr int CPW = 4, threads = 512, nw = threads / 32;
+template <bool UPPER, int CPW>
+static void launch_lu_trsm_cpw(int N, int F, int c0, int n1, int cb, int ce, const double2* L, size_t lstride, double2* X,
+                               size_t xstride, cudaStream_t s) {
+    constexpr int threads = 512, nw = threads / 32;
     const int cols = ce - cb;
     const size_t sm = sizeof(double2) * (size_t)n1 * (UPPER ? n1 + 1 : n1 - 1) / 2;
     // each CTA loads the triangle once and walks many columns: a few CTAs per matrix
@@ -482,6 +486,18 @@ static void launch_lu_trsm(int N, int F, int c0, int n1, int cb, int ce, const d
         k_lu_trsm<2, CPW, UPPER><<<g, threads, sm, s>>>(N, c0, n1, cb, ce, L, lstride, X, xstride);
     else
         k_lu_trsm<4, CPW, UPPER><<<g, threads, sm, s>>>(N, c0, n1, cb, ce, L, lstride, X, xstride);
+}
+// A step of a column's chain is a shuffle and its rows' FP64 operations, which for four columns a warp take longer than
+// the chain itself: one column a warp for the few columns of the right-hand sides and of a panel's inner solves.  The
+// substitution, ms with four columns a warp / one: 9 systems of order 645 and 9 columns 0.74 / 0.57, 8 of order 4096 and
+// 10 columns 5.2 / 4.35.
+template <bool UPPER>
+static void launch_lu_trsm(int N, int F, int c0, int n1, int cb, int ce, const double2* L, size_t lstride, double2* X,
+                           size_t xstride, cudaStream_t s) {
+    if (ce - cb <= 64)
+        launch_lu_trsm_cpw<UPPER, 1>(N, F, c0, n1, cb, ce, L, lstride, X, xstride, s);
+    else
+        launch_lu_trsm_cpw<UPPER, 4>(N, F, c0, n1, cb, ce, L, lstride, X, xstride, s);
 }
 
 // ------------------------------------------------------------------ trailing update on FP64 warp MMA
@@ -883,6 +899,10 @@ static void lu_f64_attributes() {
     cudaFuncSetAttribute(k_lu_trsm<4, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(double2) * LU_NB * (LU_NB - 1) / 2));
     cudaFuncSetAttribute(k_lu_trsm<4, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(double2) * LU_NB * (LU_NB + 1) / 2));
+    cudaFuncSetAttribute(k_lu_trsm<4, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(double2) * LU_NB * (LU_NB - 1) / 2));
+    cudaFuncSetAttribute(k_lu_trsm<4, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(double2) * LU_NB * (LU_NB + 1) / 2));
 }
 
