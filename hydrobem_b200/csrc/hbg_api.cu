@@ -467,7 +467,7 @@ static std::vector<int32_t> spatial_order(const double* v, int64_t n) {
         x = (x | (x << 2)) & 0x09249249ull;
         return x;
     };
-    std::vector<std::pair<uint64_t, int32_t>> key((size_t)n);
+    std::vector<uint32_t> key((size_t)n);
     for (int64_t j = 0; j < n; j++) {
         uint64_t code = 0;
         for (int d = 0; d < 3; d++) {
@@ -475,11 +475,18 @@ static std::vector<int32_t> spatial_order(const double* v, int64_t n) {
             const uint64_t q = span > 0.0 ? (uint64_t)std::min(1023.0, std::floor((c[3 * (size_t)j + d] - lo[d]) / span * 1023.0)) : 0;
             code |= spread(q) << d;
         }
-        key[(size_t)j] = {code, (int32_t)j};
+        key[(size_t)j] = (uint32_t)code;
     }
-    std::stable_sort(key.begin(), key.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-    std::vector<int32_t> a((size_t)n);
-    for (int64_t j = 0; j < n; j++) a[(size_t)j] = key[(size_t)j].second;
+    // a stable radix sort on the 30 bits, ten a pass
+    std::vector<int32_t> a((size_t)n), b((size_t)n);
+    for (int64_t j = 0; j < n; j++) a[(size_t)j] = (int32_t)j;
+    for (int shift = 0; shift < 30; shift += 10) {
+        size_t count[1025] = {};
+        for (int64_t j = 0; j < n; j++) count[((key[(size_t)j] >> shift) & 1023) + 1]++;
+        for (int i = 0; i < 1024; i++) count[i + 1] += count[i];
+        for (int64_t j = 0; j < n; j++) b[count[(key[(size_t)a[(size_t)j]] >> shift) & 1023]++] = a[(size_t)j];
+        a.swap(b);
+    }
     return a;
 }
 
@@ -666,21 +673,28 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
     dwork.alloc(sizeof(int32_t) * 2 * work_cap);
     dnwork.alloc(2 * sizeof(int32_t));  // [adaptive worklist size, queue cursor]
     const int32_t big = PANELS_VALID;
-    // page-locked: [first invalid panel, adaptive worklist size]
-    // [first invalid panel, adaptive worklist size, that of the field points]
-    int32_t* hflags = static_cast<int32_t*>(ws.host(HS_FLAGS, 3 * sizeof(int32_t)));
-    if (!hflags) throw Failure{HB_ERR_INTERNAL, "page-locked host memory could not be allocated", body_index};
+    // page-locked: [first invalid panel, adaptive worklist size, that of the field points], the hydrostatics records
+    // behind them; and the panels on their way to the device (every solve waits for its stream before it returns)
+    int32_t* hflags = static_cast<int32_t*>(ws.host(HS_FLAGS, 16 + sizeof(double) * nbod * HBG_HS));
+    double* hpanels = static_cast<double*>(ws.host(HS_PANELS, (sizeof(double) * 12 + 3 * sizeof(int32_t)) * (size_t)N));
+    if (!hflags || !hpanels) throw Failure{HB_ERR_INTERNAL, "page-locked host memory could not be allocated", body_index};
+    double* hhydro = reinterpret_cast<double*>(hflags + 4);
+    int32_t *hkind = reinterpret_cast<int32_t*>(hpanels + 12 * (size_t)N), *horig = hkind + N, *hbody = horig + N;
+    memcpy(hpanels, pr.body.vertices, sizeof(double) * 12 * N);
+    memcpy(hkind, kinds.data(), sizeof(int32_t) * N);
+    if (!orig.empty()) memcpy(horig, orig.data(), sizeof(int32_t) * N);
+    if (multi) memcpy(hbody, pr.body.panel_body, sizeof(int32_t) * N);
     double* prof = g_profile;
     bool statics_ran = false;
     auto run_statics = [&]() {
         if (!solve_begin().recorded) solve_begin().record(s);
-        CUDA_OK(cudaMemcpyAsync(dverts.p, pr.body.vertices, sizeof(double) * 12 * N, cudaMemcpyHostToDevice, s));
-        CUDA_OK(cudaMemcpyAsync(dkind.p, kinds.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
+        CUDA_OK(cudaMemcpyAsync(dverts.p, hpanels, sizeof(double) * 12 * N, cudaMemcpyHostToDevice, s));
+        CUDA_OK(cudaMemcpyAsync(dkind.p, hkind, sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
         CUDA_OK(cudaMemcpyAsync(dbad.p, &big, sizeof big, cudaMemcpyHostToDevice, s));
         if (!orig.empty())
-            CUDA_OK(cudaMemcpyAsync(dorig.p, orig.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
+            CUDA_OK(cudaMemcpyAsync(dorig.p, horig, sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
         if (multi)
-            CUDA_OK(cudaMemcpyAsync(dpbody.p, pr.body.panel_body, sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
+            CUDA_OK(cudaMemcpyAsync(dpbody.p, hbody, sizeof(int32_t) * N, cudaMemcpyHostToDevice, s));
         if (pr.body.rotation_centers)
             CUDA_OK(cudaMemcpyAsync(drcen.p, pr.body.rotation_centers, sizeof(double) * 3 * nbod,
                                     cudaMemcpyHostToDevice, s));
@@ -708,6 +722,8 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
                                 rigid && rigid->damping ? ext + DD2 : nullptr, opt.density, opt.gravity, hs, mm,
                                 mm + DD2, mm + 2 * DD2, s);
             g_launches++;
+            if (pr.out.hydrostatics)
+                CUDA_OK(cudaMemcpyAsync(hhydro, hs, sizeof(double) * nbod * HBG_HS, cudaMemcpyDeviceToHost, s));
         }
         CUDA_OK(cudaMemsetAsync(dnwork.p, 0, 2 * sizeof(int32_t), s));
         P.begin(s);
@@ -751,18 +767,21 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         if (hflags[1] > work_cap || hflags[2] > work_cap)
             throw Failure{HB_ERR_INTERNAL, "adaptive log-integral worklist overflow", body_index};
     };
-    // the mixed form's assembly kernels skip their work on invalid panels (the flag in device memory),
-    // so that its solve runs without a host wait until the end; the FP64 form waits here
+    // the hydrostatics records, once the stream has passed the statics
+    auto hydro_out = [&]() {
+        if (pr.out.hydrostatics) memcpy(pr.out.hydrostatics, hhydro, sizeof(double) * nbod * HBG_HS);
+    };
+    // the assembly (and field point) kernels skip their work on invalid panels (the flag in device memory), so
+    // that a solve runs without a host wait until the end of its first batch
     PanelsView pv{N, dplanes.as<double>(), dkind.as<int32_t>(), dbad.as<int32_t>(),
                   multi ? dpbody.as<int32_t>() : nullptr, pr.body.rotation_centers ? drcen.as<double>() : nullptr, nbod, G};
-    if (F == 0 || opt.precision != HBG_MIXED) {
+    if (F == 0) {
         run_statics();
         CUDA_OK(cudaStreamSynchronize(s));
         profiler().flush();
         statics_check();
-        if (pr.out.hydrostatics)
-            CUDA_OK(cudaMemcpy(pr.out.hydrostatics, dhyd.p, sizeof(double) * nbod * HBG_HS, cudaMemcpyDeviceToHost));
-        if (F == 0) return;
+        hydro_out();
+        return;
     }
     const int nrhs = D + H;
     if (opt.precision == HBG_MIXED) {
@@ -777,8 +796,7 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         if (e == cudaSuccess) statics_check();
         if (rc != 0) throw Failure{rc, msg, body_index, fq};
         CUDA_OK(e);
-        if (pr.out.hydrostatics)
-            CUDA_OK(cudaMemcpy(pr.out.hydrostatics, dhyd.p, sizeof(double) * nbod * HBG_HS, cudaMemcpyDeviceToHost));
+        hydro_out();
         if (!fallback.empty()) {
             // the frequencies whose refinement did not converge, solved again by the FP64 form (pivoted LU)
             const size_t nf = fallback.size(), DDo = (size_t)D * D, HD = (size_t)H * 2 * D;
@@ -860,21 +878,28 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         int dev_b = 0;
         cudaGetDevice(&dev_b);
         BatchChoice& c = last[dev_b < 0 || dev_b >= 16 ? 0 : dev_b];
-        const bool same = c.N == N && c.G == G && c.nrhs == nrhs && c.fin == (int)fin && c.F == F &&
-                          c.max_batch == opt.max_batch && c.budget == hbm_budget();
-        const size_t mats = NN * G * (size_t)std::max(c.B, 0);
-        if (same && c.B > 0 && ws.bytes[WS_S] >= sizeof(double2) * mats && ws.bytes[WS_A] >= sizeof(double2) * mats) {
-            B = c.B;
+        const size_t all = sizeof(double2) * NN * G * (size_t)F;
+        if (ws.bytes[WS_S] >= all && ws.bytes[WS_A] >= all && per_freq * F <= ws.held() + ((size_t)1 << 30)) {
+            // every frequency fits the buffers held (the same problem again, or another of a batch)
+            B = opt.max_batch > 0 ? std::min(F, (int)opt.max_batch) : F;
         } else {
-            size_t freeb = 0, totalb = 0;
-            CUDA_OK(cudaMemGetInfo(&freeb, &totalb));
-            const size_t reusable = ws.bytes[WS_S] + ws.bytes[WS_A];
-            size_t avail = (size_t)(0.85 * (double)(freeb + reusable));
-            if (hbm_budget() > 0) avail = std::min(avail, hbm_budget());
-            B = (int)std::max<size_t>(1, avail / per_freq);
-            if (opt.max_batch > 0) B = std::min(B, (int)opt.max_batch);
-            B = std::min(B, F);
-            c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, hbm_budget()};
+            const size_t budget = hbm_budget()();
+            const bool same = c.N == N && c.G == G && c.nrhs == nrhs && c.fin == (int)fin && c.F == F &&
+                              c.max_batch == opt.max_batch && c.budget == budget;
+            const size_t mats = NN * G * (size_t)std::max(c.B, 0);
+            if (same && c.B > 0 && ws.bytes[WS_S] >= sizeof(double2) * mats && ws.bytes[WS_A] >= sizeof(double2) * mats) {
+                B = c.B;
+            } else {
+                size_t freeb = 0, totalb = 0;
+                CUDA_OK(cudaMemGetInfo(&freeb, &totalb));
+                const size_t reusable = ws.bytes[WS_S] + ws.bytes[WS_A];
+                size_t avail = (size_t)(0.85 * (double)(freeb + reusable));
+                if (budget > 0) avail = std::min(avail, budget);
+                B = (int)std::max<size_t>(1, avail / per_freq);
+                if (opt.max_batch > 0) B = std::min(B, (int)opt.max_batch);
+                B = std::min(B, F);
+                c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, budget};
+            }
         }
     }
     const size_t BS = (size_t)B * G;  // systems per batch
@@ -925,8 +950,13 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
     int32_t* herr = info + BS;
     std::vector<FreqInfo> fi(B);
     std::vector<FdParams> fdh(B);
+    run_statics();
     for (int f0 = 0; f0 < F; f0 += B) {
-        if (opt.cancel && *opt.cancel) throw Failure{HB_ERR_CANCELLED, "the solve was cancelled", body_index, f0};
+        if (opt.cancel && *opt.cancel) {
+            cudaStreamSynchronize(s);
+            statics_check();  // an invalid panel comes first
+            throw Failure{HB_ERR_CANCELLED, "the solve was cancelled", body_index, f0};
+        }
         const int nb = std::min(B, F - f0), ns = nb * G;
         for (int i = 0; i < nb; i++) {
             double w = pr.omegas[f0 + i], K = w * w / opt.gravity;
@@ -1049,6 +1079,10 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         CUDA_OK(cudaStreamSynchronize(s));
         CUDA_OK(cudaGetLastError());
         profiler().flush();
+        if (f0 == 0) {
+            statics_check();
+            hydro_out();
+        }
         const double* hb = reinterpret_cast<const double*>(hout);
         const double* hA = hb;
         const size_t DD = (size_t)D * D;
@@ -1238,11 +1272,20 @@ static void solve_concurrent(const HbgProblem* problems, int64_t n, const HbgOpt
     // the calling thread's own buffers (from earlier one-after-another solves) are freed: the pipelines
     // share the device memory, and a solve on this thread allocates again what it needs
     workspace().release();
-    size_t freeb = 0, totalb = 0;
-    CUDA_OK(cudaMemGetInfo(&freeb, &totalb));
     size_t reusable = 0;  // the buffers of the pipelines this call uses (the others keep theirs)
     for (int w = 0; w < K; w++) reusable += g_pool_held[dev][w].load();
-    const size_t budget = (size_t)(0.85 * (double)(freeb + reusable) / K);
+    // each pipeline's share, from the memory free when the first of them asks and what they held at the call's start
+    std::mutex bm;
+    size_t share = 0;
+    const std::function<size_t()> budget = [&]() {
+        std::lock_guard<std::mutex> lk(bm);
+        if (share == 0) {
+            size_t freeb = 0, totalb = 0;
+            CUDA_OK(cudaMemGetInfo(&freeb, &totalb));
+            share = std::max<size_t>(1, (size_t)(0.85 * (double)(freeb + reusable) / K));
+        }
+        return share;
+    };
     std::vector<PipelineStats> stats((size_t)K);
     std::vector<cudaEvent_t> ends((size_t)K, nullptr);
     cudaStream_t s0;
@@ -1265,7 +1308,7 @@ static void solve_concurrent(const HbgProblem* problems, int64_t n, const HbgOpt
     };
     std::function<void(int)> job = [&](int w) {
         PipelineStats& st = stats[(size_t)w];
-        hbm_budget() = budget;
+        hbm_budget().ask = &budget;
         for (int i = 0; i < 6; i++) g_profile[i] = 0.0;
         g_launches = 0;
         last_fallback_count() = 0;
@@ -1314,7 +1357,7 @@ static void solve_concurrent(const HbgProblem* problems, int64_t n, const HbgOpt
         for (int i = 0; i < KF_COUNT; i++) st.kms[i] = P.ms[i], st.kwork[i] = P.work[i], st.klaunches[i] = P.launches[i];
         st.held = workspace().held();
         g_pool_held[dev][w].store(st.held);
-        hbm_budget() = 0;
+        hbm_budget().ask = nullptr;
     };
     pool.run(K, job);
     for (auto& e : ends) cudaStreamWaitEvent(s0, e, 0);
@@ -1341,6 +1384,40 @@ static void solve_concurrent(const HbgProblem* problems, int64_t n, const HbgOpt
     cudaEventDestroy(e1);
     cudaStreamDestroy(s0);
     if (failed.load()) throw first;
+}
+
+// The stream and timing events of this thread's one-after-another solves, per device: kept across calls (creating and
+// destroying them took a small solve 60 us), given back by hbg_release_workspace and at the thread's end.
+struct CallStream {
+    cudaStream_t s = nullptr;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    void release() {
+        if (s) cudaStreamDestroy(s);
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+        s = nullptr;
+        e0 = e1 = nullptr;
+    }
+    ~CallStream() { release(); }
+};
+static CallStream& call_stream_slot(int dev) {
+    static thread_local CallStream t[16];
+    return t[dev];
+}
+static CallStream& call_stream(int dev) {
+    if (dev < 0 || dev >= 16) throw Failure{HB_ERR_ARGUMENT, "device ordinal out of range"};
+    CallStream& c = call_stream_slot(dev);
+    if (!c.s) {
+        try {
+            CUDA_OK(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
+            CUDA_OK(cudaEventCreate(&c.e0));
+            CUDA_OK(cudaEventCreate(&c.e1));
+        } catch (...) {
+            c.release();
+            throw;
+        }
+    }
+    return c;
 }
 
 extern "C" HbStatus hbg_solve_batch(const HbgProblem* problems, int64_t n_problems, const HbgOptions* opt) {
@@ -1393,11 +1470,9 @@ extern "C" HbStatus hbg_solve_batch(const HbgProblem* problems, int64_t n_proble
                 for (int w = 0; w < 8; w++) g_pool_held[opt->device][w].store(0);
             }
         }
-        cudaStream_t s;
-        CUDA_OK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-        cudaEvent_t e0, e1;
-        cudaEventCreate(&e0);
-        cudaEventCreate(&e1);
+        CallStream& cs = call_stream(opt->device);
+        cudaStream_t s = cs.s;
+        const cudaEvent_t e0 = cs.e0, e1 = cs.e1;
         cudaEventRecord(e0, s);
         phase_timers().flush();
         solve_begin().recorded = false;
@@ -1407,9 +1482,6 @@ extern "C" HbStatus hbg_solve_batch(const HbgProblem* problems, int64_t n_proble
         } catch (...) {
             cudaStreamSynchronize(s);
             phase_timers().flush();
-            cudaStreamDestroy(s);
-            cudaEventDestroy(e0);
-            cudaEventDestroy(e1);
             throw;
         }
         cudaEventRecord(e1, s);
@@ -1419,9 +1491,6 @@ extern "C" HbStatus hbg_solve_batch(const HbgProblem* problems, int64_t n_proble
         cudaEventElapsedTime(&ms, solve_begin().recorded ? solve_begin().event() : e0,
                              solve_end().recorded ? solve_end().event() : e1);
         g_profile[5] = ms;
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        cudaStreamDestroy(s);
         return HB_OK;
     } catch (const Failure& f) {
         return fail(f);
@@ -1460,6 +1529,7 @@ extern "C" HbStatus hbg_release_workspace(void) {
             cudaGetDevice(&cur);
             cudaSetDevice(d);
             g_ws[d]->release();
+            call_stream_slot(d).release();
             cudaSetDevice(cur);
         }
     // and the buffers of the device's pipelines (concurrent solves)

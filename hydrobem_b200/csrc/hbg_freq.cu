@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(256) k_field(PanelsView pv, const double* __re
                                                double2* __restrict__ frad, double2* __restrict__ finc,
                                                double2* __restrict__ fsca, double2* __restrict__ fdif) {
     __shared__ double2 red[8][FIELD_COLS];
+    if (pv.invalid()) return;  // invalid panels: the solve reports them
     const int p = blockIdx.x, f = blockIdx.y, N = pv.N, nrad = 6 * pv.nbod, nrhs = nrad + H;
     const double x[3] = {pts[3 * p], pts[3 * p + 1], pts[3 * p + 2]};
     const FreqInfo info = fi[f];

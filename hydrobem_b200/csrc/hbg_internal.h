@@ -1,7 +1,8 @@
 // hbg_internal.h -- host-side declarations shared by the translation units of libhydrobem_gpu.
 #pragma once
-#include <vector>
 #include <cstdint>
+#include <functional>
+#include <vector>
 #include <cuda_runtime.h>
 
 #include "hbg_device.cuh"
@@ -74,7 +75,7 @@ enum WsSlot {
 
 // Page-locked host buffers of a solve: a device-to-host copy into pageable memory waits for the
 // stream, one into these does not.
-enum HostSlot { HS_FLAGS = 0, HS_NORMS, HS_OUT, HS_COUNT };
+enum HostSlot { HS_FLAGS = 0, HS_NORMS, HS_OUT, HS_PANELS, HS_COUNT };
 
 struct Workspace {
     void* p[WS_COUNT] = {};
@@ -182,9 +183,14 @@ struct PhaseTimers {
     }
 };
 // The device memory the solves of this host thread may hold in their workspace (0: no limit beyond 85 %
-// of the free memory): a pipeline's share when several problems are solved at once.
-inline size_t& hbm_budget() {
-    static thread_local size_t b = 0;
+// of the free memory): a pipeline's share when several problems are solved at once.  Asked for only by a solve whose
+// matrices do not fit the buffers held already (the answer needs cudaMemGetInfo, which can take milliseconds).
+struct HbmBudget {
+    const std::function<size_t()>* ask = nullptr;
+    size_t operator()() const { return ask ? (*ask)() : 0; }
+};
+inline HbmBudget& hbm_budget() {
+    static thread_local HbmBudget b;
     return b;
 }
 

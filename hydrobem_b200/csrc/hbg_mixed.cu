@@ -217,22 +217,30 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
         int dev_b = 0;
         cudaGetDevice(&dev_b);
         BatchChoice& c = last[dev_b < 0 || dev_b >= 16 ? 0 : dev_b];
-        const bool same = c.N == N && c.G == G && c.nrhs == nrhs && c.fin == (int)fin && c.F == F &&
-                          c.max_batch == opt.max_batch && c.budget == hbm_budget();
-        const size_t mats = MB * (size_t)std::max(c.B, 0) * G * 4;
-        if (same && c.B > 0 && ws.bytes[WS_S32] >= mats && ws.bytes[WS_W] >= mats) {
-            B = c.B;
+        const size_t all = MB * (size_t)F * G * 4;
+        if (ws.bytes[WS_S32] >= all && ws.bytes[WS_A32] >= all && ws.bytes[WS_W] >= all &&
+            per * F <= ws.held() + ((size_t)1 << 30)) {
+            // every frequency fits the buffers held (the same problem again, or another of a batch)
+            B = opt.max_batch > 0 ? std::min(F, (int)opt.max_batch) : F;
         } else {
-            size_t freeb = 0, totalb = 0;
-            if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess)
-                MIXED_FAIL(HB_ERR_INTERNAL, "cudaMemGetInfo failed", -1);
-            freeb += ws.bytes[WS_S32] + ws.bytes[WS_A32] + ws.bytes[WS_W] + ws.bytes[WS_DINV];
-            size_t avail = (size_t)(0.85 * (double)freeb);
-            if (hbm_budget() > 0) avail = std::min(avail, hbm_budget());
-            B = (int)std::max<size_t>(1, avail / per);
-            if (opt.max_batch > 0) B = std::min(B, (int)opt.max_batch);
-            B = std::min(B, F);
-            c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, hbm_budget()};
+            const size_t budget = hbm_budget()();
+            const bool same = c.N == N && c.G == G && c.nrhs == nrhs && c.fin == (int)fin && c.F == F &&
+                              c.max_batch == opt.max_batch && c.budget == budget;
+            const size_t mats = MB * (size_t)std::max(c.B, 0) * G * 4;
+            if (same && c.B > 0 && ws.bytes[WS_S32] >= mats && ws.bytes[WS_W] >= mats) {
+                B = c.B;
+            } else {
+                size_t freeb = 0, totalb = 0;
+                if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess)
+                    MIXED_FAIL(HB_ERR_INTERNAL, "cudaMemGetInfo failed", -1);
+                freeb += ws.bytes[WS_S32] + ws.bytes[WS_A32] + ws.bytes[WS_W] + ws.bytes[WS_DINV];
+                size_t avail = (size_t)(0.85 * (double)freeb);
+                if (budget > 0) avail = std::min(avail, budget);
+                B = (int)std::max<size_t>(1, avail / per);
+                if (opt.max_batch > 0) B = std::min(B, (int)opt.max_batch);
+                B = std::min(B, F);
+                c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, budget};
+            }
         }
     }
     const size_t nblk = (size_t)Np / NBL;
