@@ -338,37 +338,36 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     const int nz = (Nm + GEMV_CHUNK - 1) / GEMV_CHUNK;
     double2* part = (double2*)ws.get(WS_PART, (size_t)nz * BS * nrhs * Nm * 16);
     if (!part) MIXED_FAIL(HB_ERR_INTERNAL, "device memory allocation failed for the mixed form", -1);
-    for (auto fn : {(const void*)k_cgemv_tma<4>, (const void*)k_cgemv_tma<8>, (const void*)k_cgemv_tma<10>,
-                    (const void*)k_cgemv_tma<12>, (const void*)k_cgemv_tma<16>})
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gv_smem_bytes<16>());
-    // the column width of a chunk of w right-hand sides (the products are FP64-FMA bound: the padded
-    // columns of the last chunk cost as much as real ones)
+    // the column width of a chunk of w right-hand sides of the FP32 product (its padded columns cost as much as real ones)
     auto chunk_width = [](int w) { return w <= 4 ? 4 : w <= 8 ? 8 : w <= 10 ? 10 : w <= 12 ? 12 : 16; };
-    // the TMA form (its maps cover exactly the matrices and vectors of the batch), beyond 16 right-hand
-    // sides in column chunks of 16 (the matrix streamed once a chunk); the register form if a map fails
+    // the FP64 product by TMA and DMMA (its maps cover exactly the matrices and vectors of the batch), all right-hand
+    // sides at once in tiles of four; the register form if a map fails
+    auto dmma = [&](auto tiles, const CUtensorMap& mM, const CUtensorMap& mX, dim3 g, int nb, cudaStream_t s) {
+        constexpr int NT = decltype(tiles)::value;
+        cudaFuncSetAttribute(k_cgemv_dmma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GdCfg<NT>::SMEM);
+        k_cgemv_dmma<NT><<<g, GD_THREADS, GdCfg<NT>::SMEM, s>>>(mM, mX, Nm, nrhs, part, nb, err);
+    };
     auto gemv_tma = [&](const float* Mm, const double2* xv, int ldx, int nb, int nzt, cudaStream_t s) -> bool {
         CUtensorMap mM, mX;
         const uint64_t dm[4] = {(uint64_t)Np, (uint64_t)Np, 2, (uint64_t)nb};
         const uint64_t sm[3] = {(uint64_t)Np * 4, NP2 * 4, MB * 4};
         const uint32_t bm[4] = {GV_ROWS, GV_COLS, 1, 1};
-        if (!make_map_box(&mM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (void*)Mm, dm, sm, bm)) return false;
+        const int nt = std::max(2, (nrhs + 3) / 4);  // (one tile: padded to two, zeros beyond nrhs)
+        const uint64_t dx[4] = {2 * (uint64_t)ldx, (uint64_t)nrhs, (uint64_t)nb, 1};
+        const uint64_t sx[3] = {(uint64_t)ldx * 16, (uint64_t)nrhs * ldx * 16, (uint64_t)nb * nrhs * ldx * 16};
+        const uint32_t bx[4] = {2 * GV_COLS, (uint32_t)(4 * nt), 1, 1};
+        if (!make_map_box(&mM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (void*)Mm, dm, sm, bm) ||
+            !make_map_box(&mX, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void*)xv, dx, sx, bx))
+            return false;
         dim3 g((Nm + GV_ROWS - 1) / GV_ROWS, nb, nzt);
-        for (int c0 = 0; c0 < nrhs; c0 += 16) {
-            const int nr = chunk_width(std::min(16, nrhs - c0));
-            const uint64_t dx[4] = {2 * (uint64_t)ldx, (uint64_t)nrhs, (uint64_t)nb, 1};
-            const uint64_t sx[3] = {(uint64_t)ldx * 16, (uint64_t)nrhs * ldx * 16, (uint64_t)nb * nrhs * ldx * 16};
-            const uint32_t bx[4] = {2 * GV_COLS, (uint32_t)nr, 1, 1};
-            if (!make_map_box(&mX, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void*)xv, dx, sx, bx)) return false;
-            if (nr == 4)
-                k_cgemv_tma<4><<<g, GV_THREADS, gv_smem_bytes<4>(), s>>>(mM, mX, Nm, nrhs, c0, part, nb, err);
-            else if (nr == 8)
-                k_cgemv_tma<8><<<g, GV_THREADS, gv_smem_bytes<8>(), s>>>(mM, mX, Nm, nrhs, c0, part, nb, err);
-            else if (nr == 10)
-                k_cgemv_tma<10><<<g, GV_THREADS, gv_smem_bytes<10>(), s>>>(mM, mX, Nm, nrhs, c0, part, nb, err);
-            else if (nr == 12)
-                k_cgemv_tma<12><<<g, GV_THREADS, gv_smem_bytes<12>(), s>>>(mM, mX, Nm, nrhs, c0, part, nb, err);
-            else
-                k_cgemv_tma<16><<<g, GV_THREADS, gv_smem_bytes<16>(), s>>>(mM, mX, Nm, nrhs, c0, part, nb, err);
+        switch (nt) {
+            case 2: dmma(std::integral_constant<int, 2>(), mM, mX, g, nb, s); break;
+            case 3: dmma(std::integral_constant<int, 3>(), mM, mX, g, nb, s); break;
+            case 4: dmma(std::integral_constant<int, 4>(), mM, mX, g, nb, s); break;
+            case 5: dmma(std::integral_constant<int, 5>(), mM, mX, g, nb, s); break;
+            case 6: dmma(std::integral_constant<int, 6>(), mM, mX, g, nb, s); break;
+            case 7: dmma(std::integral_constant<int, 7>(), mM, mX, g, nb, s); break;
+            default: dmma(std::integral_constant<int, 8>(), mM, mX, g, nb, s); break;
         }
         return true;
     };
@@ -399,15 +398,15 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             const int nr = nrc[last];
             mD = mDc[last];
             if (nr == 4)
-                k_cgemv32_tma<4><<<g, GV_THREADS, gv32_smem_bytes<4>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
+                k_cgemv32_tma<4><<<g, gv32_threads<4>(), gv32_smem_bytes<4>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
             else if (nr == 8)
-                k_cgemv32_tma<8><<<g, GV_THREADS, gv32_smem_bytes<8>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
+                k_cgemv32_tma<8><<<g, gv32_threads<8>(), gv32_smem_bytes<8>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
             else if (nr == 10)
-                k_cgemv32_tma<10><<<g, GV_THREADS, gv32_smem_bytes<10>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
+                k_cgemv32_tma<10><<<g, gv32_threads<10>(), gv32_smem_bytes<10>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
             else if (nr == 12)
-                k_cgemv32_tma<12><<<g, GV_THREADS, gv32_smem_bytes<12>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
+                k_cgemv32_tma<12><<<g, gv32_threads<12>(), gv32_smem_bytes<12>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
             else
-                k_cgemv32_tma<16><<<g, GV_THREADS, gv32_smem_bytes<16>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
+                k_cgemv32_tma<16><<<g, gv32_threads<16>(), gv32_smem_bytes<16>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
         }
         k_residual_reduce<true><<<dim3((unsigned)(((size_t)npair * Nm + 255) / 256), nb), 256, 0, s>>>(
             Nm, Np, nrhs, nb, nz_tma, part, rk, out);

@@ -850,11 +850,6 @@ __global__ void __launch_bounds__(128) k_cgemv_part(int N, int Np, size_t bstrid
             if (c < nrhs) part[(((size_t)z * F + f) * nrhs + c) * N + k] = acc[c];
 }
 
-// The same partial products with the matrix and vector tiles streamed by TMA: CTA of 256 rows k
-// (two a thread: t and t + 128, so each vector entry read from shared memory feeds both) over a
-// chunk of columns n, 16 columns per stage (both FP32 planes, 32 KB, and the 16 complex entries of
-// every right-hand side), GV_STAGES stages in flight from a producer warp, so the bytes in flight do
-// not depend on registers; FP64 accumulation as above.
 // Packed FP32 pairs (fma.rn.f32x2: two FP32 FMAs per instruction), here over two right-hand sides.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 f2pack(float a, float b) {
@@ -875,100 +870,121 @@ __device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) {
 
 constexpr int GV_ROWS = 256, GV_COLS = 16, GV_STAGES = 3, GV_CHUNK = 1024;
 constexpr int GV_WORKERS = GV_ROWS / 2;
-constexpr int GV_THREADS = GV_WORKERS + 32;
-template <int NR>
-__host__ __device__ constexpr size_t gv_tx_bytes() {  // bytes one stage receives
-    return (size_t)2 * GV_COLS * GV_ROWS * 4 + (size_t)NR * GV_COLS * 16;
-}
-template <int NR>
-__host__ __device__ constexpr size_t gv_stage_bytes() {  // stage stride in shared memory (1024-byte aligned)
-    return (gv_tx_bytes<NR>() + 1023) / 1024 * 1024;
-}
-template <int NR>
-__host__ __device__ constexpr size_t gv_smem_bytes() {
-    return 1024 + GV_STAGES * gv_stage_bytes<NR>() + 128;
-}
 
-template <int NR>
-__global__ void __launch_bounds__(GV_THREADS) k_cgemv_tma(const __grid_constant__ CUtensorMap mapM,
-                                                             const __grid_constant__ CUtensorMap mapX, int N,
-                                                             int nrhs, int c0, double2* __restrict__ part, int F,
-                                                             int* __restrict__ err) {
+// The same partial products on the FP64 tensor cores (mma.sync m8n8k4): the matrix and vector tiles streamed by TMA (16
+// columns a stage, both FP32 planes of 256 rows, 32 KB, and the 16 complex entries of every right-hand side) from a
+// producer warp, eight warps of 32 rows each.  Real columns 2 c and 2 c + 1 of the product are the real and imaginary
+// part of right-hand side c: C += Mr [Xr, Xi] + Mi [-Xi, Xr].  Lane (i, k) of a warp reads rows 4 i .. 4 i + 3 of column
+// k by one 16-byte load, row tile t taking rows 4 i + t, and each pair of vector entries serves four row tiles; all
+// right-hand sides in one pass over the matrix.  Bound by the FP64 pipe (4 FMA an entry and right-hand side at 37
+// TFLOP/s, NT tiles of 4 right-hand sides); the FMA form before it (a thread two rows, at most 16 right-hand sides a
+// pass) spent as long on its shared-memory loads.  Measured, ms, before / now: 40 matrices of order 4096 and 10
+// right-hand sides 2.39 / 2.03, 4 of order 12288 and 19 5.4 / 3.0, 5 of order 18496 and 14 12.1 / 6.7.
+constexpr int GD_THREADS = GV_ROWS + 32;  // eight MMA warps of 32 rows, the producer
+template <int NT>
+struct GdCfg {  // NT: tiles of four right-hand sides
+    static constexpr size_t TX = (size_t)2 * GV_COLS * GV_ROWS * 4 + (size_t)4 * NT * GV_COLS * 16;  // bytes of a stage
+    static constexpr size_t STAGE = (TX + 1023) / 1024 * 1024;
+    static constexpr int STAGES = NT <= 2 ? 3 : 4;  // two CTAs an SM, or one
+    static constexpr size_t SMEM = 1024 + STAGES * STAGE + 128;
+};
+template <int NT>
+__global__ void __launch_bounds__(GD_THREADS, NT <= 2 ? 2 : 1) k_cgemv_dmma(const __grid_constant__ CUtensorMap mapM,
+                                                              const __grid_constant__ CUtensorMap mapX, int N,
+                                                              int nrhs, double2* __restrict__ part, int F,
+                                                              int* __restrict__ err) {
+    using C = GdCfg<NT>;
     extern __shared__ uint8_t gv_raw[];
     uint8_t* base = align1024(gv_raw);
-    uint64_t* full = reinterpret_cast<uint64_t*>(base + GV_STAGES * gv_stage_bytes<NR>());
-    uint64_t* empty = full + GV_STAGES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(base + C::STAGES * C::STAGE);
+    uint64_t* empty = full + C::STAGES;
     const int f = blockIdx.y, z = blockIdx.z;
     const int k0 = blockIdx.x * GV_ROWS;
     const int nbeg = z * GV_CHUNK, nend = min(N, nbeg + GV_CHUNK);
     const int nst = (nend - nbeg + GV_COLS - 1) / GV_COLS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < GV_STAGES; s++) {
+        for (int s = 0; s < C::STAGES; s++) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], GV_WORKERS / 32);
+            tc::mbar_init(&empty[s], GV_ROWS / 32);
         }
         tc::fence_barrier_init();
     }
     __syncthreads();
-    if (warp == GV_WORKERS / 32) {
+    if (warp == GV_ROWS / 32) {
         if (lane == 0) {
             tc::prefetch_tensormap(&mapM);
             tc::prefetch_tensormap(&mapX);
             for (int si = 0; si < nst; si++) {
-                const int s = si % GV_STAGES;
-                if (si >= GV_STAGES && !tc::mbar_wait(&empty[s], ((si / GV_STAGES) - 1) & 1)) {
+                const int s = si % C::STAGES;
+                if (si >= C::STAGES && !tc::mbar_wait(&empty[s], ((si / C::STAGES) - 1) & 1)) {
                     atomicExch(err, 6);
                     break;
                 }
-                uint8_t* st = base + s * gv_stage_bytes<NR>();
+                uint8_t* st = base + s * C::STAGE;
                 const int n0 = nbeg + si * GV_COLS;
-                tc::mbar_arrive_expect_tx(&full[s], (uint32_t)gv_tx_bytes<NR>());
+                tc::mbar_arrive_expect_tx(&full[s], (uint32_t)C::TX);
                 tc::tma_load_4d(st, &mapM, &full[s], k0, n0, 0, f);
                 tc::tma_load_4d(st + GV_COLS * GV_ROWS * 4, &mapM, &full[s], k0, n0, 1, f);
-                tc::tma_load_4d(st + 2 * GV_COLS * GV_ROWS * 4, &mapX, &full[s], 2 * n0, c0, f, 0);
+                tc::tma_load_4d(st + 2 * GV_COLS * GV_ROWS * 4, &mapX, &full[s], 2 * n0, 0, f, 0);
             }
         }
         return;
     }
-    double2 acc[NR], acd[NR];  // rows k0 + t and k0 + t + GV_WORKERS
+    const int i = lane >> 2, kq = lane & 3;  // row group (and column of B), k of a step
+    double acc[4][NT][2];
 #pragma unroll
-    for (int c = 0; c < NR; c++) acc[c] = acd[c] = make_double2(0.0, 0.0);
-    const int t = threadIdx.x;
+    for (int t = 0; t < 4; t++)
+#pragma unroll
+        for (int c = 0; c < NT; c++) acc[t][c][0] = acc[t][c][1] = 0.0;
     for (int si = 0; si < nst; si++) {
-        const int s = si % GV_STAGES;
-        if (!tc::mbar_wait(&full[s], (si / GV_STAGES) & 1)) {
+        const int s = si % C::STAGES;
+        // One barrier of the eight warps a stage: one answer for all (and the lanes together again: the mma below wants
+        // them all), and every read of the stage before is done, so that one may be filled again.  An arrival of each
+        // warp behind its unrolled loop let a stage be filled while a last read of it was still to come.
+        if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[s], (si / C::STAGES) & 1))) {
             atomicExch(err, 7);
             break;
         }
-        const uint8_t* st = base + s * gv_stage_bytes<NR>();
-        const float* sMr = reinterpret_cast<const float*>(st);
-        const float* sMi = sMr + GV_COLS * GV_ROWS;
-        const double2* sx = reinterpret_cast<const double2*>(st + 2 * GV_COLS * GV_ROWS * 4);  // [NR][GV_COLS]
-        // columns beyond N are never read (the padding may hold anything)
-        const int lim = min(GV_COLS, nend - (nbeg + si * GV_COLS));
-#pragma unroll 2
-        for (int j = 0; j < lim; j++) {
-            const double mr = sMr[j * GV_ROWS + t], mi = sMi[j * GV_ROWS + t];
-            const double nr = sMr[j * GV_ROWS + t + GV_WORKERS], ni = sMi[j * GV_ROWS + t + GV_WORKERS];
+        if (si > 0 && lane == 0) tc::mbar_arrive(&empty[(si - 1) % C::STAGES]);
+        const uint8_t* st = base + s * C::STAGE;
+        const float* sM = reinterpret_cast<const float*>(st) + 32 * warp + 4 * i;
+        const double2* sx = reinterpret_cast<const double2*>(st + 2 * GV_COLS * GV_ROWS * 4);  // [4 NT][GV_COLS]
+        // columns beyond N take no part (the padding may hold anything)
+        const int lim = nend - (nbeg + si * GV_COLS);
+#pragma unroll(NT <= 5 ? 4 : 1)
+        for (int ks = 0; ks < GV_COLS / 4; ks++) {
+            const int k = 4 * ks + kq;
+            float4 mr = *reinterpret_cast<const float4*>(sM + k * GV_ROWS);
+            float4 mi = *reinterpret_cast<const float4*>(sM + (GV_COLS + k) * GV_ROWS);
+            if (k >= lim) mr = mi = make_float4(0.f, 0.f, 0.f, 0.f);
+            const double ar[4] = {mr.x, mr.y, mr.z, mr.w}, ai[4] = {mi.x, mi.y, mi.z, mi.w};
 #pragma unroll
-            for (int c = 0; c < NR; c++) {  // four fused multiply-adds a row (the pipe's limit)
-                const double2 v = sx[c * GV_COLS + j];
-                acc[c].x = fma(-mi, v.y, fma(mr, v.x, acc[c].x));
-                acc[c].y = fma(mi, v.x, fma(mr, v.y, acc[c].y));
-                acd[c].x = fma(-ni, v.y, fma(nr, v.x, acd[c].x));
-                acd[c].y = fma(ni, v.x, fma(nr, v.y, acd[c].y));
+            for (int c = 0; c < NT; c++) {
+                const double2 v = sx[(4 * c + (i >> 1)) * GV_COLS + k];  // right-hand side 4 c + i / 2
+                const double b1 = i & 1 ? v.y : v.x, b2 = i & 1 ? v.x : -v.y;
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                                 : "+d"(acc[t][c][0]), "+d"(acc[t][c][1])
+                                 : "d"(ar[t]), "d"(b1));
+#pragma unroll
+                for (int t = 0; t < 4; t++)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                                 : "+d"(acc[t][c][0]), "+d"(acc[t][c][1])
+                                 : "d"(ai[t]), "d"(b2));
             }
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&empty[s]);
     }
-    const int k = k0 + t, kd = k + GV_WORKERS;
+    // lane (i, kq) holds right-hand sides 4 c + kq of rows 4 i + t
+    const int row = k0 + 32 * warp + 4 * i;
 #pragma unroll
-    for (int c = 0; c < NR; c++)
-        if (c0 + c < nrhs) {
-            if (k < N) part[(((size_t)z * F + f) * nrhs + c0 + c) * N + k] = acc[c];
-            if (kd < N) part[(((size_t)z * F + f) * nrhs + c0 + c) * N + kd] = acd[c];
+    for (int c = 0; c < NT; c++)
+        if (4 * c + kq < nrhs) {
+            double2* o = part + (((size_t)z * F + f) * nrhs + 4 * c + kq) * N + row;
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+                if (row + t < N) o[t] = make_double2(acc[t][c][0], acc[t][c][1]);
         }
 }
 
@@ -991,11 +1007,23 @@ __host__ __device__ constexpr size_t gv32_smem_bytes() {
     return 1024 + GV_STAGES * gv32_stage_bytes<NR>() + 128;
 }
 
+// HV = 2: two groups of workers, each half of the columns of the same rows (the FP64 sums of 12 or 16 columns of two
+// rows take 128 registers and more, which left one CTA of four warps an SM).  ms of three products, one group / two: 5
+// matrices of order 18496 and 14 columns 10.1 / 6.7, 4 of order 12288 and 19 columns (chunks of 16 and 4) 3.3 / 2.9.
 template <int NR>
-__global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constant__ CUtensorMap mapM,
+__host__ __device__ constexpr int gv32_halves() {
+    return NR >= 12 ? 2 : 1;
+}
+template <int NR>
+__host__ __device__ constexpr int gv32_threads() {
+    return gv32_halves<NR>() * GV_WORKERS + 32;
+}
+template <int NR>
+__global__ void __launch_bounds__(gv32_threads<NR>()) k_cgemv32_tma(const __grid_constant__ CUtensorMap mapM,
                                                                const __grid_constant__ CUtensorMap mapD, int N,
                                                                int nrhs, int c0, double2* __restrict__ part, int F,
                                                                int* __restrict__ err) {
+    constexpr int HV = gv32_halves<NR>(), NH = NR / HV, WARPS = HV * GV_WORKERS / 32;
     extern __shared__ uint8_t gv_raw[];
     uint8_t* base = align1024(gv_raw);
     uint64_t* full = reinterpret_cast<uint64_t*>(base + GV_STAGES * gv32_stage_bytes<NR>());
@@ -1008,12 +1036,12 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
     if (threadIdx.x == 0) {
         for (int s = 0; s < GV_STAGES; s++) {
             tc::mbar_init(&full[s], 1);
-            tc::mbar_init(&empty[s], GV_WORKERS / 32);
+            tc::mbar_init(&empty[s], WARPS);
         }
         tc::fence_barrier_init();
     }
     __syncthreads();
-    if (warp == GV_WORKERS / 32) {
+    if (warp == WARPS) {
         if (lane == 0) {
             tc::prefetch_tensormap(&mapM);
             tc::prefetch_tensormap(&mapD);
@@ -1033,10 +1061,10 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
         }
         return;
     }
-    double2 acc[NR], acd[NR];  // rows k0 + t and k0 + t + GV_WORKERS
+    double2 acc[NH], acd[NH];  // rows k0 + t and k0 + t + GV_WORKERS
 #pragma unroll
-    for (int c = 0; c < NR; c++) acc[c] = acd[c] = make_double2(0.0, 0.0);
-    const int t = threadIdx.x;
+    for (int c = 0; c < NH; c++) acc[c] = acd[c] = make_double2(0.0, 0.0);
+    const int t = threadIdx.x % GV_WORKERS, h0 = threadIdx.x / GV_WORKERS * NH;  // row, first column
     for (int si = 0; si < nst; si++) {
         const int s = si % GV_STAGES;
         if (!tc::mbar_wait(&full[s], (si / GV_STAGES) & 1)) {
@@ -1046,11 +1074,11 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
         const uint8_t* st = base + s * gv32_stage_bytes<NR>();
         const float* sMr = reinterpret_cast<const float*>(st);
         const float* sMi = sMr + GV_COLS * GV_ROWS;
-        const float4* sd = reinterpret_cast<const float4*>(st + 2 * GV_COLS * GV_ROWS * 4);  // [NR / 2][GV_COLS]
+        const float4* sd = reinterpret_cast<const float4*>(st + 2 * GV_COLS * GV_ROWS * 4) + h0 / 2 * GV_COLS;  // [pair][GV_COLS]
         const int lim = min(GV_COLS, nend - (nbeg + si * GV_COLS));
-        f32x2 r0[NR / 2], i0[NR / 2], r1[NR / 2], i1[NR / 2];
+        f32x2 r0[NH / 2], i0[NH / 2], r1[NH / 2], i1[NH / 2];
 #pragma unroll
-        for (int c = 0; c < NR / 2; c++) r0[c] = i0[c] = r1[c] = i1[c] = f2pack(0.f, 0.f);
+        for (int c = 0; c < NH / 2; c++) r0[c] = i0[c] = r1[c] = i1[c] = f2pack(0.f, 0.f);
 #pragma unroll 4
         for (int j = 0; j < lim; j++) {
             const float mr = sMr[j * GV_ROWS + t], mi = sMi[j * GV_ROWS + t];
@@ -1058,7 +1086,7 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
             const f32x2 a0 = f2pack(mr, mr), b0 = f2pack(mi, mi), e0 = f2pack(-mi, -mi);
             const f32x2 a1 = f2pack(nr, nr), b1 = f2pack(ni, ni), e1 = f2pack(-ni, -ni);
 #pragma unroll
-            for (int c = 0; c < NR / 2; c++) {
+            for (int c = 0; c < NH / 2; c++) {
                 const float4 v = sd[c * GV_COLS + j];
                 const f32x2 vr = f2pack(v.x, v.y), vi = f2pack(v.z, v.w);
                 r0[c] = ffma2(e0, vi, ffma2(a0, vr, r0[c]));
@@ -1068,7 +1096,7 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
             }
         }
 #pragma unroll
-        for (int c = 0; c < NR; c++) {
+        for (int c = 0; c < NH; c++) {
             const float2 x0 = f2unpack(r0[c / 2]), y0 = f2unpack(i0[c / 2]), x1 = f2unpack(r1[c / 2]), y1 = f2unpack(i1[c / 2]);
             acc[c].x += (double)(c & 1 ? x0.y : x0.x);
             acc[c].y += (double)(c & 1 ? y0.y : y0.x);
@@ -1080,10 +1108,10 @@ __global__ void __launch_bounds__(GV_THREADS) k_cgemv32_tma(const __grid_constan
     }
     const int k = k0 + t, kd = k + GV_WORKERS;
 #pragma unroll
-    for (int c = 0; c < NR; c++)
-        if (c0 + c < nrhs) {
-            if (k < N) part[(((size_t)z * F + f) * nrhs + c0 + c) * N + k] = acc[c];
-            if (kd < N) part[(((size_t)z * F + f) * nrhs + c0 + c) * N + kd] = acd[c];
+    for (int c = 0; c < NH; c++)
+        if (c0 + h0 + c < nrhs) {
+            if (k < N) part[(((size_t)z * F + f) * nrhs + c0 + h0 + c) * N + k] = acc[c];
+            if (kd < N) part[(((size_t)z * F + f) * nrhs + c0 + h0 + c) * N + kd] = acd[c];
         }
 }
 
