@@ -939,9 +939,9 @@ __global__ void __launch_bounds__(GD_THREADS, NT <= 2 ? 2 : 1) k_cgemv_dmma(cons
         for (int c = 0; c < NT; c++) acc[t][c][0] = acc[t][c][1] = 0.0;
     for (int si = 0; si < nst; si++) {
         const int s = si % C::STAGES;
-        // One barrier of the eight warps a stage: one answer for all (and the lanes together again: the mma below wants
-        // them all), and every read of the stage before is done, so that one may be filled again.  An arrival of each
-        // warp behind its unrolled loop let a stage be filled while a last read of it was still to come.
+        // The vote brings the lanes together again (the mma wants them all).  A stage is handed back only behind the wait
+        // for the next: an arrival straight behind the unrolled loop let TMA overwrite a last vector entry still to be
+        // read by the queued mma (seen as 1e-2 errors of one right-hand side in one call of a hundred).
         if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[s], (si / C::STAGES) & 1))) {
             atomicExch(err, 7);
             break;
