@@ -1,7 +1,7 @@
 // hbg_mixed.cu -- the mixed-precision form of the frequency solve: the pair kernels in FP64 as in
 // the FP64 form, the matrices stored as complex64 (two FP32 planes), the LU on the tensor cores
 // (tcgen05 kind::tf32 and kind::f16, FP32 accumulation, no pivoting), the right-hand sides and the residuals
-// accumulated in FP64, and iterative refinement until the correction is below 1e-12 of the solution.
+// accumulated in FP64, and iterative refinement until the predicted error is below 1e-9 of the solution (IR_TOL).
 // The result is the solution of the complex64-rounded system (the reference's production path
 // stores its matrices in complex64 too, lo_frequency.rs:1-6).
 #include <cuda.h>

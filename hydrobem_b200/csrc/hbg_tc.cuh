@@ -1,6 +1,5 @@
 // hbg_tc.cuh -- Blackwell tensor-core building blocks: TMA tile loads, mbarriers with bounded
-// waits, TMEM allocation, tcgen05.mma (kind::tf32, FP32 accumulation in TMEM) and TMEM loads, and
-// the batched TF32 GEMM of the mixed-precision LU.
+// waits, TMEM allocation, tcgen05.mma (kind::tf32 and kind::f16, FP32 accumulation in TMEM) and TMEM loads.
 //
 // Every wait is bounded: after WAIT_LIMIT failed polls a thread records an error code in the
 // caller's flag and gives up; the host turns a nonzero flag into HB_ERR_INTERNAL.  No trap.
