@@ -821,9 +821,25 @@ struct LuF64 {
     // the left half, the triangular solve of the right half's block row, the update of the right half,
     // the right half; the strips swap their rows across the whole panel, so no interchanges between)
     int pk0 = 0, pnb = 0;
+    static int n_sm() {
+        int dev = 0, n = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n;
+    }
     void panel(int c0, int w) {
-        // strips of 32 or 16 columns in registers while their rows fit a cluster, else of 8 in global memory
-        const int rows = N - c0, base = rows <= LuStrip<32>::MAXROWS ? 32 : rows <= LuStrip<16>::MAXROWS ? 16 : LU_BASE;
+        // Strips of 32 or 16 columns in registers while their rows fit a cluster and the launch's CTAs, one an SM, take
+        // few waves, else of 8 columns in global memory (one CTA a matrix): with more matrices the products beside the panel
+        // are the longer part, and the clusters take their SMs.  LU, ms, strips of 8 / of 32 and 16 everywhere / by this
+        // rule: order 3072 40 matrices 121.6 / 124.2 / 121.6, 80 236.4 / 247.6 / 235.0; 2160 24 31.6 / 29.6 / 29.6, 80 90.3 /
+        // 95.9 / 90.7; 1120 80 17.0 / 16.9 / 16.9, 160 32.0 / 32.8 / 29.7; 640 160 9.1 / 7.9 / 7.6.
+        const int rows = N - c0;
+        auto fits = [&](int maxrows, int t, int half_waves) {
+            return rows <= maxrows && 2 * F * ((rows + t - 1) / t) <= half_waves * n_sm();
+        };
+        const int base = fits(LuStrip<32>::MAXROWS, LuStrip<32>::T, 6)   ? 32
+                         : fits(LuStrip<16>::MAXROWS, LuStrip<16>::T, 3) ? 16
+                                                                         : LU_BASE;
         if (w <= base) {
             KernelProfiler& P = profiler();
             const double m = N - c0;

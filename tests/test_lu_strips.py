@@ -31,3 +31,17 @@ def test_pivot_order_of_equal_moduli():
     B = np.eye(n, 2)[None].astype(np.complex128)
     X = nv.debug_lu_f64(A, B)
     assert np.abs(X[0] - A[0].conj()[:, :2] / n).max() <= 1e-13
+
+
+@pytest.mark.gpu
+def test_residual_of_many_matrices():
+    """More matrices than the strips' clusters may take SMs for: strips of 8 in global memory, then of 32 columns once the
+    rows fit one CTA."""
+    from hydrobem_b200 import native as nv
+
+    n, batch = 270, 230
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n))
+    B = rng.standard_normal((batch, n, 3)) + 1j * rng.standard_normal((batch, n, 3))
+    X = nv.debug_lu_f64(A, B)
+    assert np.abs(A @ X - B).max() <= 1e-15 * n * np.abs(A).max() * np.abs(X).max()
