@@ -1667,6 +1667,28 @@ extern "C" HbStatus hbg_debug_gemm_tf32(int32_t M, int32_t N, int32_t K, const f
     }
 }
 
+extern "C" HbStatus hbg_debug_cgemv(int32_t n, int32_t batch, int32_t nrhs, const float* M, const double* x, double* y,
+                                    int32_t repeats, int64_t* differ) {
+    try {
+        if (!M || !x || !y || !differ) return fail({HB_ERR_ARGUMENT, "null argument"});
+        int ndev = 0;
+        if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
+            return fail({HB_ERR_UNSUPPORTED, "no CUDA device: this library runs the path on the GPU only"});
+        device_ctx(0);
+        const char* msg = "";
+        long long d = 0;
+        int rc = debug_cgemv(n, batch, nrhs, M, reinterpret_cast<const double2*>(x), reinterpret_cast<double2*>(y), repeats,
+                             &d, &msg);
+        *differ = d;
+        if (rc) return fail({rc, msg});
+        return HB_OK;
+    } catch (const Failure& f) {
+        return fail(f);
+    } catch (const std::exception& e) {
+        return fail({HB_ERR_INTERNAL, std::string("internal error: ") + e.what()});
+    }
+}
+
 extern "C" HbStatus hbg_debug_lu_f64(int32_t n, int32_t batch, const double* A, int32_t nrhs, const double* B,
                                      double* X) {
     try {

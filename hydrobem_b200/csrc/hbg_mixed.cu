@@ -111,6 +111,41 @@ inline int& ir_guess() {
     return g;
 }
 
+// The partial products of the FP64 product M x by TMA and DMMA, its maps covering exactly the nb matrices (planar FP32,
+// leading dimension Np) and vectors ([nb][nrhs][ldx]), nz column chunks; false if a map cannot be encoded.
+template <int NT>
+static void launch_cgemv_dmma_tiles(const CUtensorMap& mM, const CUtensorMap& mX, dim3 g, int N, int nrhs, double2* part,
+                                    int nb, int* err, cudaStream_t s) {
+    cudaFuncSetAttribute(k_cgemv_dmma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GdCfg<NT>::SMEM);
+    k_cgemv_dmma<NT><<<g, GD_THREADS, GdCfg<NT>::SMEM, s>>>(mM, mX, N, nrhs, part, nb, err);
+}
+static bool launch_cgemv_dmma(const float* M, int N, int Np, const double2* x, int ldx, int nrhs, int nb, int nz,
+                              double2* part, int* err, cudaStream_t s) {
+    CUtensorMap mM, mX;
+    const uint64_t plane = (uint64_t)Np * Np;
+    const uint64_t dm[4] = {(uint64_t)Np, (uint64_t)Np, 2, (uint64_t)nb};
+    const uint64_t sm[3] = {(uint64_t)Np * 4, plane * 4, 2 * plane * 4};
+    const uint32_t bm[4] = {GV_ROWS, GV_COLS, 1, 1};
+    const int nt = std::max(2, (nrhs + 3) / 4);  // (one tile: padded to two, zeros beyond nrhs)
+    const uint64_t dx[4] = {2 * (uint64_t)ldx, (uint64_t)nrhs, (uint64_t)nb, 1};
+    const uint64_t sx[3] = {(uint64_t)ldx * 16, (uint64_t)nrhs * ldx * 16, (uint64_t)nb * nrhs * ldx * 16};
+    const uint32_t bx[4] = {2 * GV_COLS, (uint32_t)(4 * nt), 1, 1};
+    if (!make_map_box(&mM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (void*)M, dm, sm, bm) ||
+        !make_map_box(&mX, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void*)x, dx, sx, bx))
+        return false;
+    const dim3 g((N + GV_ROWS - 1) / GV_ROWS, nb, nz);
+    switch (nt) {
+        case 2: launch_cgemv_dmma_tiles<2>(mM, mX, g, N, nrhs, part, nb, err, s); break;
+        case 3: launch_cgemv_dmma_tiles<3>(mM, mX, g, N, nrhs, part, nb, err, s); break;
+        case 4: launch_cgemv_dmma_tiles<4>(mM, mX, g, N, nrhs, part, nb, err, s); break;
+        case 5: launch_cgemv_dmma_tiles<5>(mM, mX, g, N, nrhs, part, nb, err, s); break;
+        case 6: launch_cgemv_dmma_tiles<6>(mM, mX, g, N, nrhs, part, nb, err, s); break;
+        case 7: launch_cgemv_dmma_tiles<7>(mM, mX, g, N, nrhs, part, nb, err, s); break;
+        default: launch_cgemv_dmma_tiles<8>(mM, mX, g, N, nrhs, part, nb, err, s); break;
+    }
+    return true;
+}
+
 // Side streams for the LU of LU_GROUPS groups of a batch and their fork/join events, per device and
 // host thread (kept across solves).
 constexpr int LU_GROUPS = 4;  // at most (the streams kept)
@@ -340,36 +375,9 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     if (!part) MIXED_FAIL(HB_ERR_INTERNAL, "device memory allocation failed for the mixed form", -1);
     // the column width of a chunk of w right-hand sides of the FP32 product (its padded columns cost as much as real ones)
     auto chunk_width = [](int w) { return w <= 4 ? 4 : w <= 8 ? 8 : w <= 10 ? 10 : w <= 12 ? 12 : 16; };
-    // the FP64 product by TMA and DMMA (its maps cover exactly the matrices and vectors of the batch), all right-hand
-    // sides at once in tiles of four; the register form if a map fails
-    auto dmma = [&](auto tiles, const CUtensorMap& mM, const CUtensorMap& mX, dim3 g, int nb, cudaStream_t s) {
-        constexpr int NT = decltype(tiles)::value;
-        cudaFuncSetAttribute(k_cgemv_dmma<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GdCfg<NT>::SMEM);
-        k_cgemv_dmma<NT><<<g, GD_THREADS, GdCfg<NT>::SMEM, s>>>(mM, mX, Nm, nrhs, part, nb, err);
-    };
+    // the FP64 product by TMA and DMMA, all right-hand sides at once; the register form if a map fails
     auto gemv_tma = [&](const float* Mm, const double2* xv, int ldx, int nb, int nzt, cudaStream_t s) -> bool {
-        CUtensorMap mM, mX;
-        const uint64_t dm[4] = {(uint64_t)Np, (uint64_t)Np, 2, (uint64_t)nb};
-        const uint64_t sm[3] = {(uint64_t)Np * 4, NP2 * 4, MB * 4};
-        const uint32_t bm[4] = {GV_ROWS, GV_COLS, 1, 1};
-        const int nt = std::max(2, (nrhs + 3) / 4);  // (one tile: padded to two, zeros beyond nrhs)
-        const uint64_t dx[4] = {2 * (uint64_t)ldx, (uint64_t)nrhs, (uint64_t)nb, 1};
-        const uint64_t sx[3] = {(uint64_t)ldx * 16, (uint64_t)nrhs * ldx * 16, (uint64_t)nb * nrhs * ldx * 16};
-        const uint32_t bx[4] = {2 * GV_COLS, (uint32_t)(4 * nt), 1, 1};
-        if (!make_map_box(&mM, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (void*)Mm, dm, sm, bm) ||
-            !make_map_box(&mX, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (void*)xv, dx, sx, bx))
-            return false;
-        dim3 g((Nm + GV_ROWS - 1) / GV_ROWS, nb, nzt);
-        switch (nt) {
-            case 2: dmma(std::integral_constant<int, 2>(), mM, mX, g, nb, s); break;
-            case 3: dmma(std::integral_constant<int, 3>(), mM, mX, g, nb, s); break;
-            case 4: dmma(std::integral_constant<int, 4>(), mM, mX, g, nb, s); break;
-            case 5: dmma(std::integral_constant<int, 5>(), mM, mX, g, nb, s); break;
-            case 6: dmma(std::integral_constant<int, 6>(), mM, mX, g, nb, s); break;
-            case 7: dmma(std::integral_constant<int, 7>(), mM, mX, g, nb, s); break;
-            default: dmma(std::integral_constant<int, 8>(), mM, mX, g, nb, s); break;
-        }
-        return true;
+        return launch_cgemv_dmma(Mm, Nm, Np, xv, ldx, nrhs, nb, nzt, part, err, s);
     };
     const int nz_tma = (Nm + GV_CHUNK - 1) / GV_CHUNK;
     for (auto fn : {(const void*)k_cgemv32_tma<4>, (const void*)k_cgemv32_tma<8>, (const void*)k_cgemv32_tma<10>,
@@ -954,6 +962,60 @@ int debug_gemm_tf32(int M, int N, int K, const float* A, const float* B, float* 
     }
     if (herr) {
         *msg = "pipeline wait timed out";
+        return HB_ERR_INTERNAL;
+    }
+    return 0;
+}
+
+// Test support: y [batch][nrhs][n] = M x by the FP64 product of the mixed form (M planar FP32 [batch][2][n][n],
+// column-major, its padding to a multiple of 128 filled with NaNs here; x [batch][nrhs][n]), repeated `repeats` times:
+// *differ counts the entries of the later results that are not those of the first to the bit.
+int debug_cgemv(int n, int batch, int nrhs, const float* M, const double2* x, double2* y, int repeats, long long* differ,
+                const char** msg) {
+    if (n <= 0 || batch <= 0 || batch > 65535 || nrhs <= 0 || nrhs > 32 || repeats <= 0) {
+        *msg = "debug product: n, repeats > 0, 0 < batch <= 65535, 0 < nrhs <= 32";
+        return HB_ERR_VALUE;
+    }
+    if (!encode_fn()) {
+        *msg = "no tensor-map encoder";
+        return HB_ERR_UNSUPPORTED;
+    }
+    MixedBuffers mb;
+    const int Np = (n + NBL - 1) / NBL * NBL, nz = (n + GV_CHUNK - 1) / GV_CHUNK;
+    const size_t nM = (size_t)2 * Np * Np * batch, nx = (size_t)n * nrhs * batch;
+    float* dM = mb.get<float>(nM);
+    double2* dx = mb.get<double2>(nx);
+    double2* dy = mb.get<double2>(nx);
+    double2* part = mb.get<double2>(nx * nz);
+    int* err = mb.get<int>(1);
+    if (!dM || !dx || !dy || !part || !err) {
+        *msg = "allocation failed";
+        return HB_ERR_INTERNAL;
+    }
+    cudaMemset(dM, 0xff, nM * sizeof(float));
+    for (size_t p = 0; p < 2 * (size_t)batch; p++)
+        cudaMemcpy2D(dM + p * Np * Np, sizeof(float) * Np, M + p * n * n, sizeof(float) * n, sizeof(float) * n, n,
+                     cudaMemcpyHostToDevice);
+    cudaMemcpy(dx, x, nx * sizeof(double2), cudaMemcpyHostToDevice);
+    cudaMemset(err, 0, sizeof(int));
+    std::vector<double2> again(repeats > 1 ? nx : 0);
+    *differ = 0;
+    for (int r = 0; r < repeats; r++) {
+        if (!launch_cgemv_dmma(dM, n, Np, dx, n, nrhs, batch, nz, part, err, nullptr)) {
+            *msg = "tensor-map encoding failed";
+            return HB_ERR_INTERNAL;
+        }
+        k_gemv_reduce<<<dim3((unsigned)((nx / batch + 255) / 256), batch), 256>>>(n, nrhs, batch, nz, part, nullptr, n, dy, n);
+        double2* to = r ? again.data() : y;
+        cudaMemcpy(to, dy, nx * sizeof(double2), cudaMemcpyDeviceToHost);
+        if (r)
+            for (size_t i = 0; i < nx; i++) *differ += memcmp(&again[i], &y[i], sizeof(double2)) != 0;
+    }
+    for (size_t i = 0; i < nx; i++) y[i] = make_double2(-y[i].x, -y[i].y);  // (the reduction forms bias - M x)
+    int herr = 0;
+    cudaMemcpy(&herr, err, sizeof(int), cudaMemcpyDeviceToHost);
+    if (cudaGetLastError() != cudaSuccess || herr) {
+        *msg = herr ? "a tensor-core pipeline wait timed out" : "CUDA error";
         return HB_ERR_INTERNAL;
     }
     return 0;

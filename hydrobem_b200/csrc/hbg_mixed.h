@@ -28,6 +28,8 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
                             const double* motion, const FieldArgs& field, std::vector<int64_t>* fallback);
 
 int debug_gemm_tf32(int M, int N, int K, const float* A, const float* B, float* C, bool subtract, const char** msg);
+int debug_cgemv(int n, int batch, int nrhs, const float* M, const double2* x, double2* y, int repeats, long long* differ,
+                const char** msg);
 int measure_peaks(double* out, const char** msg);
 // the mixed LU's groups of systems on side streams for the solves that follow (process-wide; 0: the
 // library's rule)

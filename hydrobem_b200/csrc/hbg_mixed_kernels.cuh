@@ -939,14 +939,21 @@ __global__ void __launch_bounds__(GD_THREADS, NT <= 2 ? 2 : 1) k_cgemv_dmma(cons
         for (int c = 0; c < NT; c++) acc[t][c][0] = acc[t][c][1] = 0.0;
     for (int si = 0; si < nst; si++) {
         const int s = si % C::STAGES;
-        // The vote brings the lanes together again (the mma wants them all).  A stage is handed back only behind the wait
-        // for the next: an arrival straight behind the unrolled loop let TMA overwrite a last vector entry still to be
-        // read by the queued mma (seen as 1e-2 errors of one right-hand side in one call of a hundred).
+        // (the vote: one answer for the warp, each lane leaves the wait by itself)
         if (!__all_sync(0xffffffffu, tc::mbar_wait(&full[s], (si / C::STAGES) & 1))) {
             atomicExch(err, 7);
             break;
         }
+        // The stage before is handed back: every lane orders its reads of it before the TMA writes that refill it
+        // (another proxy), the warp barrier orders those fences before lane 0's arrival, and the second one brings the
+        // lanes together for the mma.  It stands behind the wait for this stage because the fence alone is not what was
+        // measured: an arrival at the end of the stage's own unrolled loop, with a warp barrier but no fence before
+        // it, let entries be overwritten (a product done twice differed in 1.1e6 entries of 1210 calls; in none with a
+        // pause before the arrival, or with the arrival here).
+        tc::fence_proxy_async_smem();
+        __syncwarp();
         if (si > 0 && lane == 0) tc::mbar_arrive(&empty[(si - 1) % C::STAGES]);
+        __syncwarp();
         const uint8_t* st = base + s * C::STAGE;
         const float* sM = reinterpret_cast<const float*>(st) + 32 * warp + 4 * i;
         const double2* sx = reinterpret_cast<const double2*>(st + 2 * GV_COLS * GV_ROWS * 4);  // [4 NT][GV_COLS]
@@ -1103,6 +1110,7 @@ __global__ void __launch_bounds__(gv32_threads<NR>()) k_cgemv32_tma(const __grid
             acd[c].x += (double)(c & 1 ? x1.y : x1.x);
             acd[c].y += (double)(c & 1 ? y1.y : y1.x);
         }
+        tc::fence_proxy_async_smem();  // (the reads before the TMA writes that refill the stage)
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&empty[s]);
     }
@@ -1415,6 +1423,7 @@ __global__ void __launch_bounds__(TRI_THREADS, 1) k_tri_sweep(const __grid_const
                     wait(&full[s], (st / C::NST) & 1);
                     tri_stage<KS, NH, false>(reinterpret_cast<const float*>(base + s * TRI_STAGE), y + sub * TRI_SK, k0, lane, 0,
                                          false, ar, ai);
+                    tc::fence_proxy_async_smem();  // (the reads before the TMA writes that refill the stage)
                     __syncwarp();
                     if (lane == 0) tc::mbar_arrive(&empty[s]);
                 }
@@ -1434,6 +1443,7 @@ __global__ void __launch_bounds__(TRI_THREADS, 1) k_tri_sweep(const __grid_const
                 wait(&full[s], (st / C::NST) & 1);
                 tri_stage<KS, NH, true>(reinterpret_cast<const float*>(base + s * TRI_STAGE), rb + q0 * TB + sub * TRI_SK, k0, lane,
                                     sub * TRI_SK, upper_t != 0, ar, ai);
+                tc::fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) tc::mbar_arrive(&empty[s]);
             }

@@ -76,7 +76,8 @@ template <int N>
 __device__ __forceinline__ void bulk_wait_read_n() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
-// generic-proxy writes to shared memory made visible to the async proxy (before a TMA store)
+// this thread's generic-proxy accesses of shared memory ordered before later ones of the async proxy: its writes
+// before a TMA store, its reads before the TMA load that overwrites them (behind the barrier that hands them over)
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {

@@ -96,7 +96,8 @@ EXPORTS = ["hbg_default_options", "hbg_solve_batch", "hbg_debug_matrices", "hbg_
            "hb_set_ints", "hb_model_solve", "hb_results_free", "hb_results_has", "hb_results_quantity",
            "hbg_statics_noalloc", "hbg_measure_peaks", "hbg_last_ir_history", "hbg_surrogate_train",
            "hbg_surrogate_grad", "hbg_surrogate_eval", "hbg_last_surrogate_pairs", "hbg_read_gdf", "hbg_gdf_free",
-           "hb_model_load_mesh", "hbg_last_fallback_count", "hbg_debug_lu_f64", "hb_model_panels", "hbg_tuned_tiles", "hbg_last_fallback_time"]
+           "hb_model_load_mesh", "hbg_last_fallback_count", "hbg_debug_lu_f64", "hb_model_panels", "hbg_tuned_tiles", "hbg_last_fallback_time",
+           "hbg_debug_cgemv"]
 
 _lib = None
 
@@ -130,6 +131,8 @@ def lib():
     L.hbg_last_ir_iterations.argtypes = [ctypes.POINTER(ctypes.c_int32)]
     L.hbg_debug_lu_f64.argtypes = [ctypes.c_int32, ctypes.c_int32, dp, ctypes.c_int32, dp, dp]
     L.hbg_debug_lu_f64.restype = ctypes.c_int32
+    L.hbg_debug_cgemv.argtypes = [ctypes.c_int32] * 3 + [fp, dp, dp, ctypes.c_int32, ctypes.POINTER(ctypes.c_int64)]
+    L.hbg_debug_cgemv.restype = ctypes.c_int32
     L.hbg_measure_peaks.argtypes = [dp]
     L.hbg_last_ir_history.argtypes = [dp, ctypes.POINTER(ctypes.c_int32)]
     L.hbg_surrogate_train.argtypes = [ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_double,
@@ -406,6 +409,20 @@ def debug_lu_f64(A, B):
     X = np.zeros_like(Bc)
     check(lib().hbg_debug_lu_f64(n, batch, Ac.ctypes.data_as(dp), nrhs, Bc.ctypes.data_as(dp), X.ctypes.data_as(dp)))
     return X.transpose(0, 2, 1)
+
+
+def debug_cgemv(M, x, repeats=1):
+    """y = M x by the mixed form's FP64 product (test support): M [batch][n][n] complex64, x [batch][nrhs][n]
+    complex128.  Returns y and the entries of repeated products that were not the first's to the bit."""
+    M = np.asarray(M, dtype=np.complex64).transpose(0, 2, 1)
+    planes = np.ascontiguousarray(np.stack([M.real, M.imag], 1))  # [batch][2][column][row]
+    x = np.ascontiguousarray(x, dtype=np.complex128)
+    batch, nrhs, n = x.shape
+    y = np.zeros_like(x)
+    differ = ctypes.c_int64()
+    check(lib().hbg_debug_cgemv(n, batch, nrhs, planes.ctypes.data_as(ctypes.POINTER(ctypes.c_float)),
+                                x.ctypes.data_as(dp), y.ctypes.data_as(dp), int(repeats), ctypes.byref(differ)))
+    return y, differ.value
 
 
 def debug_gemm_tf32(A, B, C=None):

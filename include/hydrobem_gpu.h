@@ -304,6 +304,14 @@ HbStatus hbg_debug_gemm_tf32(int32_t M, int32_t N, int32_t K, const float *A, co
  * of Real::lu_solve, linalg.rs:100-201 and 321-354, exposed for its numerics test). */
 HbStatus hbg_debug_lu_f64(int32_t n, int32_t batch, const double *A, int32_t nrhs, const double *B, double *X);
 
+/* Test support: y = M x by the mixed form's FP64 product (the right-hand sides and residuals): M [batch][2][n][n] FP32,
+ * real and imaginary plane, each column-major; x and y [batch][nrhs][n], interleaved (re, im) host arrays; nrhs <= 32.
+ * The product is formed `repeats` times; differ receives the number of entries of the later results that are not
+ * those of the first to the bit.  Replaces no reference interface (the residual of Real::lu_solve, linalg.rs:100-201,
+ * exposed for its numerics test). */
+HbStatus hbg_debug_cgemv(int32_t n, int32_t batch, int32_t nrhs, const float *M, const double *x, double *y,
+                         int32_t repeats, int64_t *differ);
+
 /* Measured compute peaks of the current device, for the benchmark's rooflines: out3[0] FP64 FMA,
  * out3[1] FP64 warp MMA (mma.sync m8n8k4), out3[2] TF32 tcgen05 MMA, all dense TFLOP/s, each from
  * a kernel that keeps its pipe busy from registers or shared memory.  Replaces no reference
