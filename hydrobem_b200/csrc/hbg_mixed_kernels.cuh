@@ -915,7 +915,8 @@ __global__ void __launch_bounds__(GD_THREADS, NT <= 2 ? 2 : 1) k_cgemv_dmma(cons
         if (lane == 0) {
             tc::prefetch_tensormap(&mapM);
             tc::prefetch_tensormap(&mapX);
-            for (int si = 0; si < nst; si++) {
+            int si = 0;
+            for (; si < nst; si++) {
                 const int s = si % C::STAGES;
                 if (si >= C::STAGES && !tc::mbar_wait(&empty[s], ((si / C::STAGES) - 1) & 1)) {
                     atomicExch(err, 6);
@@ -928,6 +929,12 @@ __global__ void __launch_bounds__(GD_THREADS, NT <= 2 ? 2 : 1) k_cgemv_dmma(cons
                 tc::tma_load_4d(st + GV_COLS * GV_ROWS * 4, &mapM, &full[s], k0, n0, 1, f);
                 tc::tma_load_4d(st + 2 * GV_COLS * GV_ROWS * 4, &mapX, &full[s], 2 * n0, 0, f, 0);
             }
+            // every load still in flight lands before the CTA leaves, also after an error (bounded)
+            for (int q = max(0, si - C::STAGES); q < si; q++)
+                if (!tc::mbar_wait(&full[q % C::STAGES], (q / C::STAGES) & 1)) {
+                    atomicExch(err, 6);
+                    break;
+                }
         }
         return;
     }
@@ -1052,7 +1059,8 @@ __global__ void __launch_bounds__(gv32_threads<NR>()) k_cgemv32_tma(const __grid
         if (lane == 0) {
             tc::prefetch_tensormap(&mapM);
             tc::prefetch_tensormap(&mapD);
-            for (int si = 0; si < nst; si++) {
+            int si = 0;
+            for (; si < nst; si++) {
                 const int s = si % GV_STAGES;
                 if (si >= GV_STAGES && !tc::mbar_wait(&empty[s], ((si / GV_STAGES) - 1) & 1)) {
                     atomicExch(err, 6);
@@ -1065,6 +1073,12 @@ __global__ void __launch_bounds__(gv32_threads<NR>()) k_cgemv32_tma(const __grid
                 tc::tma_load_4d(st + GV_COLS * GV_ROWS * 4, &mapM, &full[s], k0, n0, 1, f);
                 tc::tma_load_4d(st + 2 * GV_COLS * GV_ROWS * 4, &mapD, &full[s], 4 * n0, c0 / 2, f, 0);
             }
+            // every load still in flight lands before the CTA leaves, also after an error (bounded)
+            for (int q = max(0, si - GV_STAGES); q < si; q++)
+                if (!tc::mbar_wait(&full[q % GV_STAGES], (q / GV_STAGES) & 1)) {
+                    atomicExch(err, 6);
+                    break;
+                }
         }
         return;
     }
