@@ -1486,8 +1486,9 @@ __global__ void k_to_pairs(int Np, int nrhs, const double2* __restrict__ b, floa
 }
 
 // x += d; per matrix the largest |d| and |x| (for the refinement's stopping test) into norms [F][2], zero before
-// (bits of non-negative doubles order as the values do).  A CTA per 256 rows of a column pair: one CTA a matrix took
-// 94 us for 40 matrices of order 4096 and 10 columns.
+// (bits of non-negative doubles order as the values do).  A correction or solution that is not finite counts as an
+// infinite |d|: fmax drops a NaN, and a system of NaNs would pass for converged.  A CTA per 256 rows of a column pair:
+// one CTA a matrix took 94 us for 40 matrices of order 4096 and 10 columns.
 __global__ void __launch_bounds__(256) k_ir_update(int Np, int nrhs, double2* __restrict__ x, const float4* __restrict__ d,
                                                    unsigned long long* __restrict__ norms) {
     __shared__ double sd[8], sx[8];
@@ -1504,7 +1505,7 @@ __global__ void __launch_bounds__(256) k_ir_update(int Np, int nrhs, double2* __
                 a.x += dx;
                 a.y += dy;
                 x[o] = a;
-                md = fmax(md, fmax(fabs(dx), fabs(dy)));
+                md = isfinite(a.x) && isfinite(a.y) ? fmax(md, fmax(fabs(dx), fabs(dy))) : INFINITY;
                 mx = fmax(mx, fmax(fabs(a.x), fabs(a.y)));
             }
     }
