@@ -383,6 +383,8 @@ struct WsBuf {
         if (!p) throw Failure{HB_ERR_INTERNAL, "device memory allocation failed"};
         bytes = b;
     }
+    // the slot's buffer as the workspace holds it
+    void held() { p = ws.p[slot], bytes = ws.bytes[slot]; }
     template <class T>
     T* as() const {
         return reinterpret_cast<T*>(p);
@@ -857,16 +859,41 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         return;
     }
     // ---- frequency batches
-    // per frequency: G systems (S, A, right-hand sides, solutions, pivots), the boundary values and incident
-    // wave of every panel, with sectors the projected right-hand sides and the recombined potentials
-    size_t per_freq = G * (2 * NN * sizeof(double2) + (size_t)2 * nrhs * Nm * sizeof(double2) + (size_t)Nm * 4 + 4 +
-                           rhs_f64_scratch(Nm, 1, nrhs)) +
-                      (size_t)(nrhs + H) * N * sizeof(double2) + (G > 1 ? (size_t)2 * nrhs * N * sizeof(double2) : 0) +
-                      (fin ? (size_t)(T1_SIZE + T2_SIZE) * 8 + (size_t)FP_PLANES * N * 8 +
-                                                              (size_t)6912 * 3 * 8
-                                                        : 0);
-    // the batch size from free memory, kept per thread and device for the same problem shape while the
-    // workspace holds its buffers (cudaMemGetInfo can take milliseconds)
+    // outputs per batch: A, B [D][D], X, FK, SC, motions [H][D], field values [P][D] and 3 x [P][H], then the Haskind
+    // exciting force [H][D], then (TK > 0) the Kochin functions kr, krt [TK][D], kd, kdt [TK][H] and the drift [H][H][3]
+    const int Pf = field ? nfp : 0;
+    const size_t kochin_per = (size_t)TK * 2 * (D + H) + (TK ? (size_t)3 * H * H : 0);
+    const size_t out_per = 2 * (size_t)D * D * sizeof(double) + 5 * (size_t)H * D * sizeof(double2) +
+                           (size_t)Pf * (D + 3 * H) * sizeof(double2) + kochin_per * sizeof(double2);
+    // the device buffers of a batch of nf frequencies: G systems each (S, A, right-hand sides, solutions, pivots), the
+    // boundary values and incident wave of every panel, with sectors the projected right-hand sides and the recombined
+    // potentials
+    auto needs = [&](int nf) {
+        const size_t n = (size_t)nf * G, f = (size_t)nf;  // systems, frequencies
+        Workspace::Needs v = {
+            {WS_S, sizeof(double2) * NN * n}, {WS_A, sizeof(double2) * NN * n},
+            {WS_U, sizeof(double2) * (size_t)nrhs * N * f}, {WS_RHS, sizeof(double2) * (size_t)nrhs * Nm * n},
+            {WS_PART, rhs_f64_scratch(Nm, (int)n, nrhs)}, {WS_X, sizeof(double2) * (size_t)nrhs * Nm * n},
+            {WS_PHII, sizeof(double2) * (size_t)std::max(H, 1) * N * f}, {WS_IPIV, sizeof(int32_t) * (size_t)Nm * n},
+            {WS_INFO, sizeof(int32_t) * n}, {WS_FI, sizeof(FreqInfo) * f}, {WS_FD, sizeof(FdParams) * f},
+            {WS_OUT, out_per * f}};
+        if (G > 1) {
+            v.push_back({WS_UP, sizeof(double2) * (size_t)nrhs * Nm * n});
+            v.push_back({WS_PHI, sizeof(double2) * (size_t)nrhs * N * f});
+        }
+        if (fin) {
+            v.push_back({WS_TILES, sizeof(double) * (size_t)(T1_SIZE + T2_SIZE) * f});
+            v.push_back({WS_SCR, sizeof(double) * (size_t)6912 * 3 * f});
+            v.push_back({WS_FPT, sizeof(double) * (size_t)FP_PLANES * N * f});
+            if (field) v.push_back({WS_FQ, sizeof(double) * FP_PLANES * (size_t)(N + nfp) * f});
+        }
+        return v;
+    };
+    size_t per_freq = 0;
+    for (const auto& q : needs(1)) per_freq += q.second;
+    // the batch size: all frequencies while the buffers held hold every one of them (the same problem again, or a smaller
+    // one of a batch), else from free memory, kept per thread and device for the same problem shape while the workspace
+    // holds its buffers (cudaMemGetInfo can take milliseconds)
     int B = 0;
     {
         struct BatchChoice {
@@ -878,16 +905,14 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         int dev_b = 0;
         cudaGetDevice(&dev_b);
         BatchChoice& c = last[dev_b < 0 || dev_b >= 16 ? 0 : dev_b];
-        const size_t all = sizeof(double2) * NN * G * (size_t)F;
-        if (ws.bytes[WS_S] >= all && ws.bytes[WS_A] >= all && per_freq * F <= ws.held() + ((size_t)1 << 30)) {
-            // every frequency fits the buffers held (the same problem again, or another of a batch)
-            B = opt.max_batch > 0 ? std::min(F, (int)opt.max_batch) : F;
+        const int most = opt.max_batch > 0 ? std::min(F, (int)opt.max_batch) : F;
+        if (ws.holds(needs(most))) {
+            B = most;
         } else {
             const size_t budget = hbm_budget()();
             const bool same = c.N == N && c.G == G && c.nrhs == nrhs && c.fin == (int)fin && c.F == F &&
                               c.max_batch == opt.max_batch && c.budget == budget;
-            const size_t mats = NN * G * (size_t)std::max(c.B, 0);
-            if (same && c.B > 0 && ws.bytes[WS_S] >= sizeof(double2) * mats && ws.bytes[WS_A] >= sizeof(double2) * mats) {
+            if (same && c.B > 0 && ws.holds(needs(c.B))) {
                 B = c.B;
             } else {
                 size_t freeb = 0, totalb = 0;
@@ -895,54 +920,31 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
                 const size_t reusable = ws.bytes[WS_S] + ws.bytes[WS_A];
                 size_t avail = (size_t)(0.85 * (double)(freeb + reusable));
                 if (budget > 0) avail = std::min(avail, budget);
-                B = (int)std::max<size_t>(1, avail / per_freq);
-                if (opt.max_batch > 0) B = std::min(B, (int)opt.max_batch);
-                B = std::min(B, F);
-                c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, budget};
+                B = (int)std::min<size_t>(most, std::max<size_t>(1, avail / per_freq));
             }
+            // buffers that cannot be had beside what else is held: all given back, half the frequencies
+            while (!ws.take(needs(B))) {
+                ws.drop(needs(B));
+                if (B == 1) throw Failure{HB_ERR_INTERNAL, "device memory allocation failed", body_index};
+                B = (B + 1) / 2;
+            }
+            c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, budget};
         }
     }
     const size_t BS = (size_t)B * G;  // systems per batch
     WsBuf dS(ws, WS_S), dA(ws, WS_A), du(ws, WS_U), drhs(ws, WS_RHS), dX(ws, WS_X), dphiI(ws, WS_PHII),
         dipiv(ws, WS_IPIV), dinfo(ws, WS_INFO), dfi(ws, WS_FI), dfd(ws, WS_FD), dtiles(ws, WS_TILES),
-        dscr(ws, WS_SCR), dfpt(ws, WS_FPT), dheads(ws, WS_HEADS), dout(ws, WS_OUT), dup(ws, WS_UP), dphi(ws, WS_PHI);
-    dS.alloc(sizeof(double2) * NN * BS);
-    dA.alloc(sizeof(double2) * NN * BS);
-    du.alloc(sizeof(double2) * (size_t)nrhs * N * B);
-    drhs.alloc(sizeof(double2) * (size_t)nrhs * Nm * BS);
-    WsBuf dpart(ws, WS_PART);
-    dpart.alloc(rhs_f64_scratch(Nm, (int)BS, nrhs));
-    dX.alloc(sizeof(double2) * (size_t)nrhs * Nm * BS);
-    if (G > 1) {
-        dup.alloc(sizeof(double2) * (size_t)nrhs * Nm * BS);
-        dphi.alloc(sizeof(double2) * (size_t)nrhs * N * B);
-    }
-    dphiI.alloc(sizeof(double2) * (size_t)std::max(H, 1) * N * B);
-    dipiv.alloc(sizeof(int32_t) * (size_t)Nm * BS);
-    dinfo.alloc(sizeof(int32_t) * BS);
-    dfi.alloc(sizeof(FreqInfo) * B);
-    dfd.alloc(sizeof(FdParams) * B);
-    if (fin) {
-        dtiles.alloc(sizeof(double) * (size_t)(T1_SIZE + T2_SIZE) * B);
-        dscr.alloc(sizeof(double) * (size_t)6912 * 3 * B);
-        dfpt.alloc(sizeof(double) * (size_t)FP_PLANES * N * B);
-    }
+        dscr(ws, WS_SCR), dfpt(ws, WS_FPT), dheads(ws, WS_HEADS), dout(ws, WS_OUT), dup(ws, WS_UP), dphi(ws, WS_PHI), dpart(ws, WS_PART),
+        dfq(ws, WS_FQ);
+    for (WsBuf* w : {&dS, &dA, &du, &drhs, &dX, &dphiI, &dipiv, &dinfo, &dfi, &dfd, &dtiles, &dscr, &dfpt, &dout, &dup, &dphi,
+                     &dpart, &dfq})
+        w->held();
     std::vector<double> heads(std::max(H, 1));
     for (int h = 0; h < H; h++) heads[h] = pr.headings_deg[h] * PI / 180.0;
     dheads.alloc(sizeof(double) * heads.size());
     CUDA_OK(cudaMemcpyAsync(dheads.p, heads.data(), sizeof(double) * heads.size(), cudaMemcpyHostToDevice, s));
-    // outputs per batch: A, B [D][D], X, FK, SC, motions [H][D], field values [P][D] and 3 x [P][H]
-    const int Pf = field ? nfp : 0;
-    // outputs per batch: ..., then the Haskind exciting force [H][D], then (TK > 0) the Kochin functions
-    // kr, krt [TK][D], kd, kdt [TK][H] and the drift [H][H][3]
-    const size_t kochin_per = (size_t)TK * 2 * (D + H) + (TK ? (size_t)3 * H * H : 0);
-    const size_t out_per = 2 * (size_t)D * D * sizeof(double) + 5 * (size_t)H * D * sizeof(double2) +
-                           (size_t)Pf * (D + 3 * H) * sizeof(double2) + kochin_per * sizeof(double2);
-    WsBuf dfq(ws, WS_FQ);
-    if (field && fin) dfq.alloc(sizeof(double) * FP_PLANES * (size_t)(N + nfp) * B);
     WsBuf derr(ws, WS_ERR);
     derr.alloc(sizeof(int32_t));
-    dout.alloc(out_per * B);
     // page-locked outputs and pivot flags: their reads queue behind the work
     unsigned char* hout = static_cast<unsigned char*>(ws.host(HS_OUT, out_per * B + sizeof(int32_t) * (BS + 1)));
     if (!hout) throw Failure{HB_ERR_INTERNAL, "page-locked host memory could not be allocated", body_index};

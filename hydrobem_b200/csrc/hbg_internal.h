@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <functional>
+#include <utility>
 #include <vector>
 #include <cuda_runtime.h>
 
@@ -103,6 +104,29 @@ struct Workspace {
         if (cudaMalloc(&p[slot], b) != cudaSuccess) return nullptr;
         bytes[slot] = b;
         return p[slot];
+    }
+    // the buffers of a batch, (slot, bytes) each: whether all are held already; taken (false when one cannot be had,
+    // the allocation's error cleared); given back
+    using Needs = std::vector<std::pair<int, size_t>>;
+    bool holds(const Needs& needs) const {
+        for (const auto& n : needs)
+            if (bytes[n.first] < n.second) return false;
+        return true;
+    }
+    bool take(const Needs& needs) {
+        for (const auto& n : needs)
+            if (!get(n.first, n.second)) {
+                cudaGetLastError();
+                return false;
+            }
+        return true;
+    }
+    void drop(const Needs& needs) {
+        for (const auto& n : needs) {
+            if (p[n.first]) cudaFree(p[n.first]);
+            p[n.first] = nullptr;
+            bytes[n.first] = 0;
+        }
     }
     size_t held() const {
         size_t t = 0;

@@ -231,15 +231,47 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     const int Q = lu_super(Np), SW = Q * PW;  // panels and columns of a super-step
     const size_t prep = 2 * (size_t)Np * PW, op16 = 2 * (size_t)Np * SW, inv = 2 * (size_t)PW * PW,
                  midsz = 2 * (size_t)NBL * NBL;
-    // per system: the matrices, the LU operands, the diagonal-block inverses, the refinement vectors
-    size_t per_sys = 3 * MB * 4 + prep * 4 + 2 * op16 * 2 + 2 * inv * 4 + midsz * 8 + 4 * (size_t)nrhs * Np * 16 + 64 +
-                     (size_t)(Np / NBL) * NBL * NBL * 8;
-    // per frequency: G systems, the boundary values and incident wave of every panel (with sectors also
-    // the projected right-hand sides and the recombined potentials), the finite-depth tiles
-    size_t per = G * per_sys + (size_t)(nrhs + H) * N * 16 + (G > 1 ? (size_t)2 * nrhs * N * 16 : 0) +
-                 (fin ? (size_t)(T1_SIZE + T2_SIZE) * 8 + (size_t)(T1F_SIZE + T2F_SIZE) * 4 + (size_t)FP_PLANES * N * 8 + (size_t)6912 * 3 * 8 : 0);
-    // The batch size from free memory; cudaMemGetInfo can take milliseconds, so the decision is kept per
-    // thread and device for the same problem shape while the workspace still holds its buffers.
+    const size_t nblk = (size_t)Np / NBL, dinv = nblk * 2 * NBL * NBL;
+    const int npair = (nrhs + 1) / 2;  // complex64 vectors by column pairs
+    const int nz = (Nm + GEMV_CHUNK - 1) / GEMV_CHUNK;
+    const int nfp = field.P;
+    // A, B [D][D], X, FK, SC, motions, Haskind [H][D], field values [P][D] and 3 x [P][H] per frequency
+    // the Kochin functions kr, krt [TK][D], kd, kdt [TK][H] and the drift [H][H][3] after them
+    const int TK = pr.kochin_angles > 0 && H > 0 ? pr.kochin_angles : 0;
+    const size_t kochin_per = ((size_t)TK * 2 * (D + H) + (TK ? (size_t)3 * H * H : 0)) * 2;
+    const size_t out_per = 2 * (size_t)D * D + 5 * (size_t)H * 2 * D + (size_t)nfp * 2 * (D + 3 * H) + kochin_per,
+                 DD = (size_t)D * D;
+    // the device buffers of a batch of nf frequencies
+    auto needs = [&](int nf) {
+        const size_t n = (size_t)nf * G, f = (size_t)nf;  // systems, frequencies
+        Workspace::Needs v = {
+            {WS_S32, MB * n * 4}, {WS_A32, MB * n * 4}, {WS_W, MB * n * 4}, {WS_P2, prep * n * 4},
+            {WS_L16, op16 * n * 2}, {WS_U16, op16 * n * 2}, {WS_PX, inv * n * 4}, {WS_PY, inv * n * 4},
+            {WS_TXY, midsz * n * sizeof(float2)}, {WS_DINV, dinv * n * 4},
+            {WS_U, (size_t)nrhs * N * f * 16}, {WS_PHII, (size_t)std::max(H, 1) * N * f * 16},
+            {WS_B, (size_t)nrhs * Np * n * 16}, {WS_XM, (size_t)nrhs * Np * n * 16},
+            {WS_R, (size_t)npair * Np * n * 16}, {WS_RS, (size_t)npair * Np * n * 16},
+            {WS_PART, (size_t)nz * n * nrhs * Nm * 16},
+            {WS_NORMS, IR_MAX_IT * 2 * n * 8}, {WS_TRI_CTRL, sizeof(int) * (1 + n * npair)},
+            {WS_FI, sizeof(FreqInfo) * f}, {WS_FD, sizeof(FdParams) * f}, {WS_OUT, sizeof(double) * out_per * f}};
+        if (G > 1) {
+            v.push_back({WS_UP, (size_t)nrhs * Nm * n * 16});
+            v.push_back({WS_PHI, (size_t)nrhs * N * f * 16});
+        }
+        if (fin) {
+            v.push_back({WS_TILES, sizeof(double) * (T1_SIZE + T2_SIZE) * f});
+            v.push_back({WS_TILES_F, sizeof(float) * (T1F_SIZE + T2F_SIZE) * f});
+            v.push_back({WS_SCR, sizeof(double) * 6912 * 3 * f});
+            v.push_back({WS_FPT, sizeof(double) * FP_PLANES * N * f});
+            if (nfp) v.push_back({WS_FQ, sizeof(double) * FP_PLANES * (size_t)(N + nfp) * f});
+        }
+        return v;
+    };
+    size_t per = 0;  // bytes a frequency
+    for (const auto& q : needs(1)) per += q.second;
+    // The batch size: all frequencies while the buffers held hold every one of them (the same problem again, or a smaller
+    // one of a batch), else from free memory.  cudaMemGetInfo can take milliseconds, so that decision is kept per thread
+    // and device for the same problem shape while the workspace still holds its buffers.
     Workspace& ws = workspace();
     int B = 0;
     {
@@ -252,17 +284,14 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
         int dev_b = 0;
         cudaGetDevice(&dev_b);
         BatchChoice& c = last[dev_b < 0 || dev_b >= 16 ? 0 : dev_b];
-        const size_t all = MB * (size_t)F * G * 4;
-        if (ws.bytes[WS_S32] >= all && ws.bytes[WS_A32] >= all && ws.bytes[WS_W] >= all &&
-            per * F <= ws.held() + ((size_t)1 << 30)) {
-            // every frequency fits the buffers held (the same problem again, or another of a batch)
-            B = opt.max_batch > 0 ? std::min(F, (int)opt.max_batch) : F;
+        const int most = opt.max_batch > 0 ? std::min(F, (int)opt.max_batch) : F;
+        if (ws.holds(needs(most))) {
+            B = most;
         } else {
             const size_t budget = hbm_budget()();
             const bool same = c.N == N && c.G == G && c.nrhs == nrhs && c.fin == (int)fin && c.F == F &&
                               c.max_batch == opt.max_batch && c.budget == budget;
-            const size_t mats = MB * (size_t)std::max(c.B, 0) * G * 4;
-            if (same && c.B > 0 && ws.bytes[WS_S32] >= mats && ws.bytes[WS_W] >= mats) {
+            if (same && c.B > 0 && ws.holds(needs(c.B))) {
                 B = c.B;
             } else {
                 size_t freeb = 0, totalb = 0;
@@ -271,14 +300,17 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
                 freeb += ws.bytes[WS_S32] + ws.bytes[WS_A32] + ws.bytes[WS_W] + ws.bytes[WS_DINV];
                 size_t avail = (size_t)(0.85 * (double)freeb);
                 if (budget > 0) avail = std::min(avail, budget);
-                B = (int)std::max<size_t>(1, avail / per);
-                if (opt.max_batch > 0) B = std::min(B, (int)opt.max_batch);
-                B = std::min(B, F);
-                c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, budget};
+                B = (int)std::min<size_t>(most, std::max<size_t>(1, avail / per));
             }
+            // buffers that cannot be had beside what else is held: all given back, half the frequencies
+            while (!ws.take(needs(B))) {
+                ws.drop(needs(B));
+                if (B == 1) MIXED_FAIL(HB_ERR_INTERNAL, "device memory allocation failed for the mixed form", -1);
+                B = (B + 1) / 2;
+            }
+            c = BatchChoice{N, G, nrhs, (int)fin, F, B, opt.max_batch, budget};
         }
     }
-    const size_t nblk = (size_t)Np / NBL;
     const int BS = B * G;  // systems per batch
     bool okb = true;
     auto get = [&](int slot, size_t bytes) -> void* {
@@ -286,52 +318,33 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
         okb = okb && q != nullptr;
         return q;
     };
-    float* S32 = (float*)get(WS_S32, MB * BS * 4);
-    float* A32 = (float*)get(WS_A32, MB * BS * 4);
-    float* W = (float*)get(WS_W, MB * BS * 4);
-    float* P2 = (float*)get(WS_P2, prep * BS * 4);
-    __half* L16 = (__half*)get(WS_L16, op16 * BS * 2);  // [BS][2 planes][Np rows][SW]
-    __half* U16 = (__half*)get(WS_U16, op16 * BS * 2);  // [BS][2 planes][SW rows][Np]
-    float* PX = (float*)get(WS_PX, inv * BS * 4);
-    float* PY = (float*)get(WS_PY, inv * BS * 4);
-    float2* TXY = (float2*)get(WS_TXY, midsz * BS * sizeof(float2));
-    const size_t dinv = nblk * 2 * NBL * NBL;
-    float* DINV = (float*)get(WS_DINV, dinv * BS * 4);
-    double2* u = (double2*)get(WS_U, (size_t)nrhs * N * B * 16);
-    double2* phiI = (double2*)get(WS_PHII, (size_t)std::max(H, 1) * N * B * 16);
+    // (of the batch: taken above)
+    float *S32 = (float*)ws.p[WS_S32], *A32 = (float*)ws.p[WS_A32], *W = (float*)ws.p[WS_W], *P2 = (float*)ws.p[WS_P2];
+    __half* L16 = (__half*)ws.p[WS_L16];  // [BS][2 planes][Np rows][SW]
+    __half* U16 = (__half*)ws.p[WS_U16];  // [BS][2 planes][SW rows][Np]
+    float *PX = (float*)ws.p[WS_PX], *PY = (float*)ws.p[WS_PY], *DINV = (float*)ws.p[WS_DINV];
+    float2* TXY = (float2*)ws.p[WS_TXY];
+    double2 *u = (double2*)ws.p[WS_U], *phiI = (double2*)ws.p[WS_PHII];
     // symmetry sectors: the right-hand sides projected on the sectors, the potentials of every panel
-    double2* up = G > 1 ? (double2*)get(WS_UP, (size_t)nrhs * Nm * BS * 16) : nullptr;
-    double2* phi = G > 1 ? (double2*)get(WS_PHI, (size_t)nrhs * N * B * 16) : nullptr;
-    double2* b = (double2*)get(WS_B, (size_t)nrhs * Np * BS * 16);
-    double2* x = (double2*)get(WS_XM, (size_t)nrhs * Np * BS * 16);
-    const int npair = (nrhs + 1) / 2;  // complex64 vectors by column pairs
-    float4* r = (float4*)get(WS_R, (size_t)npair * Np * BS * 16);
-    float4* rs = (float4*)get(WS_RS, (size_t)npair * Np * BS * 16);  // a residual kept for r - A d
-    double* norms = (double*)get(WS_NORMS, IR_MAX_IT * 2 * (size_t)BS * 8);  // [iteration][batch][2]
+    double2 *up = (double2*)ws.p[WS_UP], *phi = (double2*)ws.p[WS_PHI];
+    double2 *b = (double2*)ws.p[WS_B], *x = (double2*)ws.p[WS_XM], *part = (double2*)ws.p[WS_PART];
+    float4* r = (float4*)ws.p[WS_R];
+    float4* rs = (float4*)ws.p[WS_RS];        // a residual kept for r - A d
+    double* norms = (double*)ws.p[WS_NORMS];  // [iteration][batch][2]
+    int* tctrl = (int*)ws.p[WS_TRI_CTRL];     // the triangular sweeps' tickets
+    FreqInfo* dfi = (FreqInfo*)ws.p[WS_FI];
+    FdParams* dfd = (FdParams*)ws.p[WS_FD];
+    double *tiles = (double*)ws.p[WS_TILES], *scr = (double*)ws.p[WS_SCR], *fpt = (double*)ws.p[WS_FPT];
+    float* tiles_f = (float*)ws.p[WS_TILES_F];
+    double *dout = (double*)ws.p[WS_OUT], *fq = (double*)ws.p[WS_FQ];
     int* err = (int*)get(WS_ERR, sizeof(int));
-    int* tctrl = (int*)get(WS_TRI_CTRL, sizeof(int) * (1 + (size_t)BS * ((nrhs + 1) / 2)));  // the triangular sweeps' tickets
-    FreqInfo* dfi = (FreqInfo*)get(WS_FI, sizeof(FreqInfo) * B);
-    FdParams* dfd = (FdParams*)get(WS_FD, sizeof(FdParams) * B);
     double* dheads = (double*)get(WS_HEADS, sizeof(double) * std::max(H, 1));
-    double* tiles = fin ? (double*)get(WS_TILES, sizeof(double) * (T1_SIZE + T2_SIZE) * B) : nullptr;
-    float* tiles_f = fin ? (float*)get(WS_TILES_F, sizeof(float) * (T1F_SIZE + T2F_SIZE) * B) : nullptr;
     // the wave-term network (optional): its parameters, the packed BF16 image the assembly loads, and
     // the count of pairs it served
     const bool sg = opt.surrogate != nullptr;
     float* sg_params = sg ? (float*)get(WS_SG_PARAMS, sizeof(float) * SURROGATE_FLOATS) : nullptr;
     uint8_t* sg_img = sg ? (uint8_t*)get(WS_SG_IMG, sg_image_bytes()) : nullptr;
     unsigned long long* sg_count = sg ? (unsigned long long*)get(WS_SG_COUNT, sizeof(unsigned long long)) : nullptr;
-    double* scr = fin ? (double*)get(WS_SCR, sizeof(double) * 6912 * 3 * B) : nullptr;
-    double* fpt = fin ? (double*)get(WS_FPT, sizeof(double) * FP_PLANES * N * B) : nullptr;
-    const int nfp = field.P;
-    // A, B [D][D], X, FK, SC, motions, Haskind [H][D], field values [P][D] and 3 x [P][H] per frequency
-    // the Kochin functions kr, krt [TK][D], kd, kdt [TK][H] and the drift [H][H][3] after them
-    const int TK = pr.kochin_angles > 0 && H > 0 ? pr.kochin_angles : 0;
-    const size_t kochin_per = ((size_t)TK * 2 * (D + H) + (TK ? (size_t)3 * H * H : 0)) * 2;
-    const size_t out_per = 2 * (size_t)D * D + 5 * (size_t)H * 2 * D + (size_t)nfp * 2 * (D + 3 * H) + kochin_per,
-                 DD = (size_t)D * D;
-    double* dout = (double*)get(WS_OUT, sizeof(double) * out_per * B);
-    double* fq = nfp && fin ? (double*)get(WS_FQ, sizeof(double) * FP_PLANES * (size_t)(N + nfp) * B) : nullptr;
     if (!okb) MIXED_FAIL(HB_ERR_INTERNAL, "device memory allocation failed for the mixed form", -1);
     last_surrogate_pairs() = 0;
     // ---- tensor maps (whole batch; the batch index is the 4th coordinate)
@@ -370,9 +383,6 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     if (!hout || !hn) MIXED_FAIL(HB_ERR_INTERNAL, "page-locked host memory could not be allocated", -1);
     int* herr = reinterpret_cast<int*>(hout + out_per * B);
     // out = bias - M x over the batch (M column-major planar FP32), FP64 accumulation
-    const int nz = (Nm + GEMV_CHUNK - 1) / GEMV_CHUNK;
-    double2* part = (double2*)ws.get(WS_PART, (size_t)nz * BS * nrhs * Nm * 16);
-    if (!part) MIXED_FAIL(HB_ERR_INTERNAL, "device memory allocation failed for the mixed form", -1);
     // the column width of a chunk of w right-hand sides of the FP32 product (its padded columns cost as much as real ones)
     auto chunk_width = [](int w) { return w <= 4 ? 4 : w <= 8 ? 8 : w <= 10 ? 10 : w <= 12 ? 12 : 16; };
     // the FP64 product by TMA and DMMA, all right-hand sides at once; the register form if a map fails
