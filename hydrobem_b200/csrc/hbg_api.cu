@@ -707,6 +707,9 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
                               prod_statics ? dtiers.as<float>() : nullptr, orig.empty() ? nullptr : dorig.as<int32_t>());
         P.end(KF_GEOMETRY, 0.0, s);
         g_launches++;
+        // the first invalid panel: looked at before the FP64 form's first factorization, else at the solve's next wait
+        CUDA_OK(cudaMemcpyAsync(hflags, dbad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        panels_flag().record(s);
         PanelsView pv{N, dplanes.as<double>(), dkind.as<int32_t>()};
         pv.G = G;
         if (prod_statics) pv.tiers = dtiers.as<float>();
@@ -733,9 +736,8 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
                        dnwork.as<int32_t>(), work_cap, s, opt.precision == HBG_MIXED);
         // algorithmic bytes: the four FP64 planes written
         P.end(KF_STATICS, 32.0 * (double)NS, s);
-        // the first invalid panel (geometry) and the adaptive worklist size, read at the next wait of the
-        // solve; the adaptive kernel takes the size from device memory and does nothing on invalid panels
-        CUDA_OK(cudaMemcpyAsync(hflags, dbad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        // the adaptive worklist size, read at the next wait of the solve; the adaptive kernel takes it from device
+        // memory and does nothing on invalid panels
         CUDA_OK(cudaMemcpyAsync(hflags + 1, dnwork.p, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
         P.begin(s);
         launch_statics_adaptive_q(pv, dwork.as<int32_t>(), dnwork.as<int32_t>(), work_cap, dbad.as<int32_t>(), big,
@@ -760,12 +762,15 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         statics_ran = true;
     };
     // once the stream has passed the statics: invalid panels come first among the failures
-    auto statics_check = [&]() {
-        if (!statics_ran) return;
+    auto panels_check = [&]() {
         if (hflags[0] != big)
             throw Failure{HB_ERR_VALUE,
                           "invalid panel " + std::to_string(hflags[0] + 1) + " (degenerate, non-convex or non-finite)",
                           body_index};
+    };
+    auto statics_check = [&]() {
+        if (!statics_ran) return;
+        panels_check();
         if (hflags[1] > work_cap || hflags[2] > work_cap)
             throw Failure{HB_ERR_INTERNAL, "adaptive log-integral worklist overflow", body_index};
     };
@@ -773,8 +778,9 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
     auto hydro_out = [&]() {
         if (pr.out.hydrostatics) memcpy(pr.out.hydrostatics, hhydro, sizeof(double) * nbod * HBG_HS);
     };
-    // the assembly (and field point) kernels skip their work on invalid panels (the flag in device memory), so
-    // that a solve runs without a host wait until the end of its first batch
+    // the assembly (and field point) kernels skip their work on invalid panels (the flag in device memory), so that a
+    // solve need not wait for its statics on the host: the mixed form waits at the end of its first batch, the FP64 form,
+    // whose LU may take seconds, for the geometry alone once its first assembly is queued
     PanelsView pv{N, dplanes.as<double>(), dkind.as<int32_t>(), dbad.as<int32_t>(),
                   multi ? dpbody.as<int32_t>() : nullptr, pr.body.rotation_centers ? drcen.as<double>() : nullptr, nbod, G};
     if (F == 0) {
@@ -1004,6 +1010,10 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
             P.end(KF_RHS, 16.0 * (double)NN * ns, s);
             g_launches += 3 + 2 * (G > 1);
             t.stop();
+        }
+        if (f0 == 0) {  // (the geometry is long past when the statics and the assembly have been queued: no idle device)
+            CUDA_OK(cudaEventSynchronize(panels_flag().event()));
+            panels_check();
         }
         {
             EventTimer t(s, &prof[2]);

@@ -247,6 +247,11 @@ inline SolveMark& solve_end() {
     static thread_local SolveMark t;
     return t;
 }
+// Behind the copy of a solve's panel flag (the first invalid panel) to the host.
+inline SolveMark& panels_flag() {
+    static thread_local SolveMark t;
+    return t;
+}
 
 // Device time of a phase: events on the stream, added to *acc at the next PhaseTimers::flush().
 struct EventTimer {
