@@ -963,6 +963,7 @@ static void solve_problem(const HbgProblem& pr_in, const HbgOptions& opt, int64_
         if (opt.cancel && *opt.cancel) {
             cudaStreamSynchronize(s);
             statics_check();  // an invalid panel comes first
+            if (f0 == 0) hydro_out();
             throw Failure{HB_ERR_CANCELLED, "the solve was cancelled", body_index, f0};
         }
         const int nb = std::min(B, F - f0), ns = nb * G;
