@@ -1680,6 +1680,38 @@ extern "C" HbStatus hbg_debug_gemm_tf32(int32_t M, int32_t N, int32_t K, const f
     }
 }
 
+extern "C" HbStatus hbg_debug_lu_pivots(int32_t n, int32_t batch, const double* A, int32_t* ipiv) {
+    try {
+        if (!A || !ipiv) return fail({HB_ERR_ARGUMENT, "null argument"});
+        if (n <= 0 || batch <= 0) return fail({HB_ERR_VALUE, "debug LU: n, batch > 0"});
+        int ndev = 0;
+        if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
+            return fail({HB_ERR_UNSUPPORTED, "no CUDA device: this library runs the path on the GPU only"});
+        device_ctx(0);
+        const size_t NN = (size_t)n * n;
+        double2* dA = nullptr;
+        int32_t *dp = nullptr, *di = nullptr;
+        const bool ok = cudaMalloc(&dA, sizeof(double2) * NN * batch) == cudaSuccess &&
+                        cudaMalloc(&dp, sizeof(int32_t) * (size_t)n * batch) == cudaSuccess &&
+                        cudaMalloc(&di, sizeof(int32_t) * batch) == cudaSuccess;
+        if (ok) {
+            int64_t launches = 0;
+            cudaMemcpy(dA, A, sizeof(double2) * NN * batch, cudaMemcpyHostToDevice);
+            lu_factor_f64(n, batch, dA, NN, dp, di, nullptr, &launches);
+            cudaMemcpy(ipiv, dp, sizeof(int32_t) * (size_t)n * batch, cudaMemcpyDeviceToHost);
+        }
+        const cudaError_t e = cudaGetLastError();
+        cudaFree(dA);
+        cudaFree(dp);
+        cudaFree(di);
+        if (!ok) return fail({HB_ERR_INTERNAL, "device memory allocation failed"});
+        if (e != cudaSuccess) return fail({HB_ERR_INTERNAL, std::string("CUDA: ") + cudaGetErrorString(e)});
+        return HB_OK;
+    } catch (const Failure& f) {
+        return fail(f);
+    }
+}
+
 extern "C" HbStatus hbg_debug_cgemv(int32_t n, int32_t batch, int32_t nrhs, const float* M, const double* x, double* y,
                                     int32_t repeats, int64_t* differ) {
     try {

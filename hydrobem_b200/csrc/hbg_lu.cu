@@ -133,10 +133,11 @@ __global__ void __launch_bounds__(512) k_lu_base(int N, int c0, int w, int pk0, 
 // ------------------------------------------------------------------ strip in registers
 // The same for strips of up to W columns while the rows fit a cluster of up to eight CTAs, a row a thread: the
 // row's entries stay in registers, shifted down a column a step (so that every register index is constant and the loop
-// body short), its multipliers in shared memory.  Per column each warp finds
-// its candidate (two 32-bit reductions: the upper word of |a|^2, so a pivot is within 1e-6 of the largest modulus, and
-// the first position) and puts its row and reciprocal into shared memory, its claim into every CTA's; a cluster
-// barrier; every CTA takes the winner's row over, and updates.  Rows change places in `pos` alone and are written to
+// body short), its multipliers in shared memory.  Per column each warp finds its candidate (the largest |a|^2, the
+// first position on a tie, as k_lu_base: a 32-bit reduction of the upper words, and only where lanes share the largest
+// one of the lower words, then of the positions: by the upper words alone a strip would take 62 us instead of 63.5) and
+// puts its row and reciprocal into shared memory, its claim into every CTA's; a cluster barrier; every CTA takes the
+// winner's row over, and updates.  Rows change places in `pos` alone and are written to
 // their places at the end, where the panel's other columns are permuted too.  Bound by that chain of dependent
 // instructions, ~1.1 us a column in one CTA, ~2 in clusters: a strip of 32 columns takes 41 / 64 / 79 us with 84 / 645 /
 // 1007 rows where one of 8 columns with its rows in global memory took 18 / 23 / 28, and 64 with 4096, and a panel now
@@ -148,8 +149,8 @@ struct LuStrip {
     static constexpr int T = W == 32 ? 256 : 512, NW = T / 32;  // threads (rows) of a CTA, its warps
     static constexpr int MAXROWS = T * LU_CLUSTER;
     struct __align__(16) Slot {
-        unsigned key;  // upper word of |a|^2, plus one (0: no candidate)
-        int pos, src, low;  // low: nonzero if |a|^2 is above zero
+        unsigned long long m;  // the bits of |a|^2, the upper word plus one (0: no candidate)
+        int pos, src;
     };
     struct Shared {
         double2 L[W][T];  // multipliers
@@ -190,6 +191,24 @@ __device__ __forceinline__ void cluster_store16(uint32_t a, const void* v) {
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
 }
 
+// The lane of the largest m, the smallest pos on a tie (any lane where every m is 0).  A whole warp.
+__device__ __forceinline__ int strip_best_lane(unsigned long long m, int pos) {
+    constexpr unsigned ALL = 0xffffffffu;
+    const unsigned hi = (unsigned)(m >> 32), mh = __reduce_max_sync(ALL, hi);
+    unsigned who = __ballot_sync(ALL, hi == mh);
+    if (__builtin_expect(mh && (who & (who - 1)), 0)) {
+        const bool top = hi == mh;
+        const unsigned ml = __reduce_max_sync(ALL, top ? (unsigned)m : 0u);
+        const bool tie = top && (unsigned)m == ml;
+        who = __ballot_sync(ALL, tie);
+        if (who & (who - 1)) {
+            const unsigned mp = __reduce_min_sync(ALL, tie ? (unsigned)pos : 0x7fffffffu);
+            who = __ballot_sync(ALL, tie && pos == (int)mp);
+        }
+    }
+    return __ffs(who) - 1;
+}
+
 template <int W>
 __global__ void __launch_bounds__(LuStrip<W>::T) k_lu_strip(int N, int c0, int w, int pk0, int pnb,
                                                             double2* __restrict__ Aall, size_t stride,
@@ -219,15 +238,14 @@ __global__ void __launch_bounds__(LuStrip<W>::T) k_lu_strip(int N, int c0, int w
             // (in flight beside the search)
             const double im2 = m2 > 0.0 ? 1.0 / m2 : 0.0;
             const double2 rcp = make_double2(a[0].x * im2, -a[0].y * im2);
-            const unsigned key = active && m2 == m2 ? (unsigned)__double2hiint(m2) + 1 : 0;
-            const unsigned mk = __reduce_max_sync(0xffffffffu, key);
-            const unsigned mp = __reduce_min_sync(0xffffffffu, key == mk ? (unsigned)pos : 0x7fffffffu);
-            if (key == mk && pos == (int)mp) {  // one lane (in a warp without candidates its row is never taken)
+            const unsigned long long m =
+                active && m2 == m2 ? (unsigned long long)__double_as_longlong(m2) + (1ull << 32) : 0ull;
+            if (lane == strip_best_lane(m, pos)) {  // (in a warp without candidates its row is never taken)
                 double2* q = sh.row[par][warp];
                 q[0] = rcp;
 #pragma unroll
                 for (int c = 0; c < R; c++) q[1 + c] = a[c];
-                typename S::Slot v{mk, (int)mp, (int)(rank * T) + tid, m2 > 0.0};
+                typename S::Slot v{m, pos, (int)(rank * T) + tid};
                 typename S::Slot* o = &sh.slot[par][rank * NW + warp];
                 if (C == 1)
                     *o = v;
@@ -237,21 +255,20 @@ __global__ void __launch_bounds__(LuStrip<W>::T) k_lu_strip(int N, int c0, int w
         }
         cluster_sync(C);
         // ---- the column's pivot
-        typename S::Slot best{0, 0x7fffffff, 0, 0};
+        typename S::Slot best{0, 0x7fffffff, 0};
         for (int e = lane; e < (int)C * NW; e += 32) {
             const typename S::Slot v = sh.slot[par][e];
-            if (v.key > best.key || (v.key == best.key && v.key && v.pos < best.pos)) best = v;
+            if (v.m > best.m || (v.m == best.m && v.pos < best.pos)) best = v;
         }
-        const unsigned mk = __reduce_max_sync(0xffffffffu, best.key);
-        const unsigned mp = __reduce_min_sync(0xffffffffu, best.key == mk ? (unsigned)best.pos : 0x7fffffffu);
-        const int from = __ffs(__ballot_sync(0xffffffffu, best.key == mk && best.pos == (int)mp)) - 1;
-        const int src = __shfl_sync(0xffffffffu, best.src, from), low = __shfl_sync(0xffffffffu, best.low, from);
-        const bool none = mk == 0;  // every modulus a NaN: the row at the diagonal, its reciprocal zero
-        const int p = none ? col : (int)mp;
+        const int from = strip_best_lane(best.m, best.pos);
+        const int src = __shfl_sync(0xffffffffu, best.src, from), mp = __shfl_sync(0xffffffffu, best.pos, from);
+        const unsigned long long m = __shfl_sync(0xffffffffu, best.m, from);
+        const bool none = m == 0;  // every modulus a NaN: the row at the diagonal, its reciprocal zero
+        const int p = none ? col : mp;
         const bool mine = none ? pos == col : (int)(rank * T) + tid == src;
         if (rank == 0 && tid == 0) {
             ipiv[(size_t)f * N + col] = p;
-            if (!low && info[f] == 0) info[f] = col + 1;  // not above zero
+            if (m <= 1ull << 32 && info[f] == 0) info[f] = col + 1;  // not above zero
         }
         const double2* prow = sh.row[par][(src % T) >> 5];
         if (C > 1) {

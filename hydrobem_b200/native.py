@@ -97,7 +97,7 @@ EXPORTS = ["hbg_default_options", "hbg_solve_batch", "hbg_debug_matrices", "hbg_
            "hbg_statics_noalloc", "hbg_measure_peaks", "hbg_last_ir_history", "hbg_surrogate_train",
            "hbg_surrogate_grad", "hbg_surrogate_eval", "hbg_last_surrogate_pairs", "hbg_read_gdf", "hbg_gdf_free",
            "hb_model_load_mesh", "hbg_last_fallback_count", "hbg_debug_lu_f64", "hb_model_panels", "hbg_tuned_tiles", "hbg_last_fallback_time",
-           "hbg_debug_cgemv"]
+           "hbg_debug_cgemv", "hbg_debug_lu_pivots"]
 
 _lib = None
 
@@ -131,6 +131,8 @@ def lib():
     L.hbg_last_ir_iterations.argtypes = [ctypes.POINTER(ctypes.c_int32)]
     L.hbg_debug_lu_f64.argtypes = [ctypes.c_int32, ctypes.c_int32, dp, ctypes.c_int32, dp, dp]
     L.hbg_debug_lu_f64.restype = ctypes.c_int32
+    L.hbg_debug_lu_pivots.argtypes = [ctypes.c_int32, ctypes.c_int32, dp, ip]
+    L.hbg_debug_lu_pivots.restype = ctypes.c_int32
     L.hbg_debug_cgemv.argtypes = [ctypes.c_int32] * 3 + [fp, dp, dp, ctypes.c_int32, ctypes.POINTER(ctypes.c_int64)]
     L.hbg_debug_cgemv.restype = ctypes.c_int32
     L.hbg_measure_peaks.argtypes = [dp]
@@ -409,6 +411,16 @@ def debug_lu_f64(A, B):
     X = np.zeros_like(Bc)
     check(lib().hbg_debug_lu_f64(n, batch, Ac.ctypes.data_as(dp), nrhs, Bc.ctypes.data_as(dp), X.ctypes.data_as(dp)))
     return X.transpose(0, 2, 1)
+
+
+def debug_lu_pivots(A):
+    """The row interchanges of debug_lu_f64's factorization: [batch][n], the row swapped with row i at step i."""
+    A = np.asarray(A, dtype=np.complex128)
+    batch, n, _ = A.shape
+    Ac = np.ascontiguousarray(A.transpose(0, 2, 1))  # column-major per matrix
+    piv = np.zeros((batch, n), np.int32)
+    check(lib().hbg_debug_lu_pivots(n, batch, Ac.ctypes.data_as(dp), piv.ctypes.data_as(ip)))
+    return piv
 
 
 def debug_cgemv(M, x, repeats=1):

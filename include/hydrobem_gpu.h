@@ -304,6 +304,10 @@ HbStatus hbg_debug_gemm_tf32(int32_t M, int32_t N, int32_t K, const float *A, co
  * of Real::lu_solve, linalg.rs:100-201 and 321-354, exposed for its numerics test). */
 HbStatus hbg_debug_lu_f64(int32_t n, int32_t batch, const double *A, int32_t nrhs, const double *B, double *X);
 
+/* Test support: the row interchanges of the same factorization: ipiv [batch][n], the 0-based row swapped with row i
+ * at step i (the largest modulus of the column, the first such row; LAPACK's izamax). */
+HbStatus hbg_debug_lu_pivots(int32_t n, int32_t batch, const double *A, int32_t *ipiv);
+
 /* Test support: y = M x by the mixed form's FP64 product (the right-hand sides and residuals): M [batch][2][n][n] FP32,
  * real and imaginary plane, each column-major; x and y [batch][nrhs][n], interleaved (re, im) host arrays; nrhs <= 32.
  * The product is formed `repeats` times; differ receives the number of entries of the later results that are not
