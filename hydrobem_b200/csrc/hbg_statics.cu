@@ -693,7 +693,12 @@ __device__ inline void log_cell(const double m[4][3], const double* image, const
 // reduce them per sub-cell by shuffles), and those to be split push their sub-cells.  A cell's decision depends on
 // its own sums alone, so the cells are those of the reference's depth-first order; their sums are added per warp,
 // then over the warps in order.  (One warp a pair took 0.29-0.39 ms for the few pairs of a small hull.)
-constexpr int AD_WARPS = 8, AD_STACK = AD_WARPS * 48;
+// The stack's bound: the sub-cells of deeper cells go above those of shallower ones, so the stack stays sorted by depth
+// and a round that pushes a level has taken every deeper cell before it.  A level then has at most 4 AD_WARPS cells, of
+// which AD_WARPS went for a full next level: 3 AD_WARPS stay on each of the levels 3 .. 13 under a full level 14, 12
+// on level 2 (of 16) and 3 on level 1 (of 4), 304 in all; a round that pushes two levels shares its cells between them.
+constexpr int AD_WARPS = 8, AD_DEPTH = 14, AD_STACK = AD_WARPS * 48;
+static_assert(16 + 3 * AD_WARPS * (AD_DEPTH - 2) <= AD_STACK, "the adaptive pairs' stack");
 
 struct AdCell {
     double u0, u1, v0, v1, p0, p1;
@@ -774,8 +779,7 @@ __device__ void adaptive_pair(const PanelsView& pv, const int32_t* __restrict__ 
                               __shfl_sync(0xffffffffu, a1, 0) + __shfl_sync(0xffffffffu, a1, 16);
             const double s1 = __shfl_sync(0xffffffffu, b0, 0) + __shfl_sync(0xffffffffu, b0, 16) +
                               __shfl_sync(0xffffffffu, b1, 0) + __shfl_sync(0xffffffffu, b1, 16);
-            split = !(c.depth >= 14 || (fabs(s0 - c.p0) <= tol_l && fabs(s1 - c.p1) <= tol_d));
-            if (split && sp + 4 * AD_WARPS > AD_STACK) split = false;  // (the stack holds more than 14 levels need)
+            split = !(c.depth >= AD_DEPTH || (fabs(s0 - c.p0) <= tol_l && fabs(s1 - c.p1) <= tol_d));
             if (!split) acc0 += s0, acc1 += s1;
         }
         if (lane == 0) sh.split[warp] = split;
@@ -783,7 +787,7 @@ __device__ void adaptive_pair(const PanelsView& pv, const int32_t* __restrict__ 
         int at = sp, total = 0;
 #pragma unroll
         for (int w = 0; w < AD_WARPS; w++) {
-            if (w < warp) at += 4 * sh.split[w];
+            if (w > warp) at += 4 * sh.split[w];  // (warp 0 has the deepest cell)
             total += sh.split[w];
         }
         if (split && (lane & 15) == 0) {  // lanes 0 and 16 hold the sums of sub-cells 0, 2 and 1, 3
