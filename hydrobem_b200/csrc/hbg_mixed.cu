@@ -233,7 +233,7 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
                  midsz = 2 * (size_t)NBL * NBL;
     const size_t nblk = (size_t)Np / NBL, dinv = nblk * 2 * NBL * NBL;
     const int npair = (nrhs + 1) / 2;  // complex64 vectors by column pairs
-    const int nz = (Nm + GEMV_CHUNK - 1) / GEMV_CHUNK;
+    const int nz = (Nm + GV_CHUNK - 1) / GV_CHUNK;  // column chunks of the products
     const int nfp = field.P;
     // A, B [D][D], X, FK, SC, motions, Haskind [H][D], field values [P][D] and 3 x [P][H] per frequency
     // the Kochin functions kr, krt [TK][D], kd, kdt [TK][H] and the drift [H][H][3] after them
@@ -382,14 +382,8 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
     double* hn = (double*)ws.host(HS_NORMS, sizeof(double) * IR_MAX_IT * 2 * (size_t)BS);
     if (!hout || !hn) MIXED_FAIL(HB_ERR_INTERNAL, "page-locked host memory could not be allocated", -1);
     int* herr = reinterpret_cast<int*>(hout + out_per * B);
-    // out = bias - M x over the batch (M column-major planar FP32), FP64 accumulation
     // the column width of a chunk of w right-hand sides of the FP32 product (its padded columns cost as much as real ones)
     auto chunk_width = [](int w) { return w <= 4 ? 4 : w <= 8 ? 8 : w <= 10 ? 10 : w <= 12 ? 12 : 16; };
-    // the FP64 product by TMA and DMMA, all right-hand sides at once; the register form if a map fails
-    auto gemv_tma = [&](const float* Mm, const double2* xv, int ldx, int nb, int nzt, cudaStream_t s) -> bool {
-        return launch_cgemv_dmma(Mm, Nm, Np, xv, ldx, nrhs, nb, nzt, part, err, s);
-    };
-    const int nz_tma = (Nm + GV_CHUNK - 1) / GV_CHUNK;
     for (auto fn : {(const void*)k_cgemv32_tma<4>, (const void*)k_cgemv32_tma<8>, (const void*)k_cgemv32_tma<10>,
                     (const void*)k_cgemv32_tma<12>, (const void*)k_cgemv32_tma<16>})
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gv32_smem_bytes<16>());
@@ -410,7 +404,7 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
             if (!make_map_box(&mDc[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (void*)dv, dd, sd, bd)) return false;
         }
         P.begin(s);
-        dim3 g((Nm + GV_ROWS - 1) / GV_ROWS, nb, nz_tma);
+        dim3 g((Nm + GV_ROWS - 1) / GV_ROWS, nb, nz);
         for (int c0 = 0; c0 < nrhs; c0 += 16) {
             const bool last = c0 + 16 >= nrhs;
             const int nr = nrc[last];
@@ -427,33 +421,22 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
                 k_cgemv32_tma<16><<<g, gv32_threads<16>(), gv32_smem_bytes<16>(), s>>>(mM, mD, Nm, nrhs, c0, part, nb, err);
         }
         k_residual_reduce<true><<<dim3((unsigned)(((size_t)npair * Nm + 255) / 256), nb), 256, 0, s>>>(
-            Nm, Np, nrhs, nb, nz_tma, part, rk, out);
+            Nm, Np, nrhs, nb, nz, part, rk, out);
         P.end(KF_MIXED_RESIDUAL, 8.0 * (double)Nm * Nm * nb, s);
         *launches += 2;
         return true;
     };
+    // out = bias - M x over the batch (M column-major planar FP32), FP64 accumulation
+    bool maps_ok = true;  // the FP64 product's maps were encoded: looked at once the batch has run
     auto gemv = [&](const float* Mm, const double2* xv, int ldx, const double2* bias, auto* out, int nb, int fam,
                     cudaStream_t s) {
         P.begin(s);
-        dim3 g((Nm + 127) / 128, nb, nz);
-        int nzr = nz;
-        if (gemv_tma(Mm, xv, ldx, nb, nz_tma, s))
-            nzr = nz_tma;
-        else if (nrhs <= 8)
-            k_cgemv_part<8><<<g, 128, 0, s>>>(Nm, Np, MB, nrhs, Mm, xv, ldx, part, nb);
-        else if (nrhs <= 10)
-            k_cgemv_part<10><<<g, 128, 0, s>>>(Nm, Np, MB, nrhs, Mm, xv, ldx, part, nb);
-        else if (nrhs <= 12)
-            k_cgemv_part<12><<<g, 128, 0, s>>>(Nm, Np, MB, nrhs, Mm, xv, ldx, part, nb);
-        else if (nrhs <= 16)
-            k_cgemv_part<16><<<g, 128, 0, s>>>(Nm, Np, MB, nrhs, Mm, xv, ldx, part, nb);
-        else
-            k_cgemv_part<32><<<g, 128, 0, s>>>(Nm, Np, MB, nrhs, Mm, xv, ldx, part, nb);
+        maps_ok = launch_cgemv_dmma(Mm, Nm, Np, xv, ldx, nrhs, nb, nz, part, err, s) && maps_ok;
         if constexpr (std::is_same_v<decltype(out), float4*>)  // a residual, for the sweeps
             k_residual_reduce<false><<<dim3((unsigned)(((size_t)npair * Nm + 255) / 256), nb), 256, 0, s>>>(
-                Nm, Np, nrhs, nb, nzr, part, bias, out);
+                Nm, Np, nrhs, nb, nz, part, bias, out);
         else
-            k_gemv_reduce<<<dim3((unsigned)(((size_t)nrhs * Nm + 255) / 256), nb), 256, 0, s>>>(Nm, nrhs, nb, nzr, part,
+            k_gemv_reduce<<<dim3((unsigned)(((size_t)nrhs * Nm + 255) / 256), nb), 256, 0, s>>>(Nm, nrhs, nb, nz, part,
                                                                                                bias, Np, out, Np);
         P.end(fam, 8.0 * (double)Nm * Nm * nb, s);
         *launches += 2;
@@ -840,6 +823,7 @@ int mixed_solve_frequencies(const PanelsView& pv, const double* st, const HbgPro
                 MIXED_FAIL(HB_ERR_INTERNAL, why.c_str(), f0);
             }
         }
+        if (!maps_ok) MIXED_FAIL(HB_ERR_INTERNAL, "tensor-map encoding failed", f0);
         if (*herr == 8) MIXED_FAIL(HB_ERR_INTERNAL, "a triangular sweep wait timed out", f0);
         if (*herr == 11) MIXED_FAIL(HB_ERR_NUMERICAL, "singular motion equation", f0);
         if (*herr != 0 && *herr != 10) MIXED_FAIL(HB_ERR_INTERNAL, "a tensor-core pipeline wait timed out", f0);

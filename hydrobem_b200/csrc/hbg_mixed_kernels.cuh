@@ -34,12 +34,11 @@ struct CgemmArgs {
                            // its 128 k alone, by the same CTA (C may lie over A); CG_LEFT_LOWER: C = X B with X lower
                            // triangular, K = 256: row tile 0 with its 128 k alone
     int a_k0, a_row0;      // A's first k and row in its map
-    int b_k0, b_n0;        // B's first k and column (K-major: row) in its map
+    int b_n0;              // B's first column (K-major: row) in its map
     int subtract;          // C -= A B by a reduction at L2, else C = A B
     int o_row0, o_col0;    // C's first row and column in the planar matrix
     int batch, b0;         // matrices of the launch, the first one's index in the maps
-    // an FP16 copy of C: planes of h_plane halves, row o_row0 + i at i + h_row0 (none while negative), column o_col0 + j
-    // at j + h_col0
+    // an FP16 copy of C (or null): planes of h_plane halves, row o_row0 + i at i + h_row0, column o_col0 + j at j + h_col0
     __half* h16;
     size_t h_bstride, h_plane;
     int h_ld, h_row0, h_col0;
@@ -147,9 +146,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_cgemm(const __grid_constant
 #pragma unroll
                             for (int h = 0; h < 2; h++)  // 64 columns a box
                                 tc::tma_load_4d(sb + h * (GEMM_TILE_BYTES / 2), &mapB, &full[s], g.b_n0 + n * GBN + 64 * h,
-                                                g.b_k0 + kk, p, g.b0 + f);
+                                                kk, p, g.b0 + f);
                         } else {
-                            tc::tma_load_4d(sb, &mapB, &full[s], g.b_k0 + kk, g.b_n0 + n * GBN, p, g.b0 + f);
+                            tc::tma_load_4d(sb, &mapB, &full[s], kk, g.b_n0 + n * GBN, p, g.b0 + f);
                         }
                     }
                 }
@@ -251,7 +250,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_cgemm(const __grid_constant
                 for (int j = 0; j < 8; j++)
                     *reinterpret_cast<float4*>(row + 4 * (j ^ (r & 7))) =
                         make_float4(sg * v[4 * j], sg * v[4 * j + 1], sg * v[4 * j + 2], sg * v[4 * j + 3]);
-                if (g.h16 && hr >= 0) {
+                if (g.h16) {
                     __half* h = g.h16 + (size_t)(g.b0 + f) * g.h_bstride + (size_t)plane * g.h_plane +
                                 (size_t)hr * g.h_ld + g.h_col0 + col;
 #pragma unroll
@@ -779,77 +778,6 @@ __global__ void k_prep_block_row(const float* __restrict__ W, int Np, size_t bst
     for (int r = 0; r < 32; r += 8) Pf[(size_t)(j0 + ty + r) * PW + kk0 + tx] = t[tx][ty + r];
 }
 
-// Partial products of y = M x over column chunks: part[z][f][c][k] = sum_{n in chunk z} M(k, n) x[f][c][n],
-// M column-major planar FP32 (entry (k, n) at n Np + k), x FP64 complex [F][nrhs][ldx]; one thread
-// per row (M read once, coalesced along k), FP64 accumulation.  k_gemv_reduce then forms
-// out = bias - sum_z part[z] in a fixed order (deterministic).
-constexpr int GEMV_CHUNK = 512;
-template <int NR>
-__global__ void __launch_bounds__(128) k_cgemv_part(int N, int Np, size_t bstride, int nrhs,
-                                                    const float* __restrict__ Mall, const double2* __restrict__ xall,
-                                                    int ldx, double2* __restrict__ part, int F) {
-    constexpr int CH = 32;
-    __shared__ double2 sx[CH][NR];
-    const int f = blockIdx.y, z = blockIdx.z;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const float* Mr = Mall + (size_t)f * bstride;
-    const float* Mi = Mr + (size_t)Np * Np;
-    const double2* x = xall + (size_t)f * nrhs * ldx;
-    const int nbeg = z * GEMV_CHUNK, nend = min(N, nbeg + GEMV_CHUNK);
-    double2 acc[NR];
-#pragma unroll
-    for (int c = 0; c < NR; c++) acc[c] = make_double2(0.0, 0.0);
-    for (int n0 = nbeg; n0 < nend; n0 += CH) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < CH * NR; t += blockDim.x) {
-            int nn = t % CH, c = t / CH;
-            sx[nn][c] = (n0 + nn < nend && c < nrhs) ? x[(size_t)c * ldx + n0 + nn] : make_double2(0.0, 0.0);
-        }
-        __syncthreads();
-        if (k < N) {
-            const int lim = min(CH, nend - n0);
-            if (lim == CH) {
-                // a full chunk: the matrix entries of 8 columns loaded ahead of their products
-#pragma unroll
-                for (int q = 0; q < CH; q += 8) {
-                    float mr[8], mi[8];
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const size_t o = (size_t)(n0 + q + j) * Np + k;
-                        mr[j] = Mr[o];
-                        mi[j] = Mi[o];
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const double dr = mr[j], di = mi[j];
-#pragma unroll
-                        for (int c = 0; c < NR; c++) {
-                            const double2 v = sx[q + j][c];
-                            acc[c].x += dr * v.x - di * v.y;
-                            acc[c].y += dr * v.y + di * v.x;
-                        }
-                    }
-                }
-            } else {
-                for (int nn = 0; nn < lim; nn++) {
-                    const size_t o = (size_t)(n0 + nn) * Np + k;
-                    const double mr = Mr[o], mi = Mi[o];
-#pragma unroll
-                    for (int c = 0; c < NR; c++) {
-                        const double2 v = sx[nn][c];
-                        acc[c].x += mr * v.x - mi * v.y;
-                        acc[c].y += mr * v.y + mi * v.x;
-                    }
-                }
-            }
-        }
-    }
-    if (k < N)
-#pragma unroll
-        for (int c = 0; c < NR; c++)
-            if (c < nrhs) part[(((size_t)z * F + f) * nrhs + c) * N + k] = acc[c];
-}
-
 // Packed FP32 pairs (fma.rn.f32x2: two FP32 FMAs per instruction), here over two right-hand sides.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 f2pack(float a, float b) {
@@ -871,8 +799,10 @@ __device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) {
 constexpr int GV_ROWS = 256, GV_COLS = 16, GV_STAGES = 3, GV_CHUNK = 1024;
 constexpr int GV_WORKERS = GV_ROWS / 2;
 
-// The same partial products on the FP64 tensor cores (mma.sync m8n8k4): the matrix and vector tiles streamed by TMA (16
-// columns a stage, both FP32 planes of 256 rows, 32 KB, and the 16 complex entries of every right-hand side) from a
+// Partial products of y = M x over column chunks: part[z][f][c][k] = sum_{n in chunk z} M(k, n) x[f][c][n], M
+// column-major planar FP32 (entry (k, n) at n Np + k), x FP64 complex [F][nrhs][ldx], FP64 accumulation;
+// k_gemv_reduce or k_residual_reduce then forms bias - sum_z part[z] in a fixed order (deterministic).  On the
+// FP64 tensor cores (mma.sync m8n8k4): the matrix and vector tiles streamed by TMA (16 columns a stage, both FP32 planes of 256 rows, 32 KB, and the 16 complex entries of every right-hand side) from a
 // producer warp, eight warps of 32 rows each.  Real columns 2 c and 2 c + 1 of the product are the real and imaginary
 // part of right-hand side c: C += Mr [Xr, Xi] + Mi [-Xi, Xr].  Lane (i, k) of a warp reads rows 4 i .. 4 i + 3 of column
 // k by one 16-byte load, row tile t taking rows 4 i + t, and each pair of vector entries serves four row tiles; all
@@ -1311,7 +1241,7 @@ __global__ void __launch_bounds__(TRI_THREADS, 1) k_tri_sweep(const __grid_const
         }
         tc::fence_barrier_init();
     }
-    // a last group's missing pairs stay zero
+    // (a group's missing pairs hold zeros, or an earlier item's values: their results are not stored)
     for (int t = threadIdx.x; t < (NYB + 1) * NQ * TB; t += TRI_THREADS) ys[t] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     auto wait = [&](uint64_t* bar, uint32_t parity) {  // bounded; after an error the protocol runs on, its results discarded

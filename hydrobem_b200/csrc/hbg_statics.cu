@@ -671,22 +671,6 @@ __global__ void __launch_bounds__(256, 3) k_statics(PanelsView pv, double depth,
     st[3 * NN + o] = prod ? to_f32(dd) : dd;
 }
 
-// 4 x 4 Gauss rule of a cell of the parameter square (panel_integrals.rs:80-98)
-__device__ inline void log_cell(const double m[4][3], const double* image, const double* n, double u0, double u1,
-                                double v0, double v1, double* s) {
-    s[0] = s[1] = 0.0;
-    double hu = 0.5 * (u1 - u0), hv = 0.5 * (v1 - v0);
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++) {
-            double xi[3], jac, psi, dpsi;
-            bilinear(m, u0 + hu * (c_glx[4][i] + 1.0), v0 + hv * (c_glx[4][j] + 1.0), xi, jac);
-            double ww = c_glw[4][i] * c_glw[4][j] * hu * hv * jac;
-            psi_terms(xi, image, n, psi, dpsi);
-            s[0] += ww * psi;
-            s[1] += ww * dpsi;
-        }
-}
-
 // The adaptive pairs: quadrisection to 1e-13 of the integrals' scale, at most 14 levels
 // (panel_integrals.rs:100-120).  One CTA per pair: the cells wait on a stack in shared memory, each round the
 // AD_WARPS topmost are taken, a warp each (the 32 lanes evaluate the 4 sub-cells x 16 Gauss points, two a lane, and

@@ -54,7 +54,7 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-// 4-D tiled TMA store from this CTA's shared memory (bulk group; wait with bulk_wait_read).
+// 4-D tiled TMA store from this CTA's shared memory (bulk group; wait with bulk_wait_read_n or bulk_wait_all).
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* src, int c0, int c1, int c2, int c3) {
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(map),
                  "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
@@ -69,7 +69,6 @@ __device__ __forceinline__ void tma_reduce_add_4d(const CUtensorMap* map, const 
                  : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // wait until at most N bulk groups of this thread are still reading their shared-memory source
 template <int N>
