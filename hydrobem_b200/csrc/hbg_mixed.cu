@@ -153,14 +153,17 @@ static std::atomic<int> g_lu_groups_override{0};
 void mixed_lu_groups(int groups) { g_lu_groups_override = std::max(0, std::min(groups, LU_GROUPS)); }
 // the groups of a batch of ns systems of order Np: about eight systems a group, at most LU_GROUPS (a group's
 // launches cover its systems, so a group of a few small systems leaves its products and factors too
-// short to fill the device); fewer than eight large systems in up to three groups, so that one group's chain of
-// diagonal blocks (217 us a panel) runs beside the products of the others.  LU measured, ms with 1 / 2 / 3 / 4
-// groups: 40 systems of order 4096 17.1 / 16.2 / 15.8 / 15.5; six bodies of 16 systems of orders 1792-3840 on two
-// pipelines 48.3 / 45.8 / 49.2 / 49.6; 4 of order 12288 35.9 / 34.2 / 34.2 / 33.8; 5 of order 18560 114 / 114 /
-// 109 / 110; 10 of order 512 0.47 with any.
+// short to fill the device); fewer than eight large systems in up to two groups, from order 5120 in up to three, so that
+// one group's chain of diagonal blocks (217 us a panel) runs beside the products of the others: with smaller orders the
+// products are too short to hide much of it.  LU measured, ms with 1 / 2 / 3 / 4 groups: 40 systems of order 4096 17.1 /
+// 16.2 / 15.8 / 15.5; six bodies of 16 systems of orders 1792-3840 on two pipelines 48.3 / 45.8 / 49.2 / 49.6; 10 of
+// order 512 0.47 with any; of order 2176, 3 systems 2.27 / 2.27 / 2.34, 7 2.51 / 2.44 / 2.45 / 2.49; of order 4096, 3
+// 4.71 / 4.59 / 4.70, 5 5.25 / 5.07 / 5.07 / 5.12, 7 5.87 / 5.62 / 5.54 / 5.53; of order 6144, 3 8.19 / 7.99 / 7.93, 5
+// 9.80 / 9.41 / 9.21 / 9.17; of order 12288, 3 26.7 / 25.7 / 25.1, 4 31.7 / 29.7 / 29.9 / 29.6; 5 of order 18560 114 /
+// 114 / 109 / 110.
 static int lu_groups_for(int Np, int ns) {
     const int o = g_lu_groups_override.load();
-    const int g = ns < 8 && Np >= 2048 ? 3 : std::min(LU_GROUPS, ns / 8);
+    const int g = ns >= 8 || Np < 2048 ? std::min(LU_GROUPS, ns / 8) : Np < 5120 ? 2 : 3;
     return std::max(1, std::min(o > 0 ? o : g, ns));
 }
 // The panels of a super-step of the LU: its trailing matrix (8 bytes an entry, read and written by the

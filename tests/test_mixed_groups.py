@@ -1,5 +1,5 @@
-"""The mixed form's LU on several stream groups of few large systems: three groups of three to seven systems (uneven and
-single ones), from the smallest order that takes them, and the groups of eight systems beside them."""
+"""The mixed form's LU on several stream groups of few large systems: two and three groups of two to seven systems (uneven
+and single ones), from the smallest orders that take them, and the groups of eight systems beside them."""
 from __future__ import annotations
 
 import math
@@ -12,11 +12,11 @@ from hydrobem_b200 import meshes
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("n_phi,n_z,n_r,freqs", [(48, 20, 20, 3), (48, 22, 23, 2), (48, 22, 23, 4), (48, 22, 23, 5), (48, 22, 23, 7),
-                                                 (64, 20, 20, 8)])
+                                                 (64, 20, 20, 8), (64, 40, 41, 3), (64, 40, 41, 5)])
 def test_few_large_systems(n_phi, n_z, n_r, freqs):
     from hydrobem_b200 import native as nv
 
-    v = meshes.cylinder(1.0, 0.5, n_phi, n_z, n_r)  # 1920, 2160, 2560 panels
+    v = meshes.cylinder(1.0, 0.5, n_phi, n_z, n_r)  # 1920, 2160, 2560, 5184 panels
     omegas = np.sqrt(np.linspace(0.3, 1.1, freqs) * meshes.GRAVITY)
     ref = nv.solve(v, omegas, [20.0], depth=math.inf, precision=nv.HBG_FP64)
     got = nv.solve(v, omegas, [20.0], depth=math.inf, precision=nv.HBG_MIXED)
