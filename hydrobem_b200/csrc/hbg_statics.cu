@@ -829,8 +829,12 @@ void launch_panel_geometry(int N, const double* verts, const int32_t* kind, doub
     k_panel_geometry<<<(N + 127) / 128, 128, 0, s>>>(N, verts, kind, planes, bad, tiers, orig);
 }
 
-// Pairs up to which a warp takes four rows instead of 32.  Measured, us with 4 / 32 rows: 84 panels 35 / 56; 512 panels
-// 388 / 97 (eight rows 210): a warp costs the same with few rows, so they pay only while the device is nearly empty.
+// Pairs up to which a warp takes four rows instead of 32.  A warp costs the same with few rows, so they pay only while
+// the device is nearly empty.  Measured, us with 4 / 32 rows: the FP64 form in deep water 42 panels 23 / 66, 81 29 / 66,
+// 121 47 / 62, 144 54 / 64, 169 70 / 64, 240 117 / 64, 506 448 / 111; in depth 3 m (three times the images) 81 45 / 80,
+// 121 78 / 76, 144 92 / 78; the mixed form 121 47 / 68 and 62 / 74, 169 68 / 67 and 79 / 68; a box hull of 84 35 / 51,
+// 144 60 / 52.  The line (126 panels) is where the first of them cross; 8 and 16 rows are within 20 us of the better one
+// between 100 and 240 panels.
 constexpr double STATICS_SMALL = 1.6e4;
 
 void launch_statics(const PanelsView& pv, double depth, int logint, double tol, double* st, int32_t* work,
