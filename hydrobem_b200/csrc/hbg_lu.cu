@@ -147,7 +147,6 @@ constexpr int LU_CLUSTER = 8;  // the portable limit
 template <int W>
 struct LuStrip {
     static constexpr int T = W == 32 ? 256 : 512, NW = T / 32;  // threads (rows) of a CTA, its warps
-    static constexpr int MAXROWS = T * LU_CLUSTER;
     struct __align__(16) Slot {
         unsigned long long m;  // the bits of |a|^2, the upper word plus one (0: no candidate)
         int pos, src;
@@ -345,12 +344,18 @@ __global__ void __launch_bounds__(LuStrip<W>::T) k_lu_strip(int N, int c0, int w
     }
 }
 
+// the CTAs (threads of a row each) of a strip's cluster: the next power of two
+template <int W>
+static int strip_ctas(int rows) {
+    int c = 1;
+    while (c * LuStrip<W>::T < rows) c *= 2;
+    return c;
+}
 template <int W>
 static void launch_lu_strip(int N, int F, int c0, int w, int pk0, int pnb, double2* A, size_t stride, int32_t* ipiv,
                             int32_t* info, cudaStream_t s) {
     using S = LuStrip<W>;
-    int C = 1;
-    while (C * S::T < N - c0) C *= 2;
+    const int C = strip_ctas<W>(N - c0);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(F * C);
     cfg.blockDim = dim3(S::T);
@@ -845,18 +850,19 @@ struct LuF64 {
         return n;
     }
     void panel(int c0, int w) {
-        // Strips of 32 or 16 columns in registers while their rows fit a cluster and the launch's CTAs, one an SM, take
-        // few waves, else of 8 columns in global memory (one CTA a matrix): with more matrices the products beside the panel
-        // are the longer part, and the clusters take their SMs.  LU, ms, strips of 8 / of 32 and 16 everywhere / by this
-        // rule: order 3072 40 matrices 121.6 / 124.2 / 121.6, 80 236.4 / 247.6 / 235.0; 2160 24 31.6 / 29.6 / 29.6, 80 90.3 /
-        // 95.9 / 90.7; 1120 80 17.0 / 16.9 / 16.9, 160 32.0 / 32.8 / 29.7; 640 160 9.1 / 7.9 / 7.6.
-        const int rows = N - c0;
-        auto fits = [&](int maxrows, int t, int half_waves) {
-            return rows <= maxrows && 2 * F * ((rows + t - 1) / t) <= half_waves * n_sm();
-        };
-        const int base = fits(LuStrip<32>::MAXROWS, LuStrip<32>::T, 6)   ? 32
-                         : fits(LuStrip<16>::MAXROWS, LuStrip<16>::T, 3) ? 16
-                                                                         : LU_BASE;
+        // Strips of 32 or 16 columns in registers, else of 8 columns in global memory (one CTA a matrix): clusters take their
+        // SMs from the products that run beside the panel, so with more matrices these become the longer part, the sooner
+        // the larger the cluster.  LU, ms, without / with the form at the order where it is the first, by matrices:
+        //   32 columns, one CTA     order  256: 200 2.02 / 1.28, 900 6.62 / 4.61, 2500 16.6 / 11.7     always
+        //   32 columns, 2 CTAs      order  512: 190 5.42 / 5.22, 222 5.92 / 5.74, 260 6.65 / 6.86      to 3 waves of the SMs
+        //   32 columns, 4 CTAs      order 1024: 46 7.99 / 7.80, 56 9.01 / 9.00, 64 9.93 / 10.01        to 1.5
+        //   32 columns, 8 CTAs      order 2048: 14 17.3 / 15.4, 18 19.8 / 19.7, 22 23.1 / 23.4         to 1
+        //   16 columns, 8 CTAs      order 4096: 8 58.6 / 58.2, 10 71.7 / 72.1; 2560: 12 24.3 / 24.1    to 0.5
+        const int rows = N - c0, c32 = strip_ctas<32>(rows), c16 = strip_ctas<16>(rows);
+        auto few = [&](int ctas, int half_waves) { return 2 * F * ctas <= half_waves * n_sm(); };
+        const int base = c32 == 1 || (c32 <= LU_CLUSTER && few(c32, c32 == 2 ? 6 : c32 == 4 ? 3 : 2)) ? 32
+                         : c16 <= LU_CLUSTER && few(c16, 1)                                           ? 16
+                                                                                                      : LU_BASE;
         if (w <= base) {
             KernelProfiler& P = profiler();
             const double m = N - c0;
