@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(512) k_lu_base(int N, int c0, int w, int pk0, 
 // instructions, ~1.1 us a column in one CTA, ~2 in clusters: a strip of 32 columns takes 41 / 64 / 79 us with 84 / 645 /
 // 1007 rows where one of 8 columns with its rows in global memory took 18 / 23 / 28, and 64 with 4096, and a panel now
 // needs three products between its strips instead of fifteen.  Whole LU, ms, before / now: 9 systems of order 645 3.28
-// / 2.21, 21 of order 1007 6.8 / 4.75, 8 of order 4096 64.8 / 58.9.
+// / 2.06, 21 of order 1007 6.8 / 4.57, 8 of order 4096 64.8 / 58.3.
 constexpr int LU_CLUSTER = 8;  // the portable limit
 template <int W>
 struct LuStrip {

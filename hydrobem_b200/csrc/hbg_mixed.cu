@@ -93,10 +93,11 @@ struct MixedBuffers {
 };
 
 // Refinement stops when the error left after the last correction d_k is predicted below IR_TOL of
-// the largest solution entry: that error is about rho |d_k|, rho = |d_k| / |d_{k-1}| being the
-// observed contraction (about 1e-3 with the TF32 factors), and at most |d_k| itself.  The solution
-// is then that of the complex64 system to ~1e-9, far inside its ~1e-7 distance from the FP64
-// system's solution (the rounding of the stored matrix).
+// the largest solution entry: rho |d_k|, rho = |d_k| / |d_{k-1}| being the observed contraction (about
+// 1e-3 with the TF32 factors).  The corrections still to come add up to rho / (1 - rho) |d_k| while they
+// contract by rho: at a contraction of 0.5, the limit for a system to stay with these factors, twice that.
+// The solution is then that of the complex64 system to ~1e-9 (2e-9), far inside its ~1e-7 distance from the
+// FP64 system's solution (the rounding of the stored matrix).
 constexpr double IR_TOL = 1e-9;
 constexpr int IR_MAX_IT = 30;
 

@@ -809,7 +809,9 @@ constexpr int GV_WORKERS = GV_ROWS / 2;
 // right-hand sides in one pass over the matrix.  Bound by the FP64 pipe (4 FMA an entry and right-hand side at 37
 // TFLOP/s, NT tiles of 4 right-hand sides); the FMA form before it (a thread two rows, at most 16 right-hand sides a
 // pass) spent as long on its shared-memory loads.  Measured, ms, before / now: 40 matrices of order 4096 and 10
-// right-hand sides 2.39 / 2.03, 4 of order 12288 and 19 5.4 / 3.0, 5 of order 18496 and 14 12.1 / 6.7.
+// right-hand sides 2.39 / 2.03, 4 of order 12288 and 19 5.4 / 3.0, 5 of order 18496 and 14 12.1 / 6.7.  The steps of a
+// stage unrolled four times up to five tiles, not at all beyond (ms, 16 matrices of order 4096, unrolled / not: 8
+// right-hand sides 0.60 / 0.62, 12 0.87 / 0.91, 20 1.367 / 1.373, 24 1.66 / 1.63, 32 2.23 / 2.18).
 constexpr int GD_THREADS = GV_ROWS + 32;  // eight MMA warps of 32 rows, the producer
 template <int NT>
 struct GdCfg {  // NT: tiles of four right-hand sides

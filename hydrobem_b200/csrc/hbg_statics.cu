@@ -533,8 +533,10 @@ __device__ inline double log_in_plane(const PanelRegs& p, const double* x) {
 // Four planes of Nr x N (rows k < Nr = N / G, the sector's points, or the Nr field points; every panel
 // j), entry at k + j Nr.
 // MIXED: the mixed form's variant (far Rankine points and the order-4 log rule in FP32, above; with
-// pv.tiers the reference's production rule instead, rows in float32); the FP64 form runs the reference's
-// double-precision arithmetic to the bit.
+// pv.tiers the reference's production rule instead, rows in float32).  The FP64 form runs the reference's double-precision
+// arithmetic: its decisions, closed forms, 3 x 3 and order-4 rules in the reference's order of operations; the sums of the
+// orders 5 to 10 (lanes, then shuffles) and of the adaptive cells (warps) are added in another order, so that those log
+// integrals differ in their last bits.
 // Bound by instruction issue and the conversions' pipe (per 32 pairs of the mixed form, infinite depth: 1800
 // instructions, of them 440 FP64 and 150 conversions and reciprocals, before; FP64 closed forms near, the 3 x 3 and
 // order-4 rules far).  Three CTAs an SM (80 registers, some spills) against two: 18496 panels 32.6 / 39.3 ms.  Measured, ms
