@@ -713,8 +713,6 @@ void launch_boundary(const PanelsView& pv, int F, const FreqInfo* fi, int H, con
 // nrhs partial sums: S is read once, eight columns in flight a thread (coalesced along k), u staged in shared
 // memory; k_rhs_sum adds the chunks in order.  One thread for all columns of its row left the device to a few
 // latency-bound CTAs: 0.47 ms for 9 systems of order 645, 3.0 for 8 of order 4096, now 0.09 and 0.98.
-// Sums held: 6, 8, 16 or 32 (8 systems of order 2112, ms: 6 right-hand sides 0.143, 7 and 8 0.174, 9 and 10 0.321 with
-// ten sums and 11 to 16 0.333-0.341 with sixteen, 17 to 32 0.58-0.60: beyond eight the count of the sums matters little).
 // Columns of a chunk: 128, more where that would be over 16 chunks (a large matrix has rows enough to fill the device).
 static int rhs_chunk(int N) { return std::max(128, (N + 511) / 512 * 32); }
 template <int NR>
@@ -785,6 +783,8 @@ void launch_rhs_f64(int N, int F, int nrhs, const double2* S, size_t mat_stride,
         go(k_rhs_f64<6>);
     else if (nrhs <= 8)
         go(k_rhs_f64<8>);
+    else if (nrhs <= 10)
+        go(k_rhs_f64<10>);
     else if (nrhs <= 16)
         go(k_rhs_f64<16>);
     else
