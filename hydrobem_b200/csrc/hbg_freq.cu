@@ -713,6 +713,10 @@ void launch_boundary(const PanelsView& pv, int F, const FreqInfo* fi, int H, con
 // nrhs partial sums: S is read once, eight columns in flight a thread (coalesced along k), u staged in shared
 // memory; k_rhs_sum adds the chunks in order.  One thread for all columns of its row left the device to a few
 // latency-bound CTAs: 0.47 ms for 9 systems of order 645, 3.0 for 8 of order 4096, now 0.09 and 0.98.
+// Sums held: 6, 8, 10, 16 or 32; the padded ones cost as much as real ones until the loads of S are the longer part (ms of
+// 16 systems of order 4096: 8 right-hand sides 1.01, 9 and 10 1.91-1.92 with ten sums and 2.17 with sixteen, 11 2.18, 16
+// 2.21; of order 2160 10 0.55 and 0.64; 8 systems of order 2112: 6 0.143 with six sums, 7 and 8 0.174, 16 0.341, 17
+// 0.579, 32 0.598).
 // Columns of a chunk: 128, more where that would be over 16 chunks (a large matrix has rows enough to fill the device).
 static int rhs_chunk(int N) { return std::max(128, (N + 511) / 512 * 32); }
 template <int NR>
